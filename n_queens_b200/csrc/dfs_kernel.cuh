@@ -9,9 +9,10 @@
 //    pushed to the lane's shared-memory stack, so a pop always resumes a level
 //    with work and every DFS step places exactly one queen.
 //  * The count kernels' step (VAR 4) lists only a level's alive columns --
-//    those whose child still has a free column in the next row -- and counts
-//    the completions of a row N-2 level from its alive columns instead of
-//    stepping rows N-2 and N-1 (37 % fewer steps at N=18).
+//    those whose child still has a free column in the next row -- skips
+//    children whose row two below has none, and counts the completions of a
+//    row N-2 level from its alive columns instead of stepping rows N-2 and N-1
+//    (44 % fewer steps at N=18).
 //  * cols carries the off-board bits (~last) pre-set.  Then the free mask is
 //    one LOP3 (~(cols|ld|rd)) with no `& last`, a completed board is
 //    cols == 0xffffffff, and no depth counter is kept at all.
@@ -249,13 +250,32 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
 // alive column of it completes the board on row N-1, so the step adds the
 // popcount of its filtered list.  Rows N-2 and N-1 are never stepped and dead
 // children never cost a step or a stack push: at N=18, k=6 the steps fall from
-// 29.7e9 to 18.6e9 and the pushes from 7.8e9 to 5.0e9, for 32 instructions per
-// step instead of 20.  Tasks and saved levels on rows N-2 and N-1 are counted
-// when they are loaded.  Lane registers as in VAR 3.  Operands as in VAR 1
-// plus %12 = 0x3fffffff, %13 = -4, %14 = 30.  Pipe balance (N=21, measured):
-// taking the highest bit's mask from bfind's shift amount instead of a
-// multiply-add saved 4.2 %, negating F0 on the ALU instead of the FMA pipe
-// 0.3 %; moving the count or the first negation to the ALU pipe did not help.
+// 29.7e9 to 18.6e9 and the pushes from 7.8e9 to 5.0e9.  Tasks and saved levels
+// on rows N-2 and N-1 are counted when they are loaded.
+//
+// Look-ahead: a child above row N-2 whose row two below (F1 = ~(c | l<<2 |
+// r>>2)) has no free column even before anything is placed under it is not
+// entered either.  That takes a multiply, a shift and a LOP3 whose predicate
+// output replaces pg, and removes 9 % of the steps at N=14, 11 % at N=18 and
+// 12.6 % at N=21 (CPU model of the step); looking one row further would remove
+// 5 % more for another three operations, which is even.
+//
+// Lane registers: ld as in VAR 3; rd too is kept pre-shifted for the children
+// (right >> 1), so a child's right mask is (bit >> 1) + rd, which the compiler
+// issues as one operation (shift-and-add) where `|` and the shift took two, and
+// the shift for the grandchildren rides on the descend move.  (A multiply-high
+// in its place loads the FMA pipe more than it saves, see VAR 3.)
+// Operands as in VAR 1 plus %12 = 0x3fffffff, %13 = -4, %14 = 30.
+//
+// What bounds it: integer issue (84 % of the issue slots, ALU pipe 72 %, FMA
+// 69 %, XU 55 %, shared-memory wavefronts 62 % at N=18).  Measured without and
+// with both changes: 1.1e6 prefixes of N=18, k=6 19.47 -> 18.34 ms (pre-shifted
+// rd alone: 4 %), N=19 153.2 -> 147.8 ms, 8 % of N=21's prefixes 952 -> 911 ms.
+// Pipe balance: taking the highest bit's mask from bfind's shift amount instead
+// of a multiply-add saved 4.2 % at N=21, negating F0 on the ALU instead of the
+// FMA pipe 0.3 %.  Slower at N=18: moving avail as a float on the light half of
+// the FMA pipe (+1.5 %), moving registers in pairs by mad.wide (+30 %), one
+// compare with two outputs for pg and p2 (+12 %: the compiler adds operations).
 #define NQB_STEP4_HEAD                                                                \
     "{\n\t"                                                                           \
     ".reg .pred pt1, pb, pg, p2, pd, pk, pp, pq;\n\t"                                 \
@@ -267,8 +287,8 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "lop3.and.b32 bit|pb, t, %3, 0, 0xC0, pt1;\n\t"                                   \
     "mad.lo.s32 nc, bit, %8, %0;\n\t"                                                 \
     "mad.lo.s32 nl, bit, %9, %1;\n\t"                                                 \
-    "or.b32 nr, %2, bit;\n\t"                                                         \
-    "shr.s32 nr, nr, 1;\n\t"                                                          \
+    "shr.u32 nr, bit, 1;\n\t"                                                         \
+    "add.u32 nr, nr, %2;\n\t"                                                         \
     "lop3.b32 na, nc, nl, nr, 0x01;\n\t"                                              \
     "mul.lo.s32 xl, nl, %9;\n\t"                                                      \
     "shr.s32 xr, nr, 1;\n\t"                                                          \
@@ -281,6 +301,9 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "popc.b32 pc, nc;\n\t"                                                            \
     "setp.ne.and.u32 pg, pc, %14, pb;\n\t"                                            \
     "setp.eq.and.u32 p2, pc, %14, pb;\n\t"                                            \
+    "mul.lo.s32 t, xl, %9;\n\t"                                                       \
+    "shr.s32 pos, xr, 1;\n\t"                                                         \
+    "lop3.and.b32 t|pg, nc, t, pos, 0x01, pg;\n\t"                                    \
     "lop3.and.b32 naf|pd, na, ma, mb, 0xE0, pg;\n\t"                                  \
     "popc.b32 t, naf;\n\t"                                                            \
     "@p2 mad.lo.s32 %5, t, %8, %5;\n\t"                                               \
@@ -290,13 +313,14 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "@pp mad.lo.s32 %4, %8, %11, %4;\n\t"                                             \
     "@pd mul.lo.s32 %0, nc, %8;\n\t"                                                  \
     "@pd mul.lo.s32 %1, xl, %8;\n\t"                                                  \
-    "@pd mul.lo.s32 %2, nr, %8;\n\t"                                                  \
+    "@pd mul.lo.s32 %2, xr, %8;\n\t"                                                  \
     "@pd mul.lo.s32 %3, naf, %8;\n\t"                                                 \
     "setp.ne.and.u32 pq, %4, %7, !pk;\n\t"                                            \
     "@pq mad.lo.s32 %4, %10, %11, %4;\n\t"                                            \
     "@pq ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
 
 #define NQB_STEP4_X4 NQB_STEP4 NQB_STEP4 NQB_STEP4 NQB_STEP4
+#define NQB_STEP4_X16 NQB_STEP4_X4 NQB_STEP4_X4 NQB_STEP4_X4 NQB_STEP4_X4
 
 // Dihedral step: the VAR 1 step plus the class rules of the lane's task.
 //   pc = popc(child cols) = 32 - N + child row
@@ -419,18 +443,25 @@ constexpr int kStackRowsSpared = VAR == 4 ? 2 : 0;
 
 // Lane registers (ld, rd) from the reference's (left, right) masks of the row
 // a level enumerates, and back (for the checkpoint file, which stores the
-// reference's form).  Going back loses left's bit 31, which no later row can
-// see (a left bit only moves further left).
+// reference's form).  Going back loses left's bit 31 and right's bit 0, which
+// no later row can see (left bits only move further left, right bits further
+// right, and the level's own untried columns are stored beside them).
 template <int VAR>
 __device__ __forceinline__ uint32_t lane_ld(uint32_t left) { return VAR >= 3 ? left << 1 : left; }
 template <int VAR>
 __device__ __forceinline__ uint32_t ref_ld(uint32_t ld) { return VAR >= 3 ? ld >> 1 : ld; }
+template <int VAR>
+__device__ __forceinline__ uint32_t lane_rd(uint32_t right) {
+    return VAR == 4 ? (uint32_t)((int32_t)right >> 1) : right;
+}
+template <int VAR>
+__device__ __forceinline__ uint32_t ref_rd(uint32_t rd) { return VAR == 4 ? rd << 1 : rd; }
 
 // The alive part of a level's untried columns (VAR 4): drops every column
-// whose child would leave the next row without a free column.  ld in lane
-// form (pre-shifted), rd in the reference's form.
+// whose child would leave the next row without a free column.  ld and rd in
+// VAR 4's lane form (pre-shifted).
 __device__ __forceinline__ uint32_t alive_columns(uint32_t cols, uint32_t ld, uint32_t rd, uint32_t avail) {
-    const uint32_t f0 = ~(cols | ld | (uint32_t)((int32_t)rd >> 1));
+    const uint32_t f0 = ~(cols | ld | rd);
     if (f0 == 0) return 0;
     const uint32_t lo = f0 & (0u - f0);
     const int hi = 31 - __clz(f0);
@@ -494,19 +525,29 @@ __device__ __forceinline__ void dfs_steps3(uint32_t &cols, uint32_t &ld, uint32_
     }
 }
 
-// UNROLL steps of VAR 4 (no NODES form), four per asm block.  Operand %6 is
-// unused (it stands where the node counter sits in the other forms).
+// UNROLL steps of VAR 4 (no NODES form), sixteen per asm block where UNROLL
+// allows (0.5 % faster at N=19 than four), else four.  Operand %6 is unused (it
+// stands where the node counter sits in the other forms).
 template <int UNROLL>
 __device__ __forceinline__ void dfs_steps4(uint32_t &cols, uint32_t &ld, uint32_t &rd, uint32_t &avail, uint32_t &sp,
                                            uint32_t &cnt, uint32_t bot, const StepConsts &k) {
-    static_assert(UNROLL % 4 == 0, "VAR 4 unrolls in groups of 4");
+    static_assert(UNROLL % 4 == 0, "VAR 4 unrolls in groups of 4 or 16");
+    constexpr int kGroup = UNROLL % 16 == 0 ? 16 : 4;
 #pragma unroll
-    for (int g = 0; g < UNROLL / 4; ++g)
-        asm volatile(NQB_STEP4_HEAD NQB_STEP4_X4 "}\n\t"
-                     : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt)
-                     : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(0x3fffffffu),
-                       "r"(0xfffffffcu), "r"(30u)
-                     : "memory");
+    for (int g = 0; g < UNROLL / kGroup; ++g) {
+        if constexpr (kGroup == 16)
+            asm volatile(NQB_STEP4_HEAD NQB_STEP4_X16 "}\n\t"
+                         : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt)
+                         : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(0x3fffffffu),
+                           "r"(0xfffffffcu), "r"(30u)
+                         : "memory");
+        else
+            asm volatile(NQB_STEP4_HEAD NQB_STEP4_X4 "}\n\t"
+                         : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt)
+                         : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(0x3fffffffu),
+                           "r"(0xfffffffcu), "r"(30u)
+                         : "memory");
+    }
 }
 
 __device__ __forceinline__ void load_class_index(const DfsParams &p, uint32_t idx, DihLane &d) {
@@ -568,7 +609,7 @@ __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, u
     }
     cols = c | ~last;
     ld = lane_ld<VAR>(l);
-    rd = r;
+    rd = lane_rd<VAR>(r);
     avail = ~(cols | l | r);
     if (VAR == 4) return settle_level(n, cols, ld, rd, avail);
     return 0;
@@ -674,7 +715,7 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                         } else {
                             cols = e.x;
                             ld = lane_ld<LVAR>(e.y);
-                            rd = e.z;
+                            rd = lane_rd<LVAR>(e.z);
                             avail = e.w;
                             // a level saved on row N-2 or N-1 (by a kernel that steps those rows)
                             if (VAR == 4 && !DIH) tot += settle_level(p.N, cols, ld, rd, avail);
@@ -808,7 +849,7 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
             atomicOr(p.ctl + kCtlError, kErrContOverflow);
         } else if (mine) {
             if (avail) {
-                p.cont_out[at] = make_uint4(cols, ref_ld<LVAR>(ld), rd, avail);
+                p.cont_out[at] = make_uint4(cols, ref_ld<LVAR>(ld), ref_rd<LVAR>(rd), avail);
                 if (p.cont_out_owner) p.cont_out_owner[at] = owner;
                 if (DIH) p.cont_out_cls[at] = (uint8_t)dih.cls;
                 ++at;
@@ -816,7 +857,7 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
             for (uint32_t a = bot; a != sp; a += stride, ++at) {
                 uint32_t x, y, z, w;
                 lds128(a, x, y, z, w);
-                p.cont_out[at] = make_uint4(x, ref_ld<LVAR>(y), z, w);
+                p.cont_out[at] = make_uint4(x, ref_ld<LVAR>(y), ref_rd<LVAR>(z), w);
                 if (p.cont_out_owner) p.cont_out_owner[at] = owner;
                 if (DIH) p.cont_out_cls[at] = (uint8_t)dih.cls;
             }
