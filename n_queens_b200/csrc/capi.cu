@@ -43,7 +43,8 @@ constexpr int kMaxBlocksPerSm = 32;
 constexpr int kWordSum = kCtlWords + 0;
 constexpr int kWordNodes = kCtlWords + 1;
 constexpr int kWordStatus = kCtlWords + 2;
-constexpr int kWordBlocks = 8;
+constexpr int kWordBlocks = 16;
+constexpr uint32_t kMailCap = 1u << 15;  // mailbox slots (256 B each)
 
 thread_local std::string g_last_error;
 
@@ -115,6 +116,7 @@ struct Ctx {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[4] = {};
     unsigned long long *d_ctl = nullptr;  // control words + results + per-CTA partials
+    MailSlot *d_mail = nullptr;           // kMailCap mailbox slots
     DevBuf tasks;                         // cols | ld | rd (uint32 SoA)
     DevBuf aux;                           // order, owners, task_n, per-task outputs
     HostBuf h_tasks;                      // pinned staging for the expander
@@ -141,9 +143,12 @@ int ensure_ready(Ctx &c, int dev) {
     c.smem_optin = (int)prop.sharedMemPerBlockOptin;
     NQ_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     for (auto &e : c.ev) NQ_CUDA(cudaEventCreate(&e));
-    const size_t ctl_words = kWordBlocks + 4 * (size_t)c.sms * kMaxBlocksPerSm;
+    const size_t ctl_words = kWordBlocks + 5 * (size_t)c.sms * kMaxBlocksPerSm;
     NQ_CUDA(cudaMalloc(&c.d_ctl, ctl_words * sizeof(unsigned long long)));
     NQ_CUDA(cudaMemset(c.d_ctl, 0, ctl_words * sizeof(unsigned long long)));
+    NQ_CUDA(cudaMalloc(&c.d_mail, kMailCap * sizeof(MailSlot)));
+    NQ_CUDA(cudaMemsetAsync(c.d_mail, 0, kMailCap * sizeof(MailSlot), c.stream));
+    NQ_CUDA(cudaStreamSynchronize(c.stream));  // launches may use any stream
     // Dynamic shared memory above 48 KiB needs an opt-in per kernel.
     const int static_smem = kDfsStaticSmem;
     for (int po = 0; po < 2; ++po)
@@ -182,6 +187,7 @@ int lock_device(int dev, Ctx *&out) {
 struct Launch {
     int threads = 0, levels = 0, smem = 0, grid = 0, inner = 0, steal = 1, layout = 0;
     bool dih = false;  // dihedral-decomposition kernel
+    bool auto_inner = true;  // inner is the default, not the caller's
 };
 
 // Chooses the persistent grid: CTA size, stack slots per lane and as many
@@ -237,6 +243,7 @@ int plan_launch(Ctx &c, const nq_config *cfg, int levels_needed, bool per_owner,
         return NQ_ERR_ARG;
     }
     L.inner = (cfg && cfg->inner_steps > 0) ? ((cfg->inner_steps + 3) & ~3) : kDefaultInner;
+    L.auto_inner = !(cfg && cfg->inner_steps > 0);
     L.steal = (cfg && cfg->steal < 0) ? 0 : 1;
     L.layout = (cfg && cfg->layout == NQ_LAYOUT_LANE_MAJOR) ? 1 : 0;
     return NQ_OK;
@@ -257,7 +264,18 @@ int enqueue_dfs(Ctx &c, DfsParams p, const Launch &L, bool per_owner, bool nodes
     p.steal = L.steal;
     p.layout = L.layout;
     NQ_CUDA(cudaMemsetAsync(p.ctl, 0, kCtlWords * sizeof(unsigned long long), s));
-    if (p.cta_times) NQ_CUDA(cudaMemsetAsync(p.cta_times, 0, 2 * (size_t)L.grid * sizeof(unsigned long long), s));
+    if (p.cta_times) {
+        NQ_CUDA(cudaMemsetAsync(p.cta_times, 0, 2 * (size_t)L.grid * sizeof(unsigned long long), s));
+        p.cta_wait = c.d_ctl + kWordBlocks + 4 * (size_t)c.sms * kMaxBlocksPerSm;
+        NQ_CUDA(cudaMemsetAsync(p.cta_wait, 0, (size_t)L.grid * sizeof(unsigned long long), s));
+    }
+    // rows left in the deepest task = its stack slots + the rows never stacked
+    if (L.levels + (nodes || L.dih ? 1 : 3) >= kMailRootRows) {
+        p.mail = c.d_mail;
+        p.mail_cap = kMailCap;
+    }
+    set_shares(p, (long long)L.grid * L.threads);
+    if (p.lg_coarse > 0 && L.auto_inner) p.inner = kShareInner;
     pick_kernel(per_owner, nodes, L.dih)<<<L.grid, L.threads, L.smem, s>>>(p);
     NQ_CUDA(cudaGetLastError());
     return NQ_OK;
@@ -296,6 +314,10 @@ int queue_len_of(const nq_config *cfg, int64_t n, long long &q) {
 }
 
 int status_from_bits(unsigned long long bits) {
+    if (bits & kStatMail) {
+        g_last_error = "internal error: a shared level was left behind";
+        return NQ_ERR_CUDA;
+    }
     if (bits & kStatDepth) {
         g_last_error = "a task needed more stack levels than the launch provided";
         return NQ_ERR_DEPTH;
@@ -319,15 +341,17 @@ int levels_for_tasks(int N, const uint32_t *cols, int64_t n, bool filtered) {
 }
 
 // Per-CTA start/end stamps -> makespan, mean busy time, idle fraction.
-int timing_stats(const unsigned long long *d_times, int grid, nq_stats *st) {
-    std::vector<unsigned long long> t(2 * (size_t)grid);
+int timing_stats(const unsigned long long *d_times, const unsigned long long *d_wait, int grid, int warps,
+                 nq_stats *st) {
+    std::vector<unsigned long long> t(2 * (size_t)grid), wait((size_t)grid);
     NQ_CUDA(cudaMemcpy(t.data(), d_times, t.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
+    NQ_CUDA(cudaMemcpy(wait.data(), d_wait, wait.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
     unsigned long long t0 = ~0ull, t1 = 0;
     double busy = 0;
     for (int b = 0; b < grid; ++b) {
         t0 = std::min(t0, t[2 * b]);
         t1 = std::max(t1, t[2 * b + 1]);
-        busy += (double)(t[2 * b + 1] - t[2 * b]);
+        busy += (double)(t[2 * b + 1] - t[2 * b]) - (double)wait[b] / warps;
     }
     const double span = (double)(t1 - t0);
     st->makespan_ms = span / 1e6;
@@ -426,7 +450,8 @@ int count_resident(Ctx &c, int N, const uint32_t *d_cols, const uint32_t *d_ld, 
     NQ_CUDA(cudaEventRecord(c.ev[3], c.stream));
     NQ_CUDA(cudaStreamSynchronize(c.stream));
     if (st && p.cta_times) {
-        rc = timing_stats(p.cta_times, L.grid, st);
+        rc = timing_stats(p.cta_times, c.d_ctl + kWordBlocks + 4 * (size_t)c.sms * kMaxBlocksPerSm, L.grid,
+                          L.threads / 32, st);
         if (rc) return rc;
     }
     if (st) {

@@ -30,12 +30,15 @@
 //    largest) stacked level of a busy lane in the same warp: __ballot_sync
 //    finds donors and receivers, __shfl_sync moves the donor's slot address,
 //    and the receiver loads the entry straight from the donor's stack.
+//  * A warp with nothing left takes levels from other warps through a mailbox
+//    in global memory (see "Mailbox").
 //  * Counts are uint32 per lane inside a bounded inner loop, folded into
 //    uint64 per lane, reduced per warp (shuffles) and per CTA, and the last
 //    CTA to finish sums the per-CTA partials in a fixed order.
 //
-// The kernel has no spin-wait of any kind: a lane never waits for another
-// CTA or for host memory.  An optional %globaltimer deadline bounds its run.
+// Only warps that have no work wait (for mail, with a time and a poll limit);
+// nothing else in the kernel depends on another CTA's progress.  An optional
+// %globaltimer deadline bounds its run.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -53,12 +56,28 @@ enum CtlWord : int {
     kCtlError = 2,     // error bits (kErr*)
     kCtlTimeout = 3,   // set when the deadline stopped the kernel
     kCtlCont = 4,      // continuation entries written at a deadline stop
-    kCtlWords = 5,
+    kCtlMail = 5,      // mailbox tickets: low half requested, high half supplied
+    kCtlWork = 6,      // signed: mail posted and not taken, minus warps out of work
+    kCtlWords = 7,
 };
 enum : unsigned long long { kErrDepth = 1ull, kErrContOverflow = 2ull };
 // Bits of *status_out: a task needed more stack levels than the launch had
 // (it was skipped), and/or the run-time limit stopped the kernel early.
-enum : unsigned long long { kStatDepth = 1ull, kStatTimeout = 2ull, kStatContOverflow = 4ull };
+enum : unsigned long long { kStatDepth = 1ull, kStatTimeout = 2ull, kStatContOverflow = 4ull, kStatMail = 8ull };
+
+// One slot of the mailbox through which busy warps hand stacked levels to warps
+// that ran out of work (see "Mailbox" below).
+constexpr int kMailLevels = 8;  // most levels of one slot
+struct alignas(256) MailSlot {
+    uint4 level[kMailLevels];      // (cols, ld, rd, avail) in the kernel's lane form
+    uint32_t owner[kMailLevels];   // per-owner output slots (PER_OWNER kernels)
+    uint32_t cls[kMailLevels];     // class indices (DIH kernels)
+    uint32_t count;
+    uint32_t state;                // use of the slot << 2 | kMail*
+    uint32_t pad[14];
+};
+static_assert(sizeof(MailSlot) == 256, "slot layout");
+enum : uint32_t { kMailEmpty = 0u, kMailFull = 1u, kMailGone = 2u, kMailDone = 3u };
 
 struct DfsParams {
     const uint32_t *cols;      // task column masks (reference `cur`)
@@ -70,6 +89,9 @@ struct DfsParams {
     long long ntasks;
     long long nqueue;          // queue positions to run (<= ntasks; 0 = ntasks)
     int N;                     // board size when task_n is nullptr
+    long long coarse;          // the first `coarse` tasks are queued as 2^lg_coarse shares of their
+    uint32_t lg_coarse;        // columns each, the others as 2^lg_fine (see set_shares in launch.h)
+    uint32_t lg_fine;
     int levels;                // stack slots per lane
     int inner;                 // DFS steps per outer trip (multiple of 4)
     int steal;                 // in-warp donation on/off
@@ -108,6 +130,12 @@ struct DfsParams {
     // (in) and of each saved level (out).
     const uint8_t *cont_in_cls;
     uint8_t *cont_out_cls;
+    // Mailbox (kernels without RESUME; nullptr switches it off).  Every slot is
+    // kMailEmpty at the start of a launch and again at its end.
+    MailSlot *mail;
+    uint32_t mail_cap;
+    // With cta_times: per-CTA sum over warps of the time spent waiting for mail.
+    unsigned long long *cta_wait;
 };
 
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
@@ -615,6 +643,192 @@ __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, u
     return 0;
 }
 
+// The columns of share `way` when a level's untried columns are dealt out in
+// 2^lg shares (by column number modulo 2^lg).
+__device__ __forceinline__ uint32_t share_mask(uint32_t lg, uint32_t way) {
+    uint32_t m = kFull;
+    if (lg > 0) m = 0x55555555u;
+    if (lg > 1) m = 0x11111111u;
+    if (lg > 2) m = 0x01010101u;
+    if (lg > 3) m = 0x00010001u;
+    if (lg > 4) m = 0x00000001u;
+    return m << way;
+}
+
+// ---------------------------------------------------------------------------
+// Mailbox: work sharing between warps once the queue is empty.
+//
+// A warp that is wholly out of work takes a ticket (kCtlMail, low half) and
+// watches the slot of that number.  A warp that has stacked levels and sees
+// more tickets requested than supplied claims a supply number (high half) and
+// posts up to kMailLevels of its lanes' bottom (shallowest, largest) levels
+// into that slot.  Slot i thus belongs to ticket i, whoever comes first.
+//
+// The slots are a ring of mail_cap (a power of two) entries: ticket t lives in
+// slot t % mail_cap as its (t / mail_cap)-th use, which the state word carries
+// above the kMail* value; its taker readies the slot for the next use.  A warp
+// holds one open ticket and claims one number at a time, so fewer than twice
+// the grid's warps are live at once, which is below mail_cap.
+//
+// kCtlWork counts, as a signed number, slots posted and not yet taken minus
+// warps out of work; with the grid's warps added it is the number of parties
+// that still hold work.  The warp that brings it to zero tells every waiting
+// ticket (kMailDone).  A post is counted before it is made and its taker counts
+// as working from then on, so the sum reaches zero only when nothing is left;
+// the last CTA checks that (kStatMail).
+//
+// What it is worth (with the queue's shares, launch.h): 512 boards of N=12..17
+// split three rows deep 177 -> 10.2 ms (30 ms without the mailbox: single
+// subtrees of 4.5e6 nodes sat in one warp), 8 % of N=21's prefixes (2.1 tasks
+// per lane) 911 -> 838 ms.  Levels with fewer than kMailMinRows rows left cost
+// more to hand over (a ticket, a post and a poll, about 3 us, then a warp that
+// starts with a few lanes) than they hold: with 10 instead of 12 the N=18 list
+// was 6 % slower.  For the same reason launches whose deepest task has fewer
+// than kMailRootRows rows left run without (60,001 prefixes of N=16, k=5: 0.60 ms
+// without, 0.82 with).
+//
+// No count depends on the waiting: a waiter only watches its own slot, gives
+// up after kMailPatienceNs (it marks the slot kMailGone, so the supplier keeps
+// its levels) and then just ends.  CTAs that have not started count as working
+// and, when they start, find the queue as any other warp does.
+constexpr unsigned long long kMailPatienceNs = 20ull * 1000 * 1000;
+constexpr int kMailPolls = 1 << 16;   // second limit on a wait, in polls
+constexpr int kMailRootRows = 13;      // rows left in the deepest task from which a launch uses the mailbox
+constexpr uint32_t kMailMinRows = 12;  // rows left below which a level is not worth posting
+constexpr uint32_t kGiveMinRows = 6;   // the same for a level given to a lane of the same warp
+constexpr int kShortTrip = 48;         // DFS steps of a warp with idle lanes before it looks again
+
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *a) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ MailSlot *mail_slot(const DfsParams &p, uint32_t t) {
+    return p.mail + (t & (p.mail_cap - 1u));
+}
+__device__ __forceinline__ uint32_t mail_tag(const DfsParams &p, uint32_t t, uint32_t st) {
+    return (t / p.mail_cap) << 2 | st;
+}
+
+// Counts this warp as out of work; the last one to be so ends every wait.
+// Returns true for that one.
+__device__ __forceinline__ bool out_of_work(const DfsParams &p, uint32_t lane) {
+    const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+    unsigned long long old = 0;
+    if (lane == 0) {
+        __threadfence();
+        old = atomicAdd(p.ctl + kCtlWork, ~0ull);
+        __threadfence();
+    }
+    old = __shfl_sync(kFull, old, 0);
+    if ((long long)old - 1 + nwarps != 0) return false;
+    const unsigned long long tk = *((volatile unsigned long long *)(p.ctl + kCtlMail));
+    const uint32_t req = (uint32_t)tk;
+    for (uint32_t i = (uint32_t)(tk >> 32) + lane; i < req; i += 32)
+        atomicCAS(&mail_slot(p, i)->state, mail_tag(p, i, kMailEmpty), mail_tag(p, i, kMailDone));
+    return true;
+}
+
+// For a warp that is out of work: takes a ticket and waits for its slot.  True:
+// the lanes hold the posted levels, each dealt out over several lanes by its
+// untried columns.  False: the warp is to end.
+template <bool DIH>
+__device__ __forceinline__ bool take_mail(const DfsParams &p, uint32_t lane, uint32_t &cols, uint32_t &ld,
+                                          uint32_t &rd, uint32_t &avail, uint32_t &owner, DihLane &dih) {
+    uint32_t t = 0, got = 0;
+    unsigned long long t0 = 0;
+    if (p.cta_times) t0 = globaltimer_ns();
+    if (lane == 0) t = (uint32_t)atomicAdd(p.ctl + kCtlMail, 1ull);
+    t = __shfl_sync(kFull, t, 0);
+    if (out_of_work(p, lane)) return false;
+    MailSlot *s = mail_slot(p, t);
+    const uint32_t none = mail_tag(p, t, kMailEmpty);
+    if (lane == 0) {
+        const unsigned long long until = globaltimer_ns() + kMailPatienceNs;
+        uint32_t st = none;
+        unsigned nap = 100;
+        for (int i = 0; i < kMailPolls; ++i) {
+            st = ld_acquire(&s->state);
+            if (st > none || globaltimer_ns() > until) break;
+            __nanosleep(nap);
+            nap = min(nap * 2, 1000u);
+        }
+        if (st <= none) st = atomicCAS(&s->state, none, none | kMailGone);
+        if (st == (none | kMailFull)) {
+            __threadfence();
+            got = __ldcg(&s->count);
+        }
+        if (p.cta_times) atomicAdd(p.cta_wait + blockIdx.x, globaltimer_ns() - t0);
+    }
+    got = __shfl_sync(kFull, got, 0);
+    __syncwarp();
+    if (got == 0) return false;
+    // got levels over 32 lanes: 2^lg lanes for each
+    const uint32_t lg = 31u - __clz(32u / got);
+    const uint32_t e = lane >> lg;
+    if (e < got) {
+        const uint4 v = __ldcg(s->level + e);
+        cols = v.x;
+        ld = v.y;
+        rd = v.z;
+        avail = v.w & share_mask(lg, lane & ((1u << lg) - 1u));
+        owner = avail ? __ldcg(s->owner + e) : kNoOwner;
+        if (DIH) load_class_index(p, __ldcg(s->cls + e), dih);
+    }
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) atomicExch(&s->state, none + 4u);  // ready for the slot's next use
+    return true;
+}
+
+// Offers this warp's shallowest stacked levels to a waiting warp; returns 1 in
+// the lanes whose bottom level is handed over (the caller then drops it).
+template <bool DIH>
+__device__ __forceinline__ uint32_t post_mail(const DfsParams &p, uint32_t lane, uint32_t sp, uint32_t bot,
+                                              uint32_t owner, uint32_t cls, bool &queue_live) {
+    const unsigned long long tk = *((volatile unsigned long long *)(p.ctl + kCtlMail));
+    const uint32_t req = __shfl_sync(kFull, (uint32_t)tk, 0), sup = __shfl_sync(kFull, (uint32_t)(tk >> 32), 0);
+    if (req) queue_live = false;  // a ticket is taken only when the queue is empty
+    if (req <= sup) return 0;
+    uint32_t x = kFull, y = 0, z = 0, w = 0;
+    if (sp != bot) lds128(bot, x, y, z, w);
+    const uint32_t rows = 32u - __popc(x);  // rows the level still has to place
+    const uint32_t most = __reduce_max_sync(kFull, rows);
+    if (most < kMailMinRows) return 0;
+    const unsigned give = __ballot_sync(kFull, rows + 1u >= most && rows >= kMailMinRows);
+    const uint32_t n = min((uint32_t)kMailLevels, ((uint32_t)__popc(give) + 1u) / 2u);
+    uint32_t t = 0;
+    if (lane == 0) {
+        t = (uint32_t)(atomicAdd(p.ctl + kCtlMail, 1ull << 32) >> 32);
+        atomicAdd(p.ctl + kCtlWork, 1ull);
+        __threadfence();
+    }
+    t = __shfl_sync(kFull, t, 0);
+    MailSlot *s = mail_slot(p, t);
+    const uint32_t none = mail_tag(p, t, kMailEmpty);
+    const uint32_t k = __popc(give & lanemask_lt());
+    const bool mine = (give >> lane & 1u) && k < n;
+    uint32_t posted = 0;
+    const uint32_t ready = __shfl_sync(kFull, ld_acquire(&s->state), 0) == none;
+    if (ready) {
+        if (mine) {
+            __stcg(s->level + k, make_uint4(x, y, z, w));
+            __stcg(s->owner + k, owner);
+            if (DIH) __stcg(s->cls + k, cls);
+        }
+        if (lane == 0) __stcg(&s->count, n);
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) posted = atomicCAS(&s->state, none, none | kMailFull) == none;
+        posted = __shfl_sync(kFull, posted, 0);
+    }
+    if (!posted && lane == 0) {
+        atomicCAS(&s->state, none | kMailGone, none + 4u);
+        atomicAdd(p.ctl + kCtlWork, ~0ull);
+    }
+    return posted && mine ? 1u : 0u;
+}
+
 // RESUME adds the continuation queue and the deadline dump; it is a separate
 // instantiation so that the plain count kernel carries none of that code
 // (it measurably changed the code generated for the DFS loop).
@@ -627,6 +841,7 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
     // Lane registers and task loading of the step: the dihedral filtered step
     // keeps VAR 3's lane form and steps rows N-2 and N-1 (no settling).
     constexpr int LVAR = (DIH && VAR == 4) ? 3 : VAR;
+    constexpr bool MAIL = !RESUME;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned long long red_cnt[32];
     __shared__ unsigned long long red_nodes[32];
@@ -651,8 +866,11 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
     uint32_t owner = kNoOwner;
     DihLane dih;
     unsigned long long tot = 0, tot_nodes = 0;
-    const long long qlen = RESUME ? p.n_cont_in + p.ntasks - p.task_base : (p.nqueue > 0 ? p.nqueue : p.ntasks);
+    const long long qlen = RESUME ? p.n_cont_in + p.ntasks - p.task_base
+                                  : (p.coarse << p.lg_coarse) +
+                                        (((p.nqueue > 0 ? p.nqueue : p.ntasks) - p.coarse) << p.lg_fine);
     bool queue_live = qlen > 0;
+    unsigned looks = 0;           // trips, for the looks at the mailbox
     bool timed_out = false;
     unsigned long long deadline = 0;
     if (p.limit_ns) {
@@ -688,6 +906,7 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
             if (now > deadline) {
                 if (lane == 0) atomicExch(p.ctl + kCtlTimeout, 1ull);
                 if (RESUME) timed_out = true;
+                if (MAIL && p.mail && p.steal) out_of_work(p, lane);
                 break;
             }
         }
@@ -724,8 +943,17 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                             if (PER_OWNER && avail) owner = p.cont_in_owner ? p.cont_in_owner[q] : 0u;
                         }
                     } else if (q < (unsigned long long)qlen) {
-                        const long long pos =
-                            RESUME ? p.task_base + (long long)(q - (unsigned long long)p.n_cont_in) : (long long)q;
+                        long long pos = (long long)q;
+                        uint32_t way = 0, lg = 0;
+                        if (RESUME) {
+                            pos = p.task_base + (long long)(q - (unsigned long long)p.n_cont_in);
+                        } else {
+                            const long long fine = pos - (p.coarse << p.lg_coarse);
+                            lg = fine < 0 ? p.lg_coarse : p.lg_fine;
+                            if (fine >= 0) pos = fine;
+                            way = (uint32_t)pos & ((1u << lg) - 1u);
+                            pos = (pos >> lg) + (fine < 0 ? 0 : p.coarse);
+                        }
                         const long long t = p.order ? (long long)__ldg(p.order + pos) : pos;
                         // A permutation entry out of range is skipped, never dereferenced.
                         if (t >= 0 && t < p.ntasks) {
@@ -738,6 +966,11 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                                 // (the step applies them to children only).
                                 const uint32_t pc = (uint32_t)__popc(cols);
                                 if (avail && pc > dih.side_popc) avail &= pc == 31u ? dih.last_mask : p.noside;
+                            }
+                            if (!RESUME) {
+                                // this lane's share of the task's columns
+                                avail &= share_mask(lg, way);
+                                if (way) done = 0;
                             }
                             const uint32_t own = p.owner_of ? __ldg(p.owner_of + t) : (uint32_t)t;
                             if (PER_OWNER) {
@@ -753,53 +986,64 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                 idle = __ballot_sync(kFull, avail == 0);
             }
             if (idle && !queue_live) {
-                if (p.steal) {
-                    // ---- in-warp donation: k-th idle lane takes the bottom
-                    // stacked level of the k-th lane that has one.
-                    const unsigned rich = __ballot_sync(kFull, sp != bot);
-                    __syncwarp();  // order the donors' earlier stack stores before the reads below
-                    const int npair = min(__popc(idle), __popc(rich));
-                    if (npair > 0) {
-                        int donor = -1;
-                        if (avail == 0) {
-                            const int k = __popc(idle & lanemask_lt());
-                            if (k < npair) {
-                                unsigned m = rich;
-                                for (int i = 0; i < k; ++i) m &= m - 1;
-                                donor = __ffs(m) - 1;
-                            }
+                // ---- in-warp donation: k-th idle lane takes the bottom
+                // stacked level of the k-th lane that has one worth it.
+                uint32_t low = kFull;
+                if (sp != bot) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(low) : "r"(bot) : "memory");
+                const bool has = 32u - __popc(low) >= kGiveMinRows;
+                const unsigned rich = p.steal ? __ballot_sync(kFull, has) : 0u;
+                __syncwarp();  // order the donors' earlier stack stores before the reads below
+                const int npair = min(__popc(idle), __popc(rich));
+                if (npair > 0) {
+                    int donor = -1;
+                    if (avail == 0) {
+                        const int k = __popc(idle & lanemask_lt());
+                        if (k < npair) {
+                            unsigned m = rich;
+                            for (int i = 0; i < k; ++i) m &= m - 1;
+                            donor = __ffs(m) - 1;
                         }
-                        const uint32_t src_addr = __shfl_sync(kFull, bot, donor < 0 ? lane : donor);
-                        const uint32_t src_owner = __shfl_sync(kFull, owner, donor < 0 ? lane : donor);
-                        DihLane src_dih;
-                        if (DIH) {
-                            const int src = donor < 0 ? (int)lane : donor;
-                            src_dih.side_popc = __shfl_sync(kFull, dih.side_popc, src);
-                            src_dih.last_mask = __shfl_sync(kFull, dih.last_mask, src);
-                            src_dih.tie_bit = __shfl_sync(kFull, dih.tie_bit, src);
-                            src_dih.w = __shfl_sync(kFull, dih.w, src);
-                            src_dih.w_tie = __shfl_sync(kFull, dih.w_tie, src);
-                            if (RESUME) src_dih.cls = __shfl_sync(kFull, dih.cls, src);
-                        }
-                        if (donor >= 0) {
-                            lds128(src_addr, cols, ld, rd, avail);
-                            sp = bot = my_base;
-                            owner = src_owner;
-                            if (DIH) dih = src_dih;
-                        }
-                        __syncwarp();
-                        if (sp != bot && __popc(rich & lanemask_lt()) < npair) bot += stride;
-                        __syncwarp();
-                    } else {
-                        // Nobody can donate right now: run a full trip
-                        // without idle checks, then look again.
-                        if (idle == kFull) break;  // whole warp idle, queue empty: done
-                        check_idle = false;
                     }
+                    const uint32_t src_addr = __shfl_sync(kFull, bot, donor < 0 ? lane : donor);
+                    const uint32_t src_owner = __shfl_sync(kFull, owner, donor < 0 ? lane : donor);
+                    DihLane src_dih;
+                    if (DIH) {
+                        const int src = donor < 0 ? (int)lane : donor;
+                        src_dih.side_popc = __shfl_sync(kFull, dih.side_popc, src);
+                        src_dih.last_mask = __shfl_sync(kFull, dih.last_mask, src);
+                        src_dih.tie_bit = __shfl_sync(kFull, dih.tie_bit, src);
+                        src_dih.w = __shfl_sync(kFull, dih.w, src);
+                        src_dih.w_tie = __shfl_sync(kFull, dih.w_tie, src);
+                        src_dih.cls = __shfl_sync(kFull, dih.cls, src);
+                    }
+                    if (donor >= 0) {
+                        lds128(src_addr, cols, ld, rd, avail);
+                        sp = bot = my_base;
+                        owner = src_owner;
+                        if (DIH) dih = src_dih;
+                    }
+                    __syncwarp();
+                    if (has && __popc(rich & lanemask_lt()) < npair) bot += stride;
+                    __syncwarp();
+                    check_idle = npair == __popc(idle);
+                } else if (idle == kFull) {
+                    // whole warp idle, queue empty
+                    if (!MAIL || !p.mail || !p.steal) break;
+                    if (!take_mail<DIH>(p, lane, cols, ld, rd, avail, owner, dih)) break;
+                    sp = bot = my_base;
+                    check_idle = false;
                 } else {
-                    if (idle == kFull) break;
                     check_idle = false;
                 }
+            }
+        }
+        // Other warps may be out of work (and the queue empty): offer them
+        // stacked levels.
+        if (MAIL && p.mail && p.steal) {
+            looks += check_idle ? 4u : 1u;
+            if (looks >= 4u) {
+                looks = 0;
+                bot += stride * post_mail<DIH>(p, lane, sp, bot, owner, dih.cls, queue_live);
             }
         }
 
@@ -820,7 +1064,7 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                 if (__any_sync(kFull, avail == 0)) break;
             }
         } else {
-            for (int s = 0; s < p.inner; s += UNROLL) {
+            for (int s = 0; s < kShortTrip; s += UNROLL) {
 #pragma unroll
                 for (int u = 0; u < (VAR >= 3 && !DIH ? 1 : UNROLL); ++u) {
                     if constexpr (DIH)
@@ -901,9 +1145,15 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
         s_is_last = (ticket == (unsigned long long)gridDim.x - 1ull);
     }
     __syncthreads();
-    // ---- the last CTA sums the per-CTA partials in CTA order
+    // ---- the last CTA empties the mailbox for the next launch and sums the
+    // per-CTA partials in CTA order
     if (s_is_last) {
         __threadfence();
+        if (MAIL && p.mail) {
+            const unsigned long long tk = *((volatile unsigned long long *)(p.ctl + kCtlMail));
+            const uint32_t used = min(p.mail_cap, max((uint32_t)tk, (uint32_t)(tk >> 32)));
+            for (uint32_t i = threadIdx.x; i < used; i += blockDim.x) p.mail[i].state = kMailEmpty;
+        }
         unsigned long long s = 0, sn = 0;
         for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
             s += *((volatile unsigned long long *)(p.block_cnt + b));
@@ -930,8 +1180,12 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
             if (NODES) *p.nodes_out = an;
             const unsigned long long err = *((volatile unsigned long long *)(p.ctl + kCtlError));
             const unsigned long long tmo = *((volatile unsigned long long *)(p.ctl + kCtlTimeout));
+            // Every warp is out of work and no posted level was left behind.
+            const bool mail_ok = !MAIL || !p.mail || !p.steal || tmo ||
+                                 (long long)*((volatile unsigned long long *)(p.ctl + kCtlWork)) +
+                                         (long long)gridDim.x * (blockDim.x >> 5) == 0;
             *p.status_out = ((err & kErrDepth) ? kStatDepth : 0ull) | (tmo ? kStatTimeout : 0ull) |
-                            ((err & kErrContOverflow) ? kStatContOverflow : 0ull);
+                            ((err & kErrContOverflow) ? kStatContOverflow : 0ull) | (mail_ok ? 0ull : kStatMail);
         }
     }
 }

@@ -73,4 +73,31 @@ int resident_warp_threads(Kernel fn, int levels, int smem_optin, int cap_per_sm)
     return best;
 }
 
+// DFS steps between visits to the queue where tasks are dealt out in shares and
+// the caller names none: such runs last a few hundred microseconds to
+// milliseconds, so a warp must notice soon that others are out of work (1024
+// steps are 60-190 us).
+constexpr int kShareInner = 256;
+
+// How the queue hands out tasks: the first `coarse` tasks as 2^lg_coarse shares
+// of their root level's columns each (share_mask), the others as 2^lg_fine.
+// A lane runs a share by itself (until the queue is empty), so a share must be
+// short against the whole run: below 8 positions per lane the tasks are dealt
+// out finer, and the last ones always are.  Sixteen shares only where eight do
+// not give every lane one; half of them are empty (a level rarely has more than
+// eight alive columns), and an empty share still costs a visit to the queue.
+// Measured: 60,001 prefixes of N=16, k=5 (0.23 per lane) 0.96 ms whole, 0.60 in
+// shares; 1501 prefixes of N=13, k=4 0.19 -> 0.13 ms per call; 1.1e6 prefixes of
+// N=18 (4.8 per lane) 18.8 ms with the line at 16 per lane, 18.5 at 8, 18.6 at 4.
+inline void set_shares(DfsParams &p, long long lanes) {
+    const long long n = p.nqueue > 0 ? p.nqueue : p.ntasks;
+    p.coarse = n;
+    p.lg_coarse = p.lg_fine = 0;
+    if (!p.steal) return;
+    p.lg_fine = (n << 3) < lanes ? 4 : 3;
+    while (p.lg_coarse < p.lg_fine && (n << p.lg_coarse) < 8 * lanes) ++p.lg_coarse;
+    const long long m = (2 * lanes) >> p.lg_fine;
+    p.coarse = n > m ? n - m : 0;
+}
+
 }  // namespace nqb

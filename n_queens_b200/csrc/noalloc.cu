@@ -43,7 +43,7 @@ int status_of_exception() noexcept;
 namespace {
 
 constexpr int kNoAllocMaxCtas = 8192;
-constexpr int kNoAllocWords = 8 + kNoAllocMaxCtas;  // control + results + per-CTA partials
+constexpr int kNoAllocWords = 16 + kNoAllocMaxCtas;  // control + results + per-CTA partials
 constexpr int kNoAllocMaxDevices = 64;
 constexpr int kNoAllocMaxBlocksPerSm = 32;
 
@@ -223,15 +223,18 @@ extern "C" int nq_count_tasks_device_noalloc(int N, const uint32_t *d_cols, cons
     p.layout = (cfg && cfg->layout == NQ_LAYOUT_LANE_MAJOR) ? 1 : 0;
     p.limit_ns = cfg ? (unsigned long long)cfg->time_limit_ms * 1000000ull : 0ull;
     p.order = (cfg && cfg->order_kind == NQ_ORDER_GIVEN) ? cfg->order : nullptr;
-    p.ctl = d.scratch;  // words 0..4: queue head, CTAs done, error bits, timeout flag, continuation count
-    p.block_cnt = d.scratch + 8;
-    p.block_nodes = d.scratch + 8;  // unused: this variant counts no nodes
+    p.ctl = d.scratch;  // words 0..6, the control words
+    p.block_cnt = d.scratch + 16;
+    p.block_nodes = d.scratch + 16;  // unused: this variant counts no nodes
     p.sum_out = (unsigned long long *)d_sum;
-    p.nodes_out = d.scratch + 5;
+    p.nodes_out = d.scratch + 8;
     p.status_out = (unsigned long long *)d_sum + 1;
     p.k_one = 1;
     p.k_two = 2;
     p.k_mone = 0xffffffffu;
+
+    set_shares(p, (long long)grid * threads);
+    if (p.lg_coarse > 0 && !(cfg && cfg->inner_steps > 0)) p.inner = kShareInner;
 
     cudaStream_t s = (cudaStream_t)stream;
     // The previous call left its control words behind (queue head, done
