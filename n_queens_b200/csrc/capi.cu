@@ -107,6 +107,13 @@ struct HostBuf {
     }
 };
 
+// The default CTA size and its resident CTAs per SM of one kernel and stack
+// depth.  They depend on nothing else, and finding them takes some 16 occupancy
+// queries, about 20 us of a small call.
+struct Shape {
+    int threads = 0, per_sm = 0;
+};
+
 struct Ctx {
     std::mutex mu;
     bool ready = false;
@@ -121,6 +128,8 @@ struct Ctx {
     DevBuf aux;                           // order, owners, task_n, per-task outputs
     HostBuf h_tasks;                      // pinned staging for the expander
     DevBuf expand_scratch;                // seeds, counts, offsets of the device expander
+    HostBuf h_out;                        // pinned staging of small results
+    Shape shapes[2][2][2][NQ_MAX_STACK_LEVELS + 1];  // [per_owner][nodes][dih][levels]
 };
 
 Ctx g_ctx[kMaxDevices];
@@ -211,32 +220,41 @@ int plan_launch(Ctx &c, const nq_config *cfg, int levels_needed, bool per_owner,
     }
     const int cap_per_sm = (cfg && cfg->blocks_per_sm > 0) ? std::min(cfg->blocks_per_sm, kMaxBlocksPerSm)
                                                            : kMaxBlocksPerSm;
-    L.threads = (cfg && cfg->block_threads)
-                    ? cfg->block_threads
-                    : resident_warp_threads(pick_kernel(per_owner, nodes, dih), L.levels, c.smem_optin, cap_per_sm);
-    if (!(cfg && cfg->block_threads) && L.threads == 0) {
-        g_last_error = "no CTA size of 64 or more threads fits this stack depth in shared memory";
-        return NQ_ERR_DEPTH;
-    }
-    if (L.threads < 32 || L.threads > 1024 || (L.threads & 31)) {
-        g_last_error = "block_threads must be a multiple of 32 in [32, 1024]";
-        return NQ_ERR_ARG;
-    }
-    const long long smem = (long long)(L.threads / 32) * L.levels * kSlotBytes;
-    if (smem + kDfsStaticSmem > c.smem_optin) {
-        g_last_error = "per-CTA stack does not fit in shared memory: lower block_threads";
-        return NQ_ERR_DEPTH;
-    }
-    L.smem = (int)smem;
+    const bool plain = !(cfg && (cfg->block_threads || cfg->blocks_per_sm > 0)) && L.levels <= NQ_MAX_STACK_LEVELS;
+    Shape *known = plain ? &c.shapes[per_owner][nodes][dih][L.levels] : nullptr;
     int per_sm = 0;
-    NQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_kernel(per_owner, nodes, dih),
-                                                          L.threads, L.smem));
-    if (per_sm <= 0) {
-        g_last_error = "launch configuration cannot be resident";
-        return NQ_ERR_ARG;
+    if (known && known->threads) {
+        L.threads = known->threads;
+        per_sm = known->per_sm;
+        L.smem = (L.threads / 32) * L.levels * (int)kSlotBytes;
+    } else {
+        L.threads = (cfg && cfg->block_threads)
+                        ? cfg->block_threads
+                        : resident_warp_threads(pick_kernel(per_owner, nodes, dih), L.levels, c.smem_optin, cap_per_sm);
+        if (!(cfg && cfg->block_threads) && L.threads == 0) {
+            g_last_error = "no CTA size of 64 or more threads fits this stack depth in shared memory";
+            return NQ_ERR_DEPTH;
+        }
+        if (L.threads < 32 || L.threads > 1024 || (L.threads & 31)) {
+            g_last_error = "block_threads must be a multiple of 32 in [32, 1024]";
+            return NQ_ERR_ARG;
+        }
+        const long long smem = (long long)(L.threads / 32) * L.levels * kSlotBytes;
+        if (smem + kDfsStaticSmem > c.smem_optin) {
+            g_last_error = "per-CTA stack does not fit in shared memory: lower block_threads";
+            return NQ_ERR_DEPTH;
+        }
+        L.smem = (int)smem;
+        NQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_kernel(per_owner, nodes, dih),
+                                                              L.threads, L.smem));
+        if (per_sm <= 0) {
+            g_last_error = "launch configuration cannot be resident";
+            return NQ_ERR_ARG;
+        }
+        per_sm = std::min(per_sm, kMaxBlocksPerSm);
+        if (cfg && cfg->blocks_per_sm > 0) per_sm = std::min(per_sm, cfg->blocks_per_sm);
+        if (known) *known = Shape{L.threads, per_sm};
     }
-    per_sm = std::min(per_sm, kMaxBlocksPerSm);
-    if (cfg && cfg->blocks_per_sm > 0) per_sm = std::min(per_sm, cfg->blocks_per_sm);
     L.grid = c.sms * per_sm;
     if (cfg && cfg->inner_steps > NQ_MAX_INNER_STEPS) {
         g_last_error = "inner_steps is above NQ_MAX_INNER_STEPS";
@@ -360,6 +378,11 @@ int timing_stats(const unsigned long long *d_times, const unsigned long long *d_
     return NQ_OK;
 }
 
+// Transfers of at most this many bytes go through pinned staging: a copy from or
+// to pageable memory waits for the device by itself, which costs a small call
+// more than the extra memcpy.
+constexpr size_t kStageBytes = 1 << 20;
+
 // Counts tasks that are already in device memory (d_cols, d_ld, d_rd) and
 // downloads the results.  Used by nq_count and nq_count_tasks.
 // Class data of a dihedral launch (device pointers).
@@ -441,14 +464,20 @@ int count_resident(Ctx &c, int N, const uint32_t *d_cols, const uint32_t *d_ld, 
     rc = enqueue_dfs(c, p, L, per_owner, nodes, c.stream);
     if (rc) return rc;
     NQ_CUDA(cudaEventRecord(c.ev[2], c.stream));
-    unsigned long long res[3] = {0, 0, 0};
-    NQ_CUDA(cudaMemcpyAsync(res, c.d_ctl + kWordSum, sizeof(res), cudaMemcpyDeviceToHost, c.stream));
-    if (per_owner && h_per_task)
-        NQ_CUDA(cudaMemcpyAsync(h_per_task, p.out_cnt, (size_t)n * 8, cudaMemcpyDeviceToHost, c.stream));
-    if (per_owner && nodes && h_nodes_task)
-        NQ_CUDA(cudaMemcpyAsync(h_nodes_task, p.out_nodes, (size_t)n * 8, cudaMemcpyDeviceToHost, c.stream));
+    const bool want_cnt = per_owner && h_per_task, want_nodes = per_owner && nodes && h_nodes_task;
+    const bool staged = ((size_t)want_cnt + want_nodes) * (size_t)n * 8 <= kStageBytes;
+    rc = c.h_out.grow(64 + (staged ? 2 * (size_t)n * 8 : 0));
+    if (rc) return rc;
+    unsigned long long *res = (unsigned long long *)c.h_out.p;
+    uint64_t *to_cnt = staged ? (uint64_t *)res + 8 : h_per_task;
+    uint64_t *to_nodes = staged ? (uint64_t *)res + 8 + n : h_nodes_task;
+    NQ_CUDA(cudaMemcpyAsync(res, c.d_ctl + kWordSum, 3 * sizeof(*res), cudaMemcpyDeviceToHost, c.stream));
+    if (want_cnt) NQ_CUDA(cudaMemcpyAsync(to_cnt, p.out_cnt, (size_t)n * 8, cudaMemcpyDeviceToHost, c.stream));
+    if (want_nodes) NQ_CUDA(cudaMemcpyAsync(to_nodes, p.out_nodes, (size_t)n * 8, cudaMemcpyDeviceToHost, c.stream));
     NQ_CUDA(cudaEventRecord(c.ev[3], c.stream));
     NQ_CUDA(cudaStreamSynchronize(c.stream));
+    if (staged && want_cnt) memcpy(h_per_task, to_cnt, (size_t)n * 8);
+    if (staged && want_nodes) memcpy(h_nodes_task, to_nodes, (size_t)n * 8);
     if (st && p.cta_times) {
         rc = timing_stats(p.cta_times, c.d_ctl + kWordBlocks + 4 * (size_t)c.sms * kMaxBlocksPerSm, L.grid,
                           L.threads / 32, st);
@@ -608,28 +637,6 @@ int write_checkpoint(const char *path, const Checkpoint &ck) {
 
 constexpr int kDefaultSplit = 3;
 
-}  // namespace
-}  // namespace nqb
-
-// A batch plan: the deduplicated, split and uploaded subtasks of a set of
-// partial boards, and a CUDA graph that resets the queue, counts and copies
-// the results back.
-struct nq_batch {
-    int device = 0;
-    int64_t n_inst = 0, n_unique = 0, m_tasks = 0;
-    std::vector<int64_t> inst_to_u;
-    void *d_buf = nullptr;                 // tasks (cols | ld | rd | owner u32, task_n u8) + results
-    unsigned long long *h_res = nullptr;   // pinned: [sum, nodes, status, 2 words per unique board]
-    unsigned long long *d_out = nullptr;   // 2 words per unique board: weight-1 and weight-2 sums
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    nqb::Launch L;
-    int levels = 0;
-};
-
-namespace nqb {
-namespace {
-
 // Reverses the low N bits (column j -> N-1-j).
 uint32_t rev_bits(uint32_t x, int N) {
     uint32_t y = 0;
@@ -703,19 +710,58 @@ void split_board(const Board &b, int rows, bool symmetric, std::vector<uint32_t>
     }
 }
 
-void destroy_batch(nq_batch &b) {
-    if (b.exec) cudaGraphExecDestroy(b.exec);
-    if (b.graph) cudaGraphDestroy(b.graph);
-    if (b.d_buf) cudaFree(b.d_buf);
-    if (b.h_res) cudaFreeHost(b.h_res);
-    b.exec = nullptr;
-    b.graph = nullptr;
-    b.d_buf = nullptr;
-    b.h_res = nullptr;
+// The host part of a batch: its distinct boards and their subtasks.
+struct BatchTasks {
+    int64_t n_inst = 0, n_unique = 0;
+    std::vector<int64_t> inst_to_u;
+    std::vector<uint32_t> tc, tl, tr, own;  // subtasks and their owners (2u + (weight == 2))
+    std::vector<uint8_t> tn;                // board size of each subtask
+    int levels = 1;
+
+    size_t task_bytes() const { return (tc.size() * 17 + 255) & ~(size_t)255; }
+    size_t out_bytes() const { return (size_t)n_unique * 2 * 8; }
+    // Lays the subtasks out as the launch reads them: cols | ld | rd | owner (u32), N (u8).
+    void write(void *to) const {
+        const size_t m = tc.size();
+        uint32_t *d = (uint32_t *)to;
+        memcpy(d, tc.data(), m * 4);
+        memcpy(d + m, tl.data(), m * 4);
+        memcpy(d + 2 * m, tr.data(), m * 4);
+        memcpy(d + 3 * m, own.data(), m * 4);
+        memcpy(d + 4 * m, tn.data(), m);
+    }
+    // Launch parameters over that layout in device memory, sums to d_out.
+    DfsParams params(Ctx &c, const nq_config *cfg, const void *d_tasks, unsigned long long *d_out) const {
+        const int64_t m = (int64_t)tc.size();
+        const uint32_t *d = (const uint32_t *)d_tasks;
+        DfsParams p = base_params(c, 0, m, cfg);
+        p.cols = d;
+        p.ld = d + m;
+        p.rd = d + 2 * m;
+        p.owner_of = d + 3 * m;
+        p.task_n = (const uint8_t *)(d + 4 * m);
+        p.out_cnt = d_out;
+        p.cta_times = nullptr;
+        return p;
+    }
+    // Per-instance counts from the per-owner sums.
+    void gather(const unsigned long long *sums, uint64_t *out) const {
+        for (int64_t i = 0; i < n_inst; ++i) {
+            const int64_t u = inst_to_u[i];
+            out[i] = sums[2 * u] + 2 * sums[2 * u + 1];
+        }
+    }
+};
+
+int check_instances(const nq_instance *inst, int64_t n, int split_rows) {
+    if (n < 0 || (n > 0 && !inst) || split_rows < 0 || split_rows > 8) return NQ_ERR_ARG;
+    if (n > 0x7fffffffll) return NQ_ERR_ARG;
+    for (int64_t i = 0; i < n; ++i)
+        if (inst[i].N < 1 || inst[i].N > NQ_MAX_N) return NQ_ERR_ARG;
+    return NQ_OK;
 }
 
-int build_batch(Ctx &c, const nq_instance *inst, int64_t n, int split, const nq_config *cfg, nq_batch &B) {
-    B.device = device_of(cfg);
+void batch_tasks(const nq_instance *inst, int64_t n, int split, BatchTasks &B) {
     B.n_inst = n;
     B.inst_to_u.resize((size_t)n);
     // 1. exact dedup: identical boards, and boards equal up to mirror image
@@ -738,8 +784,8 @@ int build_batch(Ctx &c, const nq_instance *inst, int64_t n, int split, const nq_
     }
     B.n_unique = (int64_t)uniq.size();
     // 2. split every distinct board; owner = 2u + (weight == 2)
-    std::vector<uint32_t> tc, tl, tr, own;
-    std::vector<uint8_t> tw, tn;
+    std::vector<uint32_t> &tc = B.tc, &tl = B.tl, &tr = B.tr, &own = B.own;
+    std::vector<uint8_t> tw, &tn = B.tn;
     int need = 1;
     for (int64_t u = 0; u < B.n_unique; ++u) {
         const Board &b = uniq[u];
@@ -754,34 +800,63 @@ int build_batch(Ctx &c, const nq_instance *inst, int64_t n, int split, const nq_
                 need = std::max(need, stack_need(b.N, __builtin_popcount(tc[k]), true));
         }
     }
-    const int64_t m = (int64_t)tc.size();
-    B.m_tasks = m;
     B.levels = need;
-    int rc = plan_launch(c, cfg, need, true, false, B.L);
+}
+
+}  // namespace
+}  // namespace nqb
+
+// A batch plan: the deduplicated, split and uploaded subtasks of a set of
+// partial boards, and a CUDA graph that resets the queue, counts and copies
+// the results back.
+struct nq_batch {
+    int device = 0;
+    int64_t m_tasks = 0;
+    nqb::BatchTasks t;                     // (its subtask arrays are dropped once uploaded)
+    void *d_buf = nullptr;                 // tasks (cols | ld | rd | owner u32, task_n u8) + results
+    unsigned long long *h_res = nullptr;   // pinned: [sum, nodes, status, 2 words per unique board]
+    unsigned long long *d_out = nullptr;   // 2 words per unique board: weight-1 and weight-2 sums
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    nqb::Launch L;
+};
+
+namespace nqb {
+namespace {
+
+void destroy_batch(nq_batch &b) {
+    if (b.exec) cudaGraphExecDestroy(b.exec);
+    if (b.graph) cudaGraphDestroy(b.graph);
+    if (b.d_buf) cudaFree(b.d_buf);
+    if (b.h_res) cudaFreeHost(b.h_res);
+    b.exec = nullptr;
+    b.graph = nullptr;
+    b.d_buf = nullptr;
+    b.h_res = nullptr;
+}
+
+int build_batch(Ctx &c, const nq_instance *inst, int64_t n, int split, const nq_config *cfg, nq_batch &B) {
+    B.device = device_of(cfg);
+    batch_tasks(inst, n, split, B.t);
+    const int64_t m = (int64_t)B.t.tc.size();
+    B.m_tasks = m;
+    int rc = plan_launch(c, cfg, B.t.levels, true, false, B.L);
     if (rc) return rc;
     // 3. device buffer: tasks, owners, sizes, per-owner sums
-    const size_t task_bytes = ((size_t)m * 17 + 255) & ~(size_t)255;
-    const size_t out_bytes = (size_t)B.n_unique * 2 * 8;
+    const size_t task_bytes = B.t.task_bytes(), out_bytes = B.t.out_bytes();
     NQ_CUDA(cudaMalloc(&B.d_buf, task_bytes + out_bytes + 256));
-    NQ_CUDA(cudaHostAlloc((void **)&B.h_res, (3 + 2 * (size_t)B.n_unique) * 8, cudaHostAllocDefault));
-    uint32_t *d = (uint32_t *)B.d_buf;
+    NQ_CUDA(cudaHostAlloc((void **)&B.h_res, 24 + out_bytes, cudaHostAllocDefault));
     B.d_out = (unsigned long long *)((char *)B.d_buf + task_bytes);
     if (m) {
-        NQ_CUDA(cudaMemcpyAsync(d, tc.data(), (size_t)m * 4, cudaMemcpyHostToDevice, c.stream));
-        NQ_CUDA(cudaMemcpyAsync(d + m, tl.data(), (size_t)m * 4, cudaMemcpyHostToDevice, c.stream));
-        NQ_CUDA(cudaMemcpyAsync(d + 2 * m, tr.data(), (size_t)m * 4, cudaMemcpyHostToDevice, c.stream));
-        NQ_CUDA(cudaMemcpyAsync(d + 3 * m, own.data(), (size_t)m * 4, cudaMemcpyHostToDevice, c.stream));
-        NQ_CUDA(cudaMemcpyAsync(d + 4 * m, tn.data(), (size_t)m, cudaMemcpyHostToDevice, c.stream));
+        rc = c.h_tasks.grow((size_t)m * 17);
+        if (rc) return rc;
+        B.t.write(c.h_tasks.p);
+        NQ_CUDA(cudaMemcpyAsync(B.d_buf, c.h_tasks.p, (size_t)m * 17, cudaMemcpyHostToDevice, c.stream));
     }
     NQ_CUDA(cudaStreamSynchronize(c.stream));
-    DfsParams p = base_params(c, 0, m, cfg);
-    p.cols = d;
-    p.ld = d + m;
-    p.rd = d + 2 * m;
-    p.owner_of = d + 3 * m;
-    p.task_n = (const uint8_t *)(d + 4 * m);
-    p.out_cnt = B.d_out;
-    p.cta_times = nullptr;
+    const DfsParams p = B.t.params(c, cfg, B.d_buf, B.d_out);
+    for (auto *v : {&B.t.tc, &B.t.tl, &B.t.tr, &B.t.own}) std::vector<uint32_t>().swap(*v);  // uploaded
+    std::vector<uint8_t>().swap(B.t.tn);
     // 4. one graph: reset, count, copy back (result words and per-owner sums)
     NQ_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = cudaMemsetAsync(B.d_out, 0, out_bytes, c.stream);
@@ -1333,9 +1408,19 @@ int nq_count_tasks(int N, const uint32_t *cols, const uint32_t *ld, const uint32
     if (rc) return rc;
     uint32_t *d = (uint32_t *)c.tasks.p;
     NQ_CUDA(cudaEventRecord(c.ev[0], c.stream));
-    NQ_CUDA(cudaMemcpyAsync(d, cols, (size_t)n * 4, cudaMemcpyHostToDevice, c.stream));
-    NQ_CUDA(cudaMemcpyAsync(d + n, ld, (size_t)n * 4, cudaMemcpyHostToDevice, c.stream));
-    NQ_CUDA(cudaMemcpyAsync(d + 2 * n, rd, (size_t)n * 4, cudaMemcpyHostToDevice, c.stream));
+    if ((size_t)n * 12 <= kStageBytes) {
+        rc = c.h_tasks.grow((size_t)n * 12);
+        if (rc) return rc;
+        uint32_t *h = (uint32_t *)c.h_tasks.p;
+        memcpy(h, cols, (size_t)n * 4);
+        memcpy(h + n, ld, (size_t)n * 4);
+        memcpy(h + 2 * n, rd, (size_t)n * 4);
+        NQ_CUDA(cudaMemcpyAsync(d, h, (size_t)n * 12, cudaMemcpyHostToDevice, c.stream));
+    } else {
+        NQ_CUDA(cudaMemcpyAsync(d, cols, (size_t)n * 4, cudaMemcpyHostToDevice, c.stream));
+        NQ_CUDA(cudaMemcpyAsync(d + n, ld, (size_t)n * 4, cudaMemcpyHostToDevice, c.stream));
+        NQ_CUDA(cudaMemcpyAsync(d + 2 * n, rd, (size_t)n * 4, cudaMemcpyHostToDevice, c.stream));
+    }
     const bool per_owner = per_task != nullptr || nodes_per_task != nullptr;
     const bool want_nodes = nodes_per_task != nullptr;
     std::vector<uint64_t> tmp;
@@ -1402,12 +1487,10 @@ int nq_count_tasks_device(int N, const uint32_t *d_cols, const uint32_t *d_ld, c
 int nq_batch_create(const nq_instance *inst, int64_t n, int split_rows, const nq_config *cfg, nq_batch **out) try {
     if (!out) return NQ_ERR_ARG;
     *out = nullptr;
-    if (n < 0 || (n > 0 && !inst) || split_rows < 0 || split_rows > 8) return NQ_ERR_ARG;
-    if (n > 0x7fffffffll) return NQ_ERR_ARG;
-    for (int64_t i = 0; i < n; ++i)
-        if (inst[i].N < 1 || inst[i].N > NQ_MAX_N) return NQ_ERR_ARG;
+    int rc = check_instances(inst, n, split_rows);
+    if (rc) return rc;
     Ctx *cp = nullptr;
-    int rc = lock_device(device_of(cfg), cp);
+    rc = lock_device(device_of(cfg), cp);
     if (rc) return rc;
     Ctx &c = *cp;
     std::lock_guard<std::mutex> lock(c.mu);
@@ -1427,7 +1510,7 @@ int nq_batch_create(const nq_instance *inst, int64_t n, int split_rows, const nq
 }
 
 int nq_batch_run(nq_batch *b, uint64_t *out, nq_stats *stats) try {
-    if (!b || (b->n_inst > 0 && !out)) return NQ_ERR_ARG;
+    if (!b || (b->t.n_inst > 0 && !out)) return NQ_ERR_ARG;
     const double t0 = now_ms();
     if (stats) memset(stats, 0, sizeof(*stats));
     Ctx &c = g_ctx[b->device];
@@ -1435,10 +1518,7 @@ int nq_batch_run(nq_batch *b, uint64_t *out, nq_stats *stats) try {
     NQ_CUDA(cudaSetDevice(b->device));
     int rc = run_batch(c, *b, stats);
     if (rc) return rc;
-    for (int64_t i = 0; i < b->n_inst; ++i) {
-        const int64_t u = b->inst_to_u[i];
-        out[i] = b->h_res[3 + 2 * u] + 2 * b->h_res[3 + 2 * u + 1];
-    }
+    b->t.gather(b->h_res + 3, out);
     if (stats) stats->total_ms = now_ms() - t0;
     return status_from_bits(b->h_res[2]);
 } catch (...) {
@@ -1629,12 +1709,57 @@ int nq_count_batch(const nq_instance *inst, int64_t n, int split_rows, uint64_t 
                    nq_stats *stats) try {
     if (stats) memset(stats, 0, sizeof(*stats));
     if (n == 0) return (n < 0 || split_rows < 0 || split_rows > 8) ? NQ_ERR_ARG : NQ_OK;
-    nq_batch *b = nullptr;
-    int rc = nq_batch_create(inst, n, split_rows, cfg, &b);
+    // One pass needs no plan of its own: the subtasks go through the device's
+    // buffers and the launch is issued directly (an allocation, a graph capture
+    // and their release cost 2-4 ms, against some 20 us for a small board).
+    const double t0 = now_ms();
+    int rc = check_instances(inst, n, split_rows);
     if (rc) return rc;
-    rc = nq_batch_run(b, out, stats);
-    nq_batch_destroy(b);
-    return rc;
+    if (!out) return NQ_ERR_ARG;
+    Ctx *cp = nullptr;
+    rc = lock_device(device_of(cfg), cp);
+    if (rc) return rc;
+    Ctx &c = *cp;
+    std::lock_guard<std::mutex> lock(c.mu);
+    rc = ensure_ready(c, device_of(cfg));
+    if (rc) return rc;
+    BatchTasks t;
+    batch_tasks(inst, n, split_rows ? split_rows : kDefaultSplit, t);
+    Launch L;
+    rc = plan_launch(c, cfg, t.levels, true, false, L);
+    if (rc) return rc;
+    // device: subtasks | 3 result words | per-owner sums
+    const size_t res_bytes = 24 + t.out_bytes(), bytes = t.tc.size() * 17;
+    rc = c.tasks.grow(t.task_bytes() + res_bytes + 256);
+    if (!rc) rc = c.h_tasks.grow(bytes);
+    if (!rc) rc = c.h_out.grow(res_bytes);
+    if (rc) return rc;
+    unsigned long long *d_res = (unsigned long long *)((char *)c.tasks.p + t.task_bytes());
+    unsigned long long *res = (unsigned long long *)c.h_out.p;
+    t.write(c.h_tasks.p);
+    NQ_CUDA(cudaEventRecord(c.ev[0], c.stream));
+    if (bytes) NQ_CUDA(cudaMemcpyAsync(c.tasks.p, c.h_tasks.p, bytes, cudaMemcpyHostToDevice, c.stream));
+    DfsParams p = t.params(c, cfg, c.tasks.p, d_res + 3);
+    p.sum_out = d_res;
+    p.nodes_out = d_res + 1;
+    p.status_out = d_res + 2;
+    NQ_CUDA(cudaEventRecord(c.ev[1], c.stream));
+    NQ_CUDA(cudaMemsetAsync(d_res, 0, res_bytes, c.stream));
+    rc = enqueue_dfs(c, p, L, true, false, c.stream);
+    if (rc) return rc;
+    NQ_CUDA(cudaEventRecord(c.ev[2], c.stream));
+    NQ_CUDA(cudaMemcpyAsync(res, d_res, res_bytes, cudaMemcpyDeviceToHost, c.stream));
+    NQ_CUDA(cudaStreamSynchronize(c.stream));
+    t.gather(res + 3, out);
+    if (stats) {
+        float ms = 0;
+        cudaEventElapsedTime(&ms, c.ev[1], c.ev[2]);
+        stats->kernel_ms = ms;
+        stats->tasks = (int64_t)t.tc.size();
+        fill_stats_launch(stats, L);
+        stats->total_ms = now_ms() - t0;
+    }
+    return status_from_bits(res[2]);
 } catch (...) {
     return status_of_exception();
 }

@@ -129,8 +129,6 @@ int64_t expand_prefixes(int N, int rows, uint32_t *cols, uint32_t *ld, uint32_t 
 int64_t expand_prefixes_to(int N, int rows, const PrefixSink &sink, int threads) {
     if (N < 2 || N > 31 || rows < 1 || rows > N) return -1;
     const uint32_t full = (1u << N) - 1u;
-    const int nthreads = pick_threads(threads);
-
     struct Seed {
         State s;
         bool odd;
@@ -142,6 +140,11 @@ int64_t expand_prefixes_to(int N, int rows, const PrefixSink &sink, int threads)
         dfs(ps, State{0, 0, 0}, 0, seed_rows, [&](const State &s) { seeds.push_back(Seed{s, ps.odd}); });
     }
     const int64_t ns = (int64_t)seeds.size();
+    // A thread costs some 20 us to start: one for every few thousand tasks, of
+    // which a seed has about (N/2)^(rows below it).
+    double est = (double)ns;
+    for (int r = seed_rows; r < rows; ++r) est *= 0.5 * N;
+    const int nthreads = (int)std::min<double>(pick_threads(threads), 1.0 + est / 4096.0);
     std::vector<int64_t> off(ns + 1, 0);
     parallel_for(nthreads, ns, [&](int64_t i) {
         const Pass ps{N, seeds[i].odd, full};
