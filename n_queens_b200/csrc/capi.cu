@@ -71,8 +71,8 @@ KernelFn pick_kernel(bool per_owner, bool nodes, bool dih = false) {
     if (dih) return per_owner ? dfs_kernel<true, false, kDihStepVar, kUnroll, false, true>
                               : dfs_kernel<false, false, kDihStepVar, kUnroll, false, true>;
     if (per_owner)
-        return nodes ? dfs_kernel<true, true, kNodesStepVar, kUnroll> : dfs_kernel<true, false, kStepVar, kCountUnroll>;
-    return nodes ? dfs_kernel<false, true, kNodesStepVar, kUnroll> : dfs_kernel<false, false, kStepVar, kCountUnroll>;
+        return nodes ? dfs_kernel<true, true, kNodesStepVar, kNodesUnroll> : dfs_kernel<true, false, kStepVar, kCountUnroll>;
+    return nodes ? dfs_kernel<false, true, kNodesStepVar, kNodesUnroll> : dfs_kernel<false, false, kStepVar, kCountUnroll>;
 }
 
 struct DevBuf {
@@ -848,10 +848,12 @@ int build_batch(Ctx &c, const nq_instance *inst, int64_t n, int split, const nq_
     NQ_CUDA(cudaHostAlloc((void **)&B.h_res, 24 + out_bytes, cudaHostAllocDefault));
     B.d_out = (unsigned long long *)((char *)B.d_buf + task_bytes);
     if (m) {
-        rc = c.h_tasks.grow((size_t)m * 17);
-        if (rc) return rc;
-        B.t.write(c.h_tasks.p);
-        NQ_CUDA(cudaMemcpyAsync(B.d_buf, c.h_tasks.p, (size_t)m * 17, cudaMemcpyHostToDevice, c.stream));
+        // straight from the vectors: the plan is built once, a pinned buffer of its size would cost more
+        uint32_t *d = (uint32_t *)B.d_buf;
+        int k = 0;
+        for (const auto *v : {&B.t.tc, &B.t.tl, &B.t.tr, &B.t.own})
+            NQ_CUDA(cudaMemcpyAsync(d + k++ * m, v->data(), (size_t)m * 4, cudaMemcpyHostToDevice, c.stream));
+        NQ_CUDA(cudaMemcpyAsync(d + 4 * m, B.t.tn.data(), (size_t)m, cudaMemcpyHostToDevice, c.stream));
     }
     NQ_CUDA(cudaStreamSynchronize(c.stream));
     const DfsParams p = B.t.params(c, cfg, B.d_buf, B.d_out);

@@ -310,7 +310,7 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     ".reg .b32 t, bit, nc, nl, nr, na, xl, xr, f0, lo, ma, mb, pos, pc, naf;\n\t"     \
     "setp.ne.u32 pt1, %8, 0;\n\t"
 
-#define NQB_STEP4                                                                     \
+#define NQB_STEP4_CHILD                                                               \
     "mul.lo.s32 t, %3, %10;\n\t"                                                      \
     "lop3.and.b32 bit|pb, t, %3, 0, 0xC0, pt1;\n\t"                                   \
     "mad.lo.s32 nc, bit, %8, %0;\n\t"                                                 \
@@ -328,10 +328,18 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "shr.b32 mb, %12, pos;\n\t"                                                       \
     "popc.b32 pc, nc;\n\t"                                                            \
     "setp.ne.and.u32 pg, pc, %14, pb;\n\t"                                            \
-    "setp.eq.and.u32 p2, pc, %14, pb;\n\t"                                            \
+    "setp.eq.and.u32 p2, pc, %14, pb;\n\t"
+
+#define NQB_STEP4_LOOK                                                                \
     "mul.lo.s32 t, xl, %9;\n\t"                                                       \
     "shr.s32 pos, xr, 1;\n\t"                                                         \
-    "lop3.and.b32 t|pg, nc, t, pos, 0x01, pg;\n\t"                                    \
+    "lop3.and.b32 t|pg, nc, t, pos, 0x01, pg;\n\t"
+
+#define NQB_STEP4_NODES                                                               \
+    "popc.b32 t, na;\n\t"                                                             \
+    "@pb mad.lo.s32 %6, t, %8, %6;\n\t"
+
+#define NQB_STEP4_TAIL                                                                \
     "lop3.and.b32 naf|pd, na, ma, mb, 0xE0, pg;\n\t"                                  \
     "popc.b32 t, naf;\n\t"                                                            \
     "@p2 mad.lo.s32 %5, t, %8, %5;\n\t"                                               \
@@ -347,6 +355,17 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "@pq mad.lo.s32 %4, %10, %11, %4;\n\t"                                            \
     "@pq ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
 
+#define NQB_STEP4 NQB_STEP4_CHILD NQB_STEP4_LOOK NQB_STEP4_TAIL
+// Node counts (%6): a level's placements are its free columns, dead ones
+// included, so a step adds the size of its child's unfiltered list (the root
+// level's is added when a task is loaded), and rows N-2 and N-1 and dead
+// children need no steps of their own.  No look-ahead: a child whose row two
+// below is full still has placements on the row between.  33 operations on 0.63
+// steps per node where VAR 3 takes 21 on one, and 37 % fewer stack accesses,
+// which bound VAR 3 (shared-memory wavefronts 65 %); this form is bound by issue
+// (83 %).  300,007 prefixes of N=17, k=6: kernel 2.12 -> 1.79 ms.
+#define NQB_STEP4N NQB_STEP4_CHILD NQB_STEP4_NODES NQB_STEP4_TAIL
+#define NQB_STEP4N_X4 NQB_STEP4N NQB_STEP4N NQB_STEP4N NQB_STEP4N
 #define NQB_STEP4_X4 NQB_STEP4 NQB_STEP4 NQB_STEP4 NQB_STEP4
 #define NQB_STEP4_X16 NQB_STEP4_X4 NQB_STEP4_X4 NQB_STEP4_X4 NQB_STEP4_X4
 
@@ -452,15 +471,15 @@ struct StepConsts {
 
 // Step variant of the count kernels: 4 = filtered children (default), 3 =
 // pre-shifted left diagonal with LOP3 predicate outputs, 1 = the reference's
-// mask form with IMAD-form moves.  Kernels that count DFS nodes (NODES) step
-// every placement, so they run variant 3 when 4 is chosen; the dihedral
-// kernels run their own filtered step (NQB_STEP_DIH4) with 4, else variant 1.
+// mask form with IMAD-form moves.  Kernels that count DFS nodes run the same
+// variant in its node-counting form; the dihedral kernels run their own
+// filtered step (NQB_STEP_DIH4) with 4, else variant 1.
 #ifndef NQB_STEP_VAR
 #define NQB_STEP_VAR 4
 #endif
 constexpr int kStepVar = NQB_STEP_VAR;
 static_assert(kStepVar == 1 || kStepVar == 3 || kStepVar == 4, "step variant");
-constexpr int kNodesStepVar = kStepVar == 4 ? 3 : kStepVar;
+constexpr int kNodesStepVar = kStepVar;
 constexpr int kDihStepVar = kStepVar == 4 ? 4 : 1;
 
 // Stack rows a step variant never pushes beyond the reference's N-1-rows: the
@@ -553,17 +572,23 @@ __device__ __forceinline__ void dfs_steps3(uint32_t &cols, uint32_t &ld, uint32_
     }
 }
 
-// UNROLL steps of VAR 4 (no NODES form), sixteen per asm block where UNROLL
-// allows (0.5 % faster at N=19 than four), else four.  Operand %6 is unused (it
-// stands where the node counter sits in the other forms).
-template <int UNROLL>
+// UNROLL steps of VAR 4, sixteen per asm block where UNROLL allows (0.5 %
+// faster at N=19 than four), else four.  Operand %6, the node counter, is used
+// by the NODES form only.
+template <bool NODES, int UNROLL>
 __device__ __forceinline__ void dfs_steps4(uint32_t &cols, uint32_t &ld, uint32_t &rd, uint32_t &avail, uint32_t &sp,
-                                           uint32_t &cnt, uint32_t bot, const StepConsts &k) {
+                                           uint32_t &cnt, uint32_t &it, uint32_t bot, const StepConsts &k) {
     static_assert(UNROLL % 4 == 0, "VAR 4 unrolls in groups of 4 or 16");
-    constexpr int kGroup = UNROLL % 16 == 0 ? 16 : 4;
+    constexpr int kGroup = UNROLL % 16 == 0 && !NODES ? 16 : 4;
 #pragma unroll
     for (int g = 0; g < UNROLL / kGroup; ++g) {
-        if constexpr (kGroup == 16)
+        if constexpr (NODES)
+            asm volatile(NQB_STEP4_HEAD NQB_STEP4N_X4 "}\n\t"
+                         : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt), "+r"(it)
+                         : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(0x3fffffffu),
+                           "r"(0xfffffffcu), "r"(30u)
+                         : "memory");
+        else if constexpr (kGroup == 16)
             asm volatile(NQB_STEP4_HEAD NQB_STEP4_X16 "}\n\t"
                          : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt)
                          : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(0x3fffffffu),
@@ -592,6 +617,14 @@ __device__ __forceinline__ void load_class(const DfsParams &p, long long t, DihL
     load_class_index(p, __ldg(p.task_cls + t), d);
 }
 
+// DFS nodes (placements on rows before N-1) from a lane's counters: VAR 1 and 3
+// count every placement, of which a completion is the one on row N-1; VAR 4
+// counts the nodes themselves.
+template <int VAR>
+__device__ __forceinline__ uint32_t node_count(uint32_t it, uint32_t cnt) {
+    return VAR == 4 ? it : it - cnt;
+}
+
 // VAR 4 keeps only levels on rows 0..N-3, with their alive columns.  A level
 // on row N-1 (one column left) completes once per free column; on row N-2
 // once per alive column.  Returns those completions and leaves avail = 0 for
@@ -616,9 +649,11 @@ __device__ __forceinline__ uint32_t settle_level(int n, uint32_t cols, uint32_t 
 // (1 for an already-complete board) and leaves avail == 0 when the task has
 // no free column.  A column mask with off-board bits can never equal `last`,
 // so such a task counts 0, exactly as the reference recursion does.
+// VAR 4: `placed` receives the columns whose placements the nodes of the task's
+// own row are (its free columns on rows before N-1).
 template <int VAR>
 __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, uint32_t &cols, uint32_t &ld,
-                                              uint32_t &rd, uint32_t &avail) {
+                                              uint32_t &rd, uint32_t &avail, uint32_t &placed) {
     const int n = p.task_n ? (int)p.task_n[t] : p.N;
     const uint32_t last = (n >= 32) ? kFull : ((1u << n) - 1u);
     const uint32_t c = __ldg(p.cols + t);
@@ -639,7 +674,10 @@ __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, u
     ld = lane_ld<VAR>(l);
     rd = lane_rd<VAR>(r);
     avail = ~(cols | l | r);
-    if (VAR == 4) return settle_level(n, cols, ld, rd, avail);
+    if (VAR == 4) {
+        placed = __popc(c) < n - 1 ? avail : 0u;
+        return settle_level(n, cols, ld, rd, avail);
+    }
     return 0;
 }
 
@@ -836,7 +874,6 @@ __device__ __forceinline__ uint32_t post_mail(const DfsParams &p, uint32_t lane,
 // weights, see DfsParams::cls_tab) and the step is dfs_step_dih.
 template <bool PER_OWNER, bool NODES, int VAR, int UNROLL, bool RESUME = false, bool DIH = false>
 __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
-    static_assert(!(VAR == 4 && NODES), "the filtered step counts no nodes");
     static_assert(!DIH || VAR == 1 || VAR == 4, "dihedral step variants: 1 and 4");
     // Lane registers and task loading of the step: the dihedral filtered step
     // keeps VAR 3's lane form and steps rows N-2 and N-1 (no settling).
@@ -882,18 +919,18 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
     for (;;) {
         // ---- fold the per-lane 32-bit counters (bounded inner loop keeps them < 2^32)
         if (PER_OWNER) {
-            if (avail == 0 && owner != kNoOwner) {
+            if (owner != kNoOwner && (avail == 0 || ((cnt | it) >> 31))) {
                 if (cnt) atomicAdd(p.out_cnt + owner, (unsigned long long)cnt);
-                if (NODES && it) atomicAdd(p.out_nodes + owner, (unsigned long long)(it - cnt));
+                if (NODES && it) atomicAdd(p.out_nodes + owner, (unsigned long long)node_count<VAR>(it, cnt));
                 tot += cnt;
-                if (NODES) tot_nodes += it - cnt;
+                if (NODES) tot_nodes += node_count<VAR>(it, cnt);
                 cnt = 0;
                 it = 0;
-                owner = kNoOwner;
+                if (avail == 0) owner = kNoOwner;
             }
         } else {
             tot += cnt;
-            if (NODES) tot_nodes += it - cnt;
+            if (NODES) tot_nodes += node_count<VAR>(it, cnt);
             cnt = 0;
             it = 0;
         }
@@ -958,7 +995,8 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                         // A permutation entry out of range is skipped, never dereferenced.
                         if (t >= 0 && t < p.ntasks) {
                             sp = bot = my_base;
-                            uint32_t done = load_task<LVAR>(p, t, cols, ld, rd, avail);
+                            uint32_t placed = 0;
+                            uint32_t done = load_task<LVAR>(p, t, cols, ld, rd, avail, placed);
                             if (DIH) {
                                 load_class(p, t, dih);
                                 done *= dih.w;
@@ -978,6 +1016,11 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                                 if (avail) owner = own;
                             }
                             tot += done;
+                            if (NODES && VAR == 4) {
+                                const uint32_t here = __popc(placed & share_mask(lg, way));
+                                if (PER_OWNER && here) atomicAdd(p.out_nodes + own, (unsigned long long)here);
+                                tot_nodes += here;
+                            }
                         }
                     }
                 }
@@ -1055,7 +1098,7 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                     if constexpr (DIH)
                         dfs_step_dih<VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
                     else if constexpr (VAR == 4)
-                        dfs_steps4<UNROLL>(cols, ld, rd, avail, sp, cnt, bot, kc);
+                        dfs_steps4<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
                     else if constexpr (VAR == 3)
                         dfs_steps3<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
                     else
@@ -1070,7 +1113,7 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                     if constexpr (DIH)
                         dfs_step_dih<VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
                     else if constexpr (VAR == 4)
-                        dfs_steps4<UNROLL>(cols, ld, rd, avail, sp, cnt, bot, kc);
+                        dfs_steps4<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
                     else if constexpr (VAR == 3)
                         dfs_steps3<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
                     else
@@ -1115,11 +1158,11 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
     if (PER_OWNER) {
         if (owner != kNoOwner) {
             if (cnt) atomicAdd(p.out_cnt + owner, (unsigned long long)cnt);
-            if (NODES && it) atomicAdd(p.out_nodes + owner, (unsigned long long)(it - cnt));
+            if (NODES && it) atomicAdd(p.out_nodes + owner, (unsigned long long)node_count<VAR>(it, cnt));
         }
     }
     tot += cnt;
-    if (NODES) tot_nodes += it - cnt;
+    if (NODES) tot_nodes += node_count<VAR>(it, cnt);
 
     // ---- per-warp, per-CTA reduction
 #pragma unroll

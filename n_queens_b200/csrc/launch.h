@@ -17,8 +17,9 @@ namespace nqb {
 // DFS steps per warp vote (the unroll of the kernel's inner loop), a
 // compile-time choice.  The filtered count step runs 16 between votes: fewer
 // votes and loop branches per step, for lanes that wait up to 15 steps for a
-// refill (1.1 % faster than 8 at N=21, k=6).  The node-count and dihedral
-// steps keep 8; the node-count step spills registers at 16.  A trip of the
+// refill (1.1 % faster than 8 at N=21, k=6).  So does the node-count step
+// (300,007 prefixes of N=17: kernel 1.88 ms with 8, 1.79 with 16); the dihedral
+// steps keep 8.  A trip of the
 // inner loop runs inner_steps rounded up to a multiple of the unroll.
 #ifndef NQB_UNROLL
 #define NQB_UNROLL 8
@@ -26,7 +27,11 @@ namespace nqb {
 #ifndef NQB_COUNT_UNROLL
 #define NQB_COUNT_UNROLL 16
 #endif
+#ifndef NQB_NODES_UNROLL
+#define NQB_NODES_UNROLL 16
+#endif
 constexpr int kUnroll = NQB_UNROLL;
+constexpr int kNodesUnroll = NQB_NODES_UNROLL;
 constexpr int kCountUnroll = kStepVar == 4 ? NQB_COUNT_UNROLL : NQB_UNROLL;
 static_assert(kUnroll % 4 == 0 && kCountUnroll % 4 == 0, "inner_steps are rounded to multiples of 4");
 
@@ -82,20 +87,22 @@ constexpr int kShareInner = 256;
 // How the queue hands out tasks: the first `coarse` tasks as 2^lg_coarse shares
 // of their root level's columns each (share_mask), the others as 2^lg_fine.
 // A lane runs a share by itself (until the queue is empty), so a share must be
-// short against the whole run: below 8 positions per lane the tasks are dealt
+// short against the whole run: below 4 positions per lane the tasks are dealt
 // out finer, and the last ones always are.  Sixteen shares only where eight do
 // not give every lane one; half of them are empty (a level rarely has more than
 // eight alive columns), and an empty share still costs a visit to the queue.
-// Measured: 60,001 prefixes of N=16, k=5 (0.23 per lane) 0.96 ms whole, 0.60 in
-// shares; 1501 prefixes of N=13, k=4 0.19 -> 0.13 ms per call; 1.1e6 prefixes of
-// N=18 (4.8 per lane) 18.8 ms with the line at 16 per lane, 18.5 at 8, 18.6 at 4.
+// Measured: 60,001 prefixes of N=16, k=5 (0.23 per lane) 0.96 ms whole, 0.59 in
+// shares; 1501 prefixes of N=13, k=4 0.19 -> 0.13 ms per call.  The line at 8, 4
+// and 2 positions per lane: 300,007 prefixes of N=17 with node counts (1.6 per
+// lane) 3.19, 3.03, 2.98 ms; 8 % of N=21's (2.1 per lane) 840, 839, 845 ms;
+// 1.1e6 of N=18 (4.8 per lane) 18.5 ms at all three.
 inline void set_shares(DfsParams &p, long long lanes) {
     const long long n = p.nqueue > 0 ? p.nqueue : p.ntasks;
     p.coarse = n;
     p.lg_coarse = p.lg_fine = 0;
     if (!p.steal) return;
     p.lg_fine = (n << 3) < lanes ? 4 : 3;
-    while (p.lg_coarse < p.lg_fine && (n << p.lg_coarse) < 8 * lanes) ++p.lg_coarse;
+    while (p.lg_coarse < p.lg_fine && (n << p.lg_coarse) < 4 * lanes) ++p.lg_coarse;
     const long long m = (2 * lanes) >> p.lg_fine;
     p.coarse = n > m ? n - m : 0;
 }

@@ -3,7 +3,9 @@ n_queens_b200/csrc/dfs_kernel.cuh): the filtered step of test_step_model.py,
 with the right diagonal pre-shifted too (a child's right mask is
 (bit >> 1) + rd) and children above row N-2 dropped when the row two below them
 has no free column.  Checked per task against the oracle on whole boards from
-the smallest the step enters and on arbitrary 32-bit masks."""
+the smallest the step enters and on arbitrary 32-bit masks.  The node-count form
+(``NQB_STEP4N``: the size of each child's unfiltered list instead of the
+look-ahead, plus the root level's) is checked the same way."""
 import numpy as np
 import pytest
 
@@ -12,9 +14,13 @@ from test_step_model import Lanes, need_slots, popc, sar1, shiftamt, shr_clamp
 
 
 class LookAheadLanes(Lanes):
-    def __init__(self, N, c, l, r):
+    def __init__(self, N, c, l, r, nodes=False):
         super().__init__(N, c, l, r)
         self.rd = sar1(self.rd)  # lane_rd<4>
+        self.count_nodes = nodes
+        last = np.uint32((1 << N) - 1)
+        root = np.where((c & ~last) | (popc(c) >= N - 1), np.uint32(0), ~(c | l | r) & last)
+        self.nodes = popc(root).astype(np.uint64)  # load_task's `placed`
 
     def step(self):
         one, two, mone, m4 = np.uint32(1), np.uint32(2), np.uint32(0xFFFFFFFF), np.uint32(0xFFFFFFFC)
@@ -30,7 +36,11 @@ class LookAheadLanes(Lanes):
         pc = popc(nc)
         p2 = (pc == 30) & pb
         f1 = ~(nc | xl * two | sar1(xr))
-        pg = (f1 != 0) & (pc != 30) & pb
+        pg = (pc != 30) & pb
+        if self.count_nodes:
+            self.nodes += np.where(pb, popc(na), 0).astype(np.uint64)
+        else:
+            pg &= f1 != 0
         naf = na & (ma | mb)
         pd = (naf != 0) & pg
         self.cnt += np.where(p2, popc(naf), 0).astype(np.uint64)
@@ -63,3 +73,12 @@ def test_arbitrary_32bit_tasks(N):
     got = LookAheadLanes(N, c, l, r).run()
     np.testing.assert_array_equal(got, oracle.count_tasks(N, c, l, r))
     assert got.sum() > 0
+
+
+@pytest.mark.parametrize("N,k", [(4, 1), (5, 2), (7, 5), (8, 3), (8, 6), (10, 4)])
+def test_node_counts(N, k):
+    c, l, r = oracle.expand(N, k)
+    lanes = LookAheadLanes(N, c, l, r, nodes=True)
+    want, nodes = oracle.count_tasks(N, c, l, r, nodes=True)
+    np.testing.assert_array_equal(lanes.run(), want)
+    np.testing.assert_array_equal(lanes.nodes, nodes)
