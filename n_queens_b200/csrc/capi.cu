@@ -68,8 +68,8 @@ double now_ms() {
 typedef void (*KernelFn)(DfsParams);
 
 KernelFn pick_kernel(bool per_owner, bool nodes, bool dih = false) {
-    if (dih) return per_owner ? dfs_kernel<true, false, kDihStepVar, kUnroll, false, true>
-                              : dfs_kernel<false, false, kDihStepVar, kUnroll, false, true>;
+    if (dih) return per_owner ? dfs_kernel<true, false, kDihStepVar, kDihUnroll, false, true>
+                              : dfs_kernel<false, false, kDihStepVar, kDihUnroll, false, true>;
     if (per_owner)
         return nodes ? dfs_kernel<true, true, kNodesStepVar, kNodesUnroll> : dfs_kernel<true, false, kStepVar, kCountUnroll>;
     return nodes ? dfs_kernel<false, true, kNodesStepVar, kNodesUnroll> : dfs_kernel<false, false, kStepVar, kCountUnroll>;
@@ -166,7 +166,7 @@ int ensure_ready(Ctx &c, int dev) {
                                          c.smem_optin - static_smem));
     NQ_CUDA(cudaFuncSetAttribute(dfs_kernel<false, false, kStepVar, kCountUnroll, true>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, c.smem_optin - static_smem));
-    NQ_CUDA(cudaFuncSetAttribute(dfs_kernel<false, false, kDihStepVar, kUnroll, true, true>,
+    NQ_CUDA(cudaFuncSetAttribute(dfs_kernel<false, false, kDihResumeStepVar, kUnroll, true, true>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, c.smem_optin - static_smem));
     for (int po = 0; po < 2; ++po)
         NQ_CUDA(cudaFuncSetAttribute(pick_kernel(po, false, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -983,7 +983,7 @@ int count_resumable_impl(int N, int rows, const nq_config *cfg, const char *chec
         NQ_CUDA(cudaMemcpyAsync(d_cont_in, ck.cont.data(), ncont * 16, cudaMemcpyHostToDevice, c.stream));
         if (dih) NQ_CUDA(cudaMemcpyAsync(d_cont_cls, ck.cls.data(), ncont, cudaMemcpyHostToDevice, c.stream));
     }
-    KernelFn fn = dih ? dfs_kernel<false, false, kDihStepVar, kUnroll, true, true> : dfs_kernel<false, false, kStepVar, kCountUnroll, true>;
+    KernelFn fn = dih ? dfs_kernel<false, false, kDihResumeStepVar, kUnroll, true, true> : dfs_kernel<false, false, kStepVar, kCountUnroll, true>;
     Launch L;
     rc = plan_launch(c, cfg, stack_need(N, rows, !dih), false, false, L, dih);
     if (rc) return rc;

@@ -459,6 +459,76 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "@pq ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"                                \
     "}\n\t"
 
+// VAR 5, the dihedral kernels' default: VAR 4's step (both diagonals
+// pre-shifted, alive columns, row N-2 counted, look-ahead) under the class rules.
+//  * Side columns barred past side_row: whoever enters such a row with a side
+//    column still unused can never complete the board (every column needs a
+//    queen), so the child's list becomes empty; with both used no list holds
+//    them.  One compare, one LOP3 with a predicate, one predicated move, as many
+//    as masking the list took, and 8 % fewer nodes (N=16..17, k=6).
+//  * Row N-1's columns: a child on row N-2 masks the free columns of row N-1
+//    (F0) with them before its alive columns are taken; its completions are then
+//    its alive columns, as in VAR 4 (the mask is all ones in the classes that do
+//    not bar row N-1).
+//  * Weights: each completion weighs w, and the one whose row N-1 queen stands
+//    at the tie column weighs w + dw; there is one when the tie column is unused
+//    and a column other than it is alive.
+// 41 operations where the form above has 40, on fewer steps (0.85 at N=11, CPU
+// model; the launch's instructions fall from 111.9e9 to 98.6e9 at N=19, k=6).
+// Bound by issue (84 %, was 79 %) and the ALU pipe (79 %).  N=19, k=6: kernel
+// 122.7 -> 100.7 ms.  Operands as above, with %16 the tie's extra weight dw.
+#define NQB_STEP5_HEAD                                                                \
+    "{\n\t"                                                                           \
+    ".reg .pred pt1, pb, pg, p2, pd, pk, pp, pq, ps;\n\t"                             \
+    ".reg .b32 t, bit, nc, nl, nr, na, xl, xr, f0, lo, ma, mb, pos, pc, naf;\n\t"     \
+    "setp.ne.u32 pt1, %8, 0;\n\t"
+
+#define NQB_STEP5                                                                     \
+    "mul.lo.s32 t, %3, %10;\n\t"                                                      \
+    "lop3.and.b32 bit|pb, t, %3, 0, 0xC0, pt1;\n\t"                                   \
+    "mad.lo.s32 nc, bit, %8, %0;\n\t"                                                 \
+    "mad.lo.s32 nl, bit, %9, %1;\n\t"                                                 \
+    "shr.u32 nr, bit, 1;\n\t"                                                         \
+    "add.u32 nr, nr, %2;\n\t"                                                         \
+    "lop3.b32 na, nc, nl, nr, 0x01;\n\t"                                              \
+    "mul.lo.s32 xl, nl, %9;\n\t"                                                      \
+    "shr.s32 xr, nr, 1;\n\t"                                                          \
+    "lop3.b32 f0, nc, xl, xr, 0x01;\n\t"                                              \
+    "popc.b32 pc, nc;\n\t"                                                            \
+    "setp.eq.and.u32 p2, pc, 30, pb;\n\t"                                             \
+    "setp.ne.and.u32 pg, pc, 30, pb;\n\t"                                             \
+    "setp.gt.u32 ps, pc, %12;\n\t"                                                    \
+    "lop3.and.b32 t|ps, nc, %17, 0, 0x03, ps;\n\t"                                    \
+    "@ps mul.lo.s32 na, na, 0;\n\t"                                                   \
+    "@p2 and.b32 f0, f0, %13;\n\t"                                                    \
+    "neg.s32 t, f0;\n\t"                                                              \
+    "and.b32 lo, t, f0;\n\t"                                                          \
+    "mul.lo.s32 ma, lo, -4;\n\t"                                                      \
+    "bfind.shiftamt.u32 pos, f0;\n\t"                                                 \
+    "shr.b32 mb, 0x3fffffff, pos;\n\t"                                                \
+    "mul.lo.s32 t, xl, %9;\n\t"                                                       \
+    "shr.s32 pos, xr, 1;\n\t"                                                         \
+    "lop3.and.b32 t|pg, nc, t, pos, 0x01, pg;\n\t"                                    \
+    "lop3.and.b32 naf|pd, na, ma, mb, 0xE0, pg;\n\t"                                  \
+    "popc.b32 t, naf;\n\t"                                                            \
+    "@p2 mad.lo.s32 %5, t, %15, %5;\n\t"                                              \
+    "lop3.and.b32 t|p2, %14, nc, 0, 0x30, p2;\n\t"                                    \
+    "lop3.and.b32 t|p2, naf, %14, 0, 0x30, p2;\n\t"                                   \
+    "@p2 mad.lo.s32 %5, %16, %8, %5;\n\t"                                             \
+    "lop3.or.b32 %3|pk, %3, bit, 0, 0x3C, pd;\n\t"                                    \
+    "setp.ne.and.u32 pp, %3, 0, pd;\n\t"                                              \
+    "@pp st.shared.v4.u32 [%4], {%0, %1, %2, %3};\n\t"                                \
+    "@pp mad.lo.s32 %4, %8, %11, %4;\n\t"                                             \
+    "@pd mul.lo.s32 %0, nc, %8;\n\t"                                                  \
+    "@pd mul.lo.s32 %1, xl, %8;\n\t"                                                  \
+    "@pd mul.lo.s32 %2, xr, %8;\n\t"                                                  \
+    "@pd mul.lo.s32 %3, naf, %8;\n\t"                                                 \
+    "setp.ne.and.u32 pq, %4, %7, !pk;\n\t"                                            \
+    "@pq mad.lo.s32 %4, %10, %11, %4;\n\t"                                            \
+    "@pq ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
+
+#define NQB_STEP5_X4 NQB_STEP5 NQB_STEP5 NQB_STEP5 NQB_STEP5
+
 // Class registers of a lane in a DIH kernel (cls: the class index, kept for
 // the deadline dump of resumable runs).
 struct DihLane {
@@ -480,7 +550,10 @@ struct StepConsts {
 constexpr int kStepVar = NQB_STEP_VAR;
 static_assert(kStepVar == 1 || kStepVar == 3 || kStepVar == 4, "step variant");
 constexpr int kNodesStepVar = kStepVar;
-constexpr int kDihStepVar = kStepVar == 4 ? 4 : 1;
+constexpr int kDihStepVar = kStepVar == 4 ? 5 : 1;
+// The resumable dihedral kernel keeps the form that steps rows N-2 and N-1: its
+// checkpoints hold levels on those rows.
+constexpr int kDihResumeStepVar = kStepVar == 4 ? 4 : 1;
 
 // Stack rows a step variant never pushes beyond the reference's N-1-rows: the
 // filtered step enters no level on row N-2 or N-1, so the deepest level it
@@ -603,6 +676,22 @@ __device__ __forceinline__ void dfs_steps4(uint32_t &cols, uint32_t &ld, uint32_
     }
 }
 
+// UNROLL steps of VAR 5, four per asm block.
+template <int UNROLL>
+__device__ __forceinline__ void dfs_steps5(uint32_t &cols, uint32_t &ld, uint32_t &rd, uint32_t &avail, uint32_t &sp,
+                                           uint32_t &cnt, uint32_t &it, uint32_t bot, const StepConsts &k,
+                                           const DihLane &d, uint32_t noside) {
+    static_assert(UNROLL % 4 == 0, "VAR 5 unrolls in groups of 4");
+    const uint32_t dw = d.w_tie - d.w;
+#pragma unroll
+    for (int g = 0; g < UNROLL / 4; ++g)
+        asm volatile(NQB_STEP5_HEAD NQB_STEP5_X4 "}\n\t"
+                     : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt), "+r"(it)
+                     : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(d.side_popc),
+                       "r"(d.last_mask), "r"(d.tie_bit), "r"(d.w), "r"(dw), "r"(noside)
+                     : "memory");
+}
+
 __device__ __forceinline__ void load_class_index(const DfsParams &p, uint32_t idx, DihLane &d) {
     const uint4 c = __ldg(p.cls_tab + idx);
     d.cls = idx;
@@ -645,13 +734,32 @@ __device__ __forceinline__ uint32_t settle_level(int n, uint32_t cols, uint32_t 
     return 0;
 }
 
+// The same for VAR 5: weighted completions of a level on rows N-2 and N-1, whose
+// avail already follows the class rules of its own row.
+__device__ __forceinline__ uint32_t settle_level_dih(int n, uint32_t cols, uint32_t ld, uint32_t rd, uint32_t &avail,
+                                                     const DihLane &d) {
+    const int row = __popc(cols) - (32 - n);
+    if (row >= n - 1) {
+        const uint32_t done = (avail & ~d.tie_bit) ? d.w : avail ? d.w_tie : 0u;  // one column at most
+        avail = 0;
+        return done;
+    }
+    const bool n2 = row == n - 2;
+    // columns that row N-1 may not use count as taken there
+    avail = alive_columns(cols, ld | (n2 ? ~d.last_mask : 0u), rd, avail);
+    if (!n2) return 0;
+    const uint32_t done = __popc(avail) * d.w + ((d.tie_bit & ~cols) && (avail & ~d.tie_bit) ? d.w_tie - d.w : 0u);
+    avail = 0;
+    return done;
+}
+
 // Loads task t into a lane.  Returns the completions credited immediately
 // (1 for an already-complete board) and leaves avail == 0 when the task has
 // no free column.  A column mask with off-board bits can never equal `last`,
 // so such a task counts 0, exactly as the reference recursion does.
 // VAR 4: `placed` receives the columns whose placements the nodes of the task's
 // own row are (its free columns on rows before N-1).
-template <int VAR>
+template <int VAR, bool SETTLE = true>
 __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, uint32_t &cols, uint32_t &ld,
                                               uint32_t &rd, uint32_t &avail, uint32_t &placed) {
     const int n = p.task_n ? (int)p.task_n[t] : p.N;
@@ -674,7 +782,7 @@ __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, u
     ld = lane_ld<VAR>(l);
     rd = lane_rd<VAR>(r);
     avail = ~(cols | l | r);
-    if (VAR == 4) {
+    if (VAR == 4 && SETTLE) {
         placed = __popc(c) < n - 1 ? avail : 0u;
         return settle_level(n, cols, ld, rd, avail);
     }
@@ -874,10 +982,10 @@ __device__ __forceinline__ uint32_t post_mail(const DfsParams &p, uint32_t lane,
 // weights, see DfsParams::cls_tab) and the step is dfs_step_dih.
 template <bool PER_OWNER, bool NODES, int VAR, int UNROLL, bool RESUME = false, bool DIH = false>
 __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
-    static_assert(!DIH || VAR == 1 || VAR == 4, "dihedral step variants: 1 and 4");
-    // Lane registers and task loading of the step: the dihedral filtered step
-    // keeps VAR 3's lane form and steps rows N-2 and N-1 (no settling).
-    constexpr int LVAR = (DIH && VAR == 4) ? 3 : VAR;
+    static_assert(DIH ? VAR == 1 || VAR == 4 || VAR == 5 : VAR != 5, "dihedral step variants: 1, 4 and 5");
+    // Lane registers of the step: the dihedral VAR 4 keeps VAR 3's form, VAR 5
+    // has VAR 4's.
+    constexpr int LVAR = (DIH && VAR == 4) ? 3 : VAR == 5 ? 4 : VAR;
     constexpr bool MAIL = !RESUME;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned long long red_cnt[32];
@@ -996,7 +1104,7 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                         if (t >= 0 && t < p.ntasks) {
                             sp = bot = my_base;
                             uint32_t placed = 0;
-                            uint32_t done = load_task<LVAR>(p, t, cols, ld, rd, avail, placed);
+                            uint32_t done = load_task<LVAR, !DIH>(p, t, cols, ld, rd, avail, placed);
                             if (DIH) {
                                 load_class(p, t, dih);
                                 done *= dih.w;
@@ -1004,6 +1112,7 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                                 // (the step applies them to children only).
                                 const uint32_t pc = (uint32_t)__popc(cols);
                                 if (avail && pc > dih.side_popc) avail &= pc == 31u ? dih.last_mask : p.noside;
+                                if (VAR == 5 && avail) done += settle_level_dih(p.N, cols, ld, rd, avail, dih);
                             }
                             if (!RESUME) {
                                 // this lane's share of the task's columns
@@ -1094,8 +1203,10 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
         if (check_idle) {
             for (int s = 0; s < p.inner; s += UNROLL) {
 #pragma unroll
-                for (int u = 0; u < (VAR >= 3 && !DIH ? 1 : UNROLL); ++u) {
-                    if constexpr (DIH)
+                for (int u = 0; u < ((VAR >= 3 && !DIH) || VAR == 5 ? 1 : UNROLL); ++u) {
+                    if constexpr (VAR == 5)
+                        dfs_steps5<UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
+                    else if constexpr (DIH)
                         dfs_step_dih<VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
                     else if constexpr (VAR == 4)
                         dfs_steps4<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
@@ -1109,8 +1220,10 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
         } else {
             for (int s = 0; s < kShortTrip; s += UNROLL) {
 #pragma unroll
-                for (int u = 0; u < (VAR >= 3 && !DIH ? 1 : UNROLL); ++u) {
-                    if constexpr (DIH)
+                for (int u = 0; u < ((VAR >= 3 && !DIH) || VAR == 5 ? 1 : UNROLL); ++u) {
+                    if constexpr (VAR == 5)
+                        dfs_steps5<UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
+                    else if constexpr (DIH)
                         dfs_step_dih<VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
                     else if constexpr (VAR == 4)
                         dfs_steps4<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);

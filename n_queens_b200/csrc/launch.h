@@ -31,7 +31,11 @@ namespace nqb {
 #define NQB_NODES_UNROLL 16
 #endif
 constexpr int kUnroll = NQB_UNROLL;
+#ifndef NQB_DIH_UNROLL
+#define NQB_DIH_UNROLL 8
+#endif
 constexpr int kNodesUnroll = NQB_NODES_UNROLL;
+constexpr int kDihUnroll = NQB_DIH_UNROLL;
 constexpr int kCountUnroll = kStepVar == 4 ? NQB_COUNT_UNROLL : NQB_UNROLL;
 static_assert(kUnroll % 4 == 0 && kCountUnroll % 4 == 0, "inner_steps are rounded to multiples of 4");
 
