@@ -10,9 +10,8 @@
 // Model: x (96 bits: cols, ld, rd, each as 32 bits with the columns >= N
 // cleared) -> 128 ReLU -> 128 ReLU -> 1.  Weights are BF16 for compute with
 // FP32 master copies for Adam; biases are FP32; every sum accumulates in
-// FP32.  Kernels (all hand-written, CUDA cores; at 29k parameters the model
-// is far too small for tensor-core tiles to pay):
-//   mlp_predict_kernel  forward for many tasks, 32 tasks per group per CTA
+// FP32.  Kernels (all hand-written):
+//   mlp_forward_kernel  forward for many tasks on the tensor cores
 //   mlp_train_kernel    forward + backward of a minibatch slice; per-CTA
 //                       partial gradients (no atomics: deterministic)
 //   mlp_adam_kernel     sums the partials in CTA order, Adam step, refreshes
@@ -55,8 +54,20 @@ constexpr int kOffB3 = kOffW3 + kH2;
 constexpr int kParams = kOffB3 + 1;
 constexpr int kGroup = 32;  // tasks per group (one per lane of the layer-3 reduction)
 
+// Offset (bytes) of element (row, k) of a K-major tensor-core operand without
+// swizzle: 8-row x 16-byte core matrices, sbo bytes between 8-row groups.
+__host__ __device__ constexpr uint32_t off_kmajor(uint32_t row, uint32_t k, uint32_t sbo) {
+    return (row >> 3) * sbo + (k >> 3) * 128u + (row & 7u) * 16u + (k & 7u) * 2u;
+}
+constexpr uint32_t kSbo1 = (kIn / 8) * 128;  // 1536 B: operands with K = 96
+constexpr uint32_t kSbo2 = (kH1 / 8) * 128;  // 2048 B: operands with K = 128
+
 // Compute copy of the weights in device memory.
 struct Weights {
+    // W1 and W2 as the forward kernel's B operands lie in shared memory, so that
+    // a CTA loads them by straight 16-byte copies.
+    alignas(16) __nv_bfloat16 w1c[kIn * kH1];
+    alignas(16) __nv_bfloat16 w2c[kH2 * kH1];
     __nv_bfloat16 w1t[kIn * kH1];  // [input bit][hidden unit]
     __nv_bfloat16 w2[kH2 * kH1];   // [unit of layer 2][unit of layer 1]
     __nv_bfloat16 w3[kH2];
@@ -128,80 +139,54 @@ __device__ __forceinline__ void load_w2row(const Weights *w, int j, uint32_t (&w
     for (int i = 0; i < kH1 / 2; ++i) w2row[i] = src[i];
 }
 
-// Forward over n tasks: out[t] = predicted log2(1 + nodes).  128 threads,
-// thread j = hidden unit j.
-__global__ void __launch_bounds__(128) mlp_predict_kernel(TaskView tv, long long n, const Weights *w, float *out) {
-    __shared__ __align__(16) __nv_bfloat16 s_w1t[kIn * kH1];
-    __shared__ __align__(16) float s_h[kGroup * kH1];
-    __shared__ uint32_t s_m[3][kGroup];
-    const int j = threadIdx.x;
-    for (int i = j; i < kIn * kH1 / 8; i += blockDim.x)
-        reinterpret_cast<uint4 *>(s_w1t)[i] = reinterpret_cast<const uint4 *>(w->w1t)[i];
-    uint32_t w2row[kH1 / 2];
-    load_w2row(w, j, w2row);
-    const float b1 = w->b1[j], b2 = w->b2[j], w3 = __bfloat162float(w->w3[j]), b3 = w->b3;
-    const int warp = j >> 5, lane = j & 31;
-    __syncthreads();
-    for (long long g0 = (long long)blockIdx.x * kGroup; g0 < n; g0 += (long long)gridDim.x * kGroup) {
-        const int gn = (int)min((long long)kGroup, n - g0);
-        if (j < gn) load_masks(tv, g0 + j, s_m[0][j], s_m[1][j], s_m[2][j]);
-        __syncthreads();
-        for (int s = 0; s < gn; ++s)
-            s_h[s * kH1 + j] = fmaxf(layer1(s_w1t, b1, s_m[0][s], s_m[1][s], s_m[2][s], j), 0.f);
-        __syncthreads();
-        float v[kGroup];
-#pragma unroll
-        for (int s = 0; s < kGroup; ++s) v[s] = (s < gn) ? fmaxf(layer2(w2row, b2, s_h + s * kH1), 0.f) * w3 : 0.f;
-        __syncthreads();
-#pragma unroll
-        for (int s = 0; s < kGroup; ++s) s_h[s * kH1 + j] = v[s];
-        __syncthreads();
-        // layer 3: warp w reduces tasks 8w..8w+7, each lane summing 4 units
-        for (int s = warp * 8; s < warp * 8 + 8; ++s) {
-            const float4 q = *reinterpret_cast<const float4 *>(s_h + s * kH1 + lane * 4);
-            float a = (q.x + q.y) + (q.z + q.w);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-            if (lane == 0 && s < gn) out[g0 + s] = a + b3;
-        }
-        __syncthreads();
-    }
-}
-
 // ---------------------------------------------------------------------------
-// Tensor-core inference (tcgen05).  Per tile of 128 tasks, one CTA of 128
-// threads (thread t = task row t = TMEM lane t):
-//   X (128 x 96 binary, BF16) --tcgen05.mma--> D1 (TMEM, FP32) --relu+b1,
-//   BF16--> H1 (128 x 128, smem) --tcgen05.mma--> D2 (TMEM) --relu+b2, dot W3,
-//   +b3--> out.
+// Forward pass on the tensor cores (tcgen05).  A CTA runs GROUPS groups of 128
+// threads, each on its own tiles of 128 tasks (thread t of a group = task row t
+// = TMEM lane t):
+//   X (128 x 96 binary, BF16) --tcgen05.mma--> D1 (TMEM, FP32) --relu+b1-->
+//   H1 (128 x 128, smem) --tcgen05.mma--> D2 (TMEM) --relu+b2, dot W3, +b3-->
+//   out.
+// H1 is BF16 in one of two forms: rounded (PARTS 1, the scheduler's forward,
+// nq_mlp_predict_tensor), or split into three BF16 parts that add up to the FP32
+// value (PARTS 3, nq_mlp_predict), each multiplied by the exact BF16 weights into
+// the same FP32 accumulator.
 // Operands use the SM100 K-major canonical layout without swizzle: 8-row x
 // 16-byte core matrices, LBO = 128 B between the two core matrices of one
-// K=16 step, SBO = K/8 * 128 B between 8-row groups.  One thread issues the
-// MMAs; completion is signalled through an mbarrier (tcgen05.commit) and every
-// wait on it is bounded (on expiry the kernel sets *err and stops).
+// K=16 step, SBO = K/8 * 128 B between 8-row groups.  One thread of a group
+// issues its MMAs; completion is signalled through the group's mbarrier
+// (tcgen05.commit) and every wait on it is bounded (on expiry the kernel sets
+// *err and stops).
+//
+// What bounds it: the latency of a tile's chain (X build, MMA, epilogue, MMA,
+// epilogue), then issue in the epilogues (52 % at 1.9e6 tasks, tensor pipe 38 %).
+// Four groups share one copy of the weights, which is what fits shared memory
+// (56 KiB + 4 x 32 KiB) and TMEM (D2 overwrites D1 once its group has read it:
+// 128 columns each): 1.9e6 tasks with their sort keys 226 + 10 -> 154 us against two
+// CTAs per SM with one tile each and a key kernel of its own.  PARTS 3 keeps D1
+// for the later parts (256 columns) and needs two operand buffers, so two groups
+// run: 200,000 tasks 889 us on the CUDA cores in FP32 -> 55 us, error against 64
+// bits 2.4e-8 (2.3e-8 before; the rounding of the result).
 namespace tc {
 
-constexpr uint32_t kSbo1 = (kIn / 8) * 128;   // 1536 B
-constexpr uint32_t kSbo2 = (kH1 / 8) * 128;   // 2048 B
-constexpr uint32_t kOffB1 = 0;                 // W1: 128 units x 96  (24 KiB)
-constexpr uint32_t kOffB2 = kOffB1 + kH1 * kSbo1 / 8;  // 24576: W2: 128 x 128 (32 KiB)
-constexpr uint32_t kOffA = kOffB2 + kH2 * kSbo2 / 8;   // 57344: X / H1 tile (32 KiB)
-constexpr uint32_t kOffBias = kOffA + 128 * kSbo2 / 8;  // 90112: b1, b2, w3 (fp32)
-constexpr uint32_t kOffBar = kOffBias + 3 * 128 * 4;    // 91648: mbarrier (8 B)
-constexpr uint32_t kOffTmem = kOffBar + 8;              // TMEM base address word
-constexpr uint32_t kSmemBytes = kOffTmem + 8;
-constexpr uint32_t kTmemCols = 256;  // D1 at column 0, D2 at column 128
+constexpr uint32_t kOffB1 = 0;                          // W1: 128 units x 96  (24 KiB)
+constexpr uint32_t kOffB2 = kOffB1 + kH1 * kSbo1 / 8;   // 24576: W2: 128 x 128 (32 KiB)
+constexpr uint32_t kOffA = kOffB2 + kH2 * kSbo2 / 8;    // 57344: operand buffers (4 x 32 KiB)
+constexpr uint32_t kABytes = 128 * kSbo2 / 8;
+constexpr uint32_t kOffBias = kOffA + 4 * kABytes;      // b1, b2, w3 (fp32)
+constexpr uint32_t kOffLut = kOffBias + 3 * 128 * 4;    // 4 bits -> 4 BF16 values (16 x 8 B)
+constexpr uint32_t kOffBar = kOffLut + 128;             // one mbarrier per group (8 B)
+constexpr uint32_t kOffTmem = kOffBar + 4 * 8;          // TMEM base address word, fail words
+constexpr uint32_t kSmemBytes = kOffTmem + 32;
+constexpr uint32_t kTmemCols = 512;
 // Instruction descriptor, kind::f16: D F32, A and B BF16, both K-major,
 // N = 128 (N>>3 at bit 17), M = 128 (M>>4 at bit 24).
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 constexpr unsigned long long kWaitLimit = 1ull << 22;  // a few seconds at most
 
-__host__ __device__ constexpr uint32_t off_kmajor(uint32_t row, uint32_t k, uint32_t sbo) {
-    return (row >> 3) * sbo + (k >> 3) * 128u + (row & 7u) * 16u + (k & 7u) * 2u;
-}
 static_assert(off_kmajor(127, 95, kSbo1) < kOffB2 - kOffB1, "W1 tile bounds");
 static_assert(off_kmajor(127, 127, kSbo2) < kOffA - kOffB2, "W2 tile bounds");
-static_assert(off_kmajor(127, 127, kSbo2) < kOffBias - kOffA, "A tile bounds");
+static_assert(off_kmajor(127, 127, kSbo2) < kABytes, "A tile bounds");
+static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
 
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
@@ -257,31 +242,55 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, ui
 
 }  // namespace tc
 
-__global__ void __launch_bounds__(128, 1)
-    mlp_predict_tc_kernel(TaskView tv, long long n, const Weights *w, float *out, int *err) {
+// One barrier per group of 128 threads (barrier 0 is the CTA's).
+__device__ __forceinline__ void group_sync(uint32_t group) {
+    asm volatile("bar.sync %0, 128;" ::"r"(group + 1u) : "memory");
+}
+
+// Sort key of the longest-first order: 1 + predicted log2 cost in 1/8 units
+// (key 0 is kept for tasks that must go last, mlp_last_kernel).
+__device__ __forceinline__ uint16_t order_key(float pred) {
+    const float v = fminf(fmaxf(pred * 8.f + 0.5f, 0.f), 65534.f);
+    return (uint16_t)(1.f + v);
+}
+
+// out (optional): predictions.  key and idx (both or neither): sort keys and the
+// identity permutation for the scheduler.
+template <int PARTS>
+__global__ void __launch_bounds__(PARTS == 1 ? 512 : 256, 1)
+    mlp_forward_kernel(TaskView tv, long long n, const Weights *w, float *out, uint16_t *key, uint32_t *idx, int *err) {
+    constexpr uint32_t kGroups = PARTS == 1 ? 4 : 2;
+    constexpr uint32_t kBufs = 4 / kGroups;  // operand buffers of a group
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(tc_smem);
-    const uint32_t t = threadIdx.x, warp = t >> 5;
-    float *bias = reinterpret_cast<float *>(tc_smem + tc::kOffBias);
-    const uint32_t bar = base + tc::kOffBar;
+    const uint32_t tid = threadIdx.x, t = tid & 127u, g = tid >> 7, warp = t >> 5;
+    const float *bias = reinterpret_cast<const float *>(tc_smem + tc::kOffBias);
+    const uint32_t bar = base + tc::kOffBar + 8 * g;
+    const uint32_t abuf = base + tc::kOffA + g * kBufs * tc::kABytes;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tc_smem + tc::kOffTmem);
+    volatile int *fail = reinterpret_cast<volatile int *>(tmem_slot + 1 + g);
 
-    // Weights into the canonical operand layouts (BF16 copies as stored).
-    for (uint32_t i = t; i < (uint32_t)(kH1 * kIn); i += blockDim.x) {
-        const uint32_t unit = i / kIn, k = i % kIn;
-        *reinterpret_cast<__nv_bfloat16 *>(tc_smem + tc::kOffB1 + tc::off_kmajor(unit, k, tc::kSbo1)) =
-            w->w1t[k * kH1 + unit];
+    {
+        const uint4 *src1 = reinterpret_cast<const uint4 *>(w->w1c), *src2 = reinterpret_cast<const uint4 *>(w->w2c);
+        uint4 *dst1 = reinterpret_cast<uint4 *>(tc_smem + tc::kOffB1);
+        uint4 *dst2 = reinterpret_cast<uint4 *>(tc_smem + tc::kOffB2);
+        for (uint32_t i = tid; i < kIn * kH1 / 8; i += blockDim.x) dst1[i] = src1[i];
+        for (uint32_t i = tid; i < kH2 * kH1 / 8; i += blockDim.x) dst2[i] = src2[i];
+        float *b = reinterpret_cast<float *>(tc_smem + tc::kOffBias);
+        if (tid < 128) {
+            b[tid] = w->b1[tid];
+            b[128 + tid] = w->b2[tid];
+            b[256 + tid] = __bfloat162float(w->w3[tid]);
+        }
+        if (tid < 16) {
+            uint32_t *lut = reinterpret_cast<uint32_t *>(tc_smem + tc::kOffLut) + 2 * tid;
+            lut[0] = (tid & 1u ? 0x3F80u : 0u) | (tid & 2u ? 0x3F800000u : 0u);
+            lut[1] = (tid & 4u ? 0x3F80u : 0u) | (tid & 8u ? 0x3F800000u : 0u);
+        }
+        if (t == 0) *fail = 0;
     }
-    for (uint32_t i = t; i < (uint32_t)(kH2 * kH1); i += blockDim.x) {
-        const uint32_t unit = i / kH1, k = i % kH1;
-        *reinterpret_cast<__nv_bfloat16 *>(tc_smem + tc::kOffB2 + tc::off_kmajor(unit, k, tc::kSbo2)) =
-            w->w2[unit * kH1 + k];
-    }
-    bias[t] = w->b1[t];
-    bias[128 + t] = w->b2[t];
-    bias[256 + t] = __bfloat162float(w->w3[t]);
     const float b3 = w->b3;
-    if (warp == 0) {
+    if (tid < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(base + tc::kOffTmem),
                      "r"(tc::kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -295,77 +304,113 @@ __global__ void __launch_bounds__(128, 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    const uint32_t d1 = tmem + g * (tc::kTmemCols / kGroups);  // this group's columns
+    const uint32_t d2 = PARTS == 1 ? d1 : d1 + 128;
     const uint32_t lane_off = (warp * 32u) << 16;  // this warp's TMEM lanes
-    const uint32_t d1 = tmem, d2 = tmem + 128;
+    const uint32_t lut = base + tc::kOffLut;
     uint32_t phase = 0;
-    __shared__ int s_fail;
-    if (t == 0) s_fail = 0;
-    __syncthreads();
 
-    for (long long g0 = (long long)blockIdx.x * 128; g0 < n; g0 += (long long)gridDim.x * 128) {
-        // ---- X row of this thread's task (zeros past the end)
-        uint32_t m0 = 0, m1 = 0, m2 = 0;
-        if (g0 + t < n) load_masks(tv, g0 + t, m0, m1, m2);
-        const uint32_t masks[3] = {m0, m1, m2};
-#pragma unroll
-        for (int c = 0; c < kIn / 8; ++c) {
-            const uint32_t byte = (masks[c >> 2] >> ((c & 3) * 8)) & 0xFFu;
-            uint32_t q[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                q[j] = ((byte >> (2 * j)) & 1u ? 0x3F80u : 0u) | ((byte >> (2 * j + 1)) & 1u ? 0x3F800000u : 0u);
-            tc::sts128(base + tc::kOffA + tc::off_kmajor(t, 8 * c, tc::kSbo1), q[0], q[1], q[2], q[3]);
-        }
+    // Waits for the group's MMAs; false when the wait expired for some thread.
+    auto mma_done = [&]() -> bool {
+        if (!tc::wait_phase(bar, phase)) *fail = 1;
+        phase ^= 1u;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        group_sync(g);
+        return *fail == 0;
+    };
+    // Makes the group's operand writes visible to the MMAs.
+    auto operands_ready = [&]() {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
+        group_sync(g);
+    };
+
+    const long long tiles = (n + 127) / 128;
+    const long long step = (long long)gridDim.x * kGroups;
+    long long tile = blockIdx.x + (long long)gridDim.x * g;
+    uint32_t m[3] = {0, 0, 0};
+    if (tile * 128 + t < n) load_masks(tv, tile * 128 + t, m[0], m[1], m[2]);
+    for (; tile < tiles; tile += step) {
+        const long long task = tile * 128 + t;
+        // ---- X row of this thread's task (zeros past the end)
+#pragma unroll
+        for (int c = 0; c < kIn / 8; ++c) {
+            const uint32_t byte = m[c >> 2] >> ((c & 3) * 8);
+            uint32_t q[4];
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(q[0]), "=r"(q[1]) : "r"(lut + (byte & 15u) * 8u));
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(q[2]), "=r"(q[3]) : "r"(lut + (byte >> 4 & 15u) * 8u));
+            tc::sts128(abuf + off_kmajor(t, 8 * c, kSbo1), q[0], q[1], q[2], q[3]);
+        }
+        operands_ready();
         // ---- layer 1 on the tensor cores: D1 = X * W1^T, K = 96 in 6 steps
         if (t == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
             for (int kk = 0; kk < kIn / 16; ++kk)
-                tc::mma(d1, tc::smem_desc(base + tc::kOffA + kk * 256, 128, tc::kSbo1),
-                        tc::smem_desc(base + tc::kOffB1 + kk * 256, 128, tc::kSbo1), kk > 0);
+                tc::mma(d1, tc::smem_desc(abuf + kk * 256, 128, kSbo1),
+                        tc::smem_desc(base + tc::kOffB1 + kk * 256, 128, kSbo1), kk > 0);
             tc::commit(bar);
         }
-        if (!tc::wait_phase(bar, phase)) s_fail = 1;
-        phase ^= 1u;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (s_fail) break;
-        // ---- relu(D1 + b1) -> BF16 -> H1 rows (the A operand of layer 2)
+        m[0] = m[1] = m[2] = 0;  // the next tile's masks load meanwhile
+        if (task + step * 128 < n) load_masks(tv, task + step * 128, m[0], m[1], m[2]);
+        if (!mma_done()) break;
+        // ---- relu(D1 + b1) -> BF16 -> H1 rows (the A operand of layer 2); with
+        // three parts: the first two, then the third over the first's buffer
 #pragma unroll 1
-        for (int c = 0; c < kH1 / 16; ++c) {
-            float v[16];
-            tc::ld16(d1 + lane_off + 16 * c, v);
-            uint32_t q[8];
+        for (int pass = 0; pass < (PARTS == 1 ? 1 : 2); ++pass) {
+#pragma unroll 2
+            for (int c = 0; c < kH1 / 16; ++c) {
+                float v[16];
+                tc::ld16(d1 + lane_off + 16 * c, v);
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                q[j] = tc::pack_bf16(fmaxf(v[2 * j] + bias[16 * c + 2 * j], 0.f),
-                                     fmaxf(v[2 * j + 1] + bias[16 * c + 2 * j + 1], 0.f));
-            tc::sts128(base + tc::kOffA + tc::off_kmajor(t, 16 * c, tc::kSbo2), q[0], q[1], q[2], q[3]);
-            tc::sts128(base + tc::kOffA + tc::off_kmajor(t, 16 * c + 8, tc::kSbo2), q[4], q[5], q[6], q[7]);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        // ---- layer 2: D2 = H1 * W2^T, K = 128 in 8 steps
-        if (t == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j] + bias[16 * c + j], 0.f);
+                uint32_t q[8];
 #pragma unroll
-            for (int kk = 0; kk < kH1 / 16; ++kk)
-                tc::mma(d2, tc::smem_desc(base + tc::kOffA + kk * 256, 128, tc::kSbo2),
-                        tc::smem_desc(base + tc::kOffB2 + kk * 256, 128, tc::kSbo2), kk > 0);
-            tc::commit(bar);
+                for (int j = 0; j < 8; ++j) q[j] = tc::pack_bf16(v[2 * j], v[2 * j + 1]);
+                if (PARTS == 3) {
+                    // what the first part leaves (exact), rounded to the second
+                    uint32_t r[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        v[2 * j] -= __uint_as_float(q[j] << 16);
+                        v[2 * j + 1] -= __uint_as_float(q[j] & 0xffff0000u);
+                        r[j] = tc::pack_bf16(v[2 * j], v[2 * j + 1]);
+                    }
+                    if (pass == 0) {
+                        const uint32_t second = abuf + tc::kABytes;
+                        tc::sts128(second + off_kmajor(t, 16 * c, kSbo2), r[0], r[1], r[2], r[3]);
+                        tc::sts128(second + off_kmajor(t, 16 * c + 8, kSbo2), r[4], r[5], r[6], r[7]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            q[j] = tc::pack_bf16(v[2 * j] - __uint_as_float(r[j] << 16),
+                                                 v[2 * j + 1] - __uint_as_float(r[j] & 0xffff0000u));
+                    }
+                }
+                tc::sts128(abuf + off_kmajor(t, 16 * c, kSbo2), q[0], q[1], q[2], q[3]);
+                tc::sts128(abuf + off_kmajor(t, 16 * c + 8, kSbo2), q[4], q[5], q[6], q[7]);
+            }
+            operands_ready();
+            // ---- layer 2: D2 += H1 part * W2^T, 8 steps for each part
+            if (t == 0) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int kk = 0; kk < kH1 / 16; ++kk)
+                    tc::mma(d2, tc::smem_desc(abuf + kk * 256, 128, kSbo2),
+                            tc::smem_desc(base + tc::kOffB2 + kk * 256, 128, kSbo2), kk > 0 || pass > 0);
+                if (PARTS == 3 && pass == 0)
+#pragma unroll
+                    for (int kk = 0; kk < kH1 / 16; ++kk)
+                        tc::mma(d2, tc::smem_desc(abuf + tc::kABytes + kk * 256, 128, kSbo2),
+                                tc::smem_desc(base + tc::kOffB2 + kk * 256, 128, kSbo2), 1);
+                tc::commit(bar);
+            }
+            if (!mma_done()) break;
         }
-        if (!tc::wait_phase(bar, phase)) s_fail = 1;
-        phase ^= 1u;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (s_fail) break;
+        if (*fail) break;
         // ---- layer 3: sum_j relu(D2 + b2)_j * w3_j + b3
         float acc = 0.f;
-#pragma unroll 1
+#pragma unroll 2
         for (int c = 0; c < kH2 / 16; ++c) {
             float v[16];
             tc::ld16(d2 + lane_off + 16 * c, v);
@@ -373,15 +418,23 @@ __global__ void __launch_bounds__(128, 1)
             for (int j = 0; j < 16; ++j)
                 acc = fmaf(fmaxf(v[j] + bias[128 + 16 * c + j], 0.f), bias[256 + 16 * c + j], acc);
         }
-        if (g0 + t < n) out[g0 + t] = acc + b3;
+        if (task < n) {
+            if (out) out[task] = acc + b3;
+            if (key) {
+                key[task] = order_key(acc + b3);
+                idx[task] = (uint32_t)task;
+            }
+        }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
+        group_sync(g);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
-    if (s_fail && t == 0) atomicExch(err, 1);
+    if (*fail && t == 0) atomicExch(err, 1);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tc::kTmemCols));
+    if (tid < 32)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tc::kTmemCols));
 }
 
 // Shared memory of the training kernel (about 216 KiB; one CTA per SM).
@@ -549,10 +602,13 @@ __device__ __forceinline__ void refresh_one(int p, float v, Weights *w) {
     if (p < kOffB1) {
         const int i = (p - kOffW1) / kIn, f = (p - kOffW1) % kIn;
         w->w1t[f * kH1 + i] = __float2bfloat16_rn(v);
+        w->w1c[off_kmajor(i, f, kSbo1) / 2] = __float2bfloat16_rn(v);
     } else if (p < kOffW2) {
         w->b1[p - kOffB1] = v;
     } else if (p < kOffB2) {
+        const int j = (p - kOffW2) / kH1, i = (p - kOffW2) % kH1;
         w->w2[p - kOffW2] = __float2bfloat16_rn(v);
+        w->w2c[off_kmajor(j, i, kSbo2) / 2] = __float2bfloat16_rn(v);
     } else if (p < kOffW3) {
         w->b2[p - kOffB2] = v;
     } else if (p < kOffB3) {
@@ -586,16 +642,6 @@ __global__ void mlp_adam_kernel(float *master, float *m1, float *m2, const float
         const float nw = master[p] - lr * upd;
         master[p] = nw;
         refresh_one(p, nw, w);
-    }
-}
-
-// Sort keys for the longest-first order: 1 + predicted log2 cost in 1/8
-// units (key 0 is kept for tasks that must go last, mlp_last_kernel).
-__global__ void mlp_bin_kernel(const float *pred, long long n, uint16_t *key, uint32_t *idx) {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const float v = fminf(fmaxf(pred[t] * 8.f + 0.5f, 0.f), 65534.f);
-        key[t] = (uint16_t)(1.f + v);
-        idx[t] = (uint32_t)t;
     }
 }
 
@@ -724,12 +770,38 @@ int launch_train(nq_mlp *m, const TaskView &tv, const float *target, long long b
     return NQ_OK;
 }
 
-// Tensor-core forward over n device-resident tasks of board size N.
-int launch_predict_tc(nq_mlp *m, const TaskView &tv, long long n, float *d_out, cudaStream_t s) {
-    const long long tiles = (n + 127) / 128;
-    const int grid = (int)std::min<long long>(tiles, (long long)m->sms * 2);
-    mlp_predict_tc_kernel<<<grid, 128, tc::kSmemBytes, s>>>(tv, n, m->w, d_out, m->tc_err);
+// Forward pass over n device-resident tasks of board size N (parts: see
+// mlp_forward_kernel).  One CTA per SM; a short list spreads its tiles over the
+// SMs before it fills their groups.
+int launch_forward(nq_mlp *m, int parts, const TaskView &tv, long long n, float *d_out, uint16_t *key, uint32_t *idx,
+                   cudaStream_t s) {
+    const int grid = (int)std::min<long long>((n + 127) / 128, m->sms);
+    if (parts == 1)
+        mlp_forward_kernel<1><<<grid, 512, tc::kSmemBytes, s>>>(tv, n, m->w, d_out, key, idx, m->tc_err);
+    else
+        mlp_forward_kernel<3><<<grid, 256, tc::kSmemBytes, s>>>(tv, n, m->w, d_out, key, idx, m->tc_err);
     MLP_CUDA(cudaGetLastError());
+    return NQ_OK;
+}
+
+// Predictions of n host tasks into a host array.
+int predict_host(nq_mlp *m, int parts, int N, const uint32_t *cols, const uint32_t *ld, const uint32_t *rd, int64_t n,
+                 float *out) {
+    Staged st;
+    int rc = stage(m, nullptr, cols, ld, rd, nullptr, n, st);
+    if (rc) return rc;
+    TaskView tv{st.cols, st.ld, st.rd, nullptr, nullptr, N};
+    MLP_CUDA(cudaMemsetAsync(m->tc_err, 0, sizeof(int), m->stream));
+    rc = launch_forward(m, parts, tv, n, st.target, nullptr, nullptr, m->stream);
+    if (rc) return rc;
+    int err = 0;
+    MLP_CUDA(cudaMemcpyAsync(out, st.target, (size_t)n * 4, cudaMemcpyDeviceToHost, m->stream));
+    MLP_CUDA(cudaMemcpyAsync(&err, m->tc_err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+    MLP_CUDA(cudaStreamSynchronize(m->stream));
+    if (err) {
+        set_last_error("tensor-core MMA completion wait expired");
+        return NQ_ERR_TIMEOUT;
+    }
     return NQ_OK;
 }
 
@@ -768,7 +840,9 @@ int nq_mlp_create(int device, uint64_t seed, nq_mlp **out) try {
     if (e == cudaSuccess) e = cudaMalloc(&m->tc_err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(m->tc_err, 0, sizeof(int));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(mlp_predict_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes);
+        e = cudaFuncSetAttribute(mlp_forward_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(mlp_forward_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(TrainSmem));
     if (e != cudaSuccess) {
@@ -852,17 +926,7 @@ int nq_mlp_predict(nq_mlp *m, int N, const uint32_t *cols, const uint32_t *ld, c
     if (N < 1 || N > NQ_MAX_N || n < 0 || (n > 0 && (!cols || !ld || !rd || !out))) return NQ_ERR_ARG;
     if (n == 0) return NQ_OK;
     std::lock_guard<std::mutex> lock(m->mu);
-    Staged st;
-    rc = stage(m, nullptr, cols, ld, rd, nullptr, n, st);
-    if (rc) return rc;
-    TaskView tv{st.cols, st.ld, st.rd, nullptr, nullptr, N};
-    float *d_out = st.target;
-    const int grid = (int)std::min<long long>((n + kGroup - 1) / kGroup, (long long)m->sms * 8);
-    mlp_predict_kernel<<<grid, kH1, 0, m->stream>>>(tv, n, m->w, d_out);
-    MLP_CUDA(cudaGetLastError());
-    MLP_CUDA(cudaMemcpyAsync(out, d_out, (size_t)n * 4, cudaMemcpyDeviceToHost, m->stream));
-    MLP_CUDA(cudaStreamSynchronize(m->stream));
-    return NQ_OK;
+    return predict_host(m, 3, N, cols, ld, rd, n, out);
 } catch (...) {
     return status_of_exception();
 }
@@ -874,22 +938,7 @@ int nq_mlp_predict_tensor(nq_mlp *m, int N, const uint32_t *cols, const uint32_t
     if (N < 1 || N > NQ_MAX_N || n < 0 || (n > 0 && (!cols || !ld || !rd || !out))) return NQ_ERR_ARG;
     if (n == 0) return NQ_OK;
     std::lock_guard<std::mutex> lock(m->mu);
-    Staged st;
-    rc = stage(m, nullptr, cols, ld, rd, nullptr, n, st);
-    if (rc) return rc;
-    TaskView tv{st.cols, st.ld, st.rd, nullptr, nullptr, N};
-    MLP_CUDA(cudaMemsetAsync(m->tc_err, 0, sizeof(int), m->stream));
-    rc = launch_predict_tc(m, tv, n, st.target, m->stream);
-    if (rc) return rc;
-    int err = 0;
-    MLP_CUDA(cudaMemcpyAsync(out, st.target, (size_t)n * 4, cudaMemcpyDeviceToHost, m->stream));
-    MLP_CUDA(cudaMemcpyAsync(&err, m->tc_err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
-    MLP_CUDA(cudaStreamSynchronize(m->stream));
-    if (err) {
-        set_last_error("tensor-core MMA completion wait expired");
-        return NQ_ERR_TIMEOUT;
-    }
-    return NQ_OK;
+    return predict_host(m, 1, N, cols, ld, rd, n, out);
 } catch (...) {
     return status_of_exception();
 }
@@ -999,19 +1048,16 @@ int nq_schedule_device_last(nq_mlp *m, int N, const uint32_t *d_cols, const uint
     if (n == 0) return NQ_OK;
     std::lock_guard<std::mutex> lock(m->mu);
     cudaStream_t s = (cudaStream_t)stream;  // NULL: the legacy default stream, as in every device entry
-    // scratch: pred f32 | key u16 | key_out u16 | idx u32
-    const size_t need = (size_t)n * (4 + 2 + 2 + 4) + 1024;
+    // scratch: key u16 | key_out u16 | idx u32
+    const size_t need = (size_t)n * (2 + 2 + 4) + 1024;
     rc = grow(m->data, m->data_cap, need);
     if (rc) return rc;
-    float *pred = d_pred ? d_pred : (float *)m->data;
-    uint16_t *key = (uint16_t *)((char *)m->data + (size_t)n * 4);
+    uint16_t *key = (uint16_t *)m->data;
     uint16_t *key2 = key + n;
     uint32_t *idx = (uint32_t *)(((uintptr_t)(key2 + n) + 15) & ~(uintptr_t)15);
     TaskView tv{d_cols, d_ld, d_rd, nullptr, nullptr, N};
-    rc = launch_predict_tc(m, tv, n, pred, s);
+    rc = launch_forward(m, 1, tv, n, d_pred, key, idx, s);
     if (rc) return rc;
-    mlp_bin_kernel<<<m->sms * 4, 256, 0, s>>>(pred, n, key, idx);
-    MLP_CUDA(cudaGetLastError());
     if (n_last > 0) {
         mlp_last_kernel<<<m->sms * 4, 256, 0, s>>>(d_last, n_last, n, key);
         MLP_CUDA(cudaGetLastError());
