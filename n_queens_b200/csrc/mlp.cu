@@ -16,9 +16,8 @@
 //                       partial gradients (no atomics: deterministic)
 //   mlp_adam_kernel     sums the partials in CTA order, Adam step, refreshes
 //                       the BF16 copies
-// The first layer exploits binary inputs: h1 = b1 + sum of the W1 columns of
-// the set bits (about 3k of them for a k-row prefix), so no feature matrix
-// is ever materialised.
+// The training kernel's first layer exploits binary inputs: h1 = b1 + sum of the
+// W1 columns of the set bits (about 3k of them for a k-row prefix).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -52,7 +51,7 @@ constexpr int kOffB2 = kOffW2 + kH2 * kH1;
 constexpr int kOffW3 = kOffB2 + kH2;
 constexpr int kOffB3 = kOffW3 + kH2;
 constexpr int kParams = kOffB3 + 1;
-constexpr int kGroup = 32;  // tasks per group (one per lane of the layer-3 reduction)
+constexpr int kGroup = 32;  // tasks per tile of the training kernel
 
 // Offset (bytes) of element (row, k) of a K-major tensor-core operand without
 // swizzle: 8-row x 16-byte core matrices, sbo bytes between 8-row groups.
@@ -91,52 +90,6 @@ __device__ __forceinline__ void load_masks(const TaskView &tv, long long t, uint
     m0 = tv.cols[i] & last;
     m1 = tv.ld[i] & last;
     m2 = tv.rd[i] & last;
-}
-
-// Layer 1 for one task and hidden unit j: b1[j] + sum of W1 columns of the
-// set input bits.  Every thread of the CTA walks the same bits (uniform).
-__device__ __forceinline__ float layer1(const __nv_bfloat16 *w1t, float b, uint32_t m0, uint32_t m1, uint32_t m2,
-                                        int j) {
-    float acc = b;
-    while (m0) {
-        const int f = __ffs(m0) - 1;
-        m0 &= m0 - 1;
-        acc += __bfloat162float(w1t[f * kH1 + j]);
-    }
-    while (m1) {
-        const int f = __ffs(m1) - 1 + 32;
-        m1 &= m1 - 1;
-        acc += __bfloat162float(w1t[f * kH1 + j]);
-    }
-    while (m2) {
-        const int f = __ffs(m2) - 1 + 64;
-        m2 &= m2 - 1;
-        acc += __bfloat162float(w1t[f * kH1 + j]);
-    }
-    return acc;
-}
-
-// Layer 2 pre-activation of unit j for one task: w2row holds W2[j][:] as
-// 64 packed BF16 pairs, h1 the task's 128 layer-1 outputs (broadcast reads).
-__device__ __forceinline__ float layer2(const uint32_t (&w2row)[kH1 / 2], float b, const float *h1) {
-    float acc = b;
-#pragma unroll
-    for (int i = 0; i < kH1; i += 4) {
-        const float4 h = *reinterpret_cast<const float4 *>(h1 + i);
-        const __nv_bfloat162 wa = *reinterpret_cast<const __nv_bfloat162 *>(&w2row[i / 2]);
-        const __nv_bfloat162 wb = *reinterpret_cast<const __nv_bfloat162 *>(&w2row[i / 2 + 1]);
-        acc = fmaf(__low2float(wa), h.x, acc);
-        acc = fmaf(__high2float(wa), h.y, acc);
-        acc = fmaf(__low2float(wb), h.z, acc);
-        acc = fmaf(__high2float(wb), h.w, acc);
-    }
-    return acc;
-}
-
-__device__ __forceinline__ void load_w2row(const Weights *w, int j, uint32_t (&w2row)[kH1 / 2]) {
-    const uint32_t *src = reinterpret_cast<const uint32_t *>(w->w2 + j * kH1);
-#pragma unroll
-    for (int i = 0; i < kH1 / 2; ++i) w2row[i] = src[i];
 }
 
 // ---------------------------------------------------------------------------
@@ -437,165 +390,270 @@ __global__ void __launch_bounds__(PARTS == 1 ? 512 : 256, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tc::kTmemCols));
 }
 
-// Shared memory of the training kernel (about 216 KiB; one CTA per SM).
+// Training: forward + backward of a minibatch slice in FP32 on the CUDA cores
+// (the gradient of a batch is 0.4 GFLOP; what counts is that every SM works and
+// that a multiply-add costs little more than its own issue slot).  One CTA of 256
+// threads per SM takes tiles of 32 tasks:
+//   H1 = relu(b1 + X W1^T)   bit by bit of X, a warp per task, four units a lane
+//   H2 = relu(b2 + H1 W2^T)  4 tasks x 4 units a thread, steps of 4 along K
+//   out, dout                a warp per task
+//   dH2 = relu' . dout w3    (over H2)
+//   dH1 = relu' . dH2 W2     4 x 4 a thread
+//   dW2 += dH2^T H1          8 x 8 a thread, accumulated in registers
+//   dW1 += dH1^T X           8 x 6 a thread, accumulated in registers
+// The products read rows of 16-byte vectors; rows are padded to 132 floats, so
+// the eight lanes of a quarter-warp that read eight rows cover the banks once.
+// What bounds it: the shared-memory reads of the two 32 x 128 x 128 products (5
+// wavefronts for 16 multiply-adds of a warp), then FMA issue.  4096 tasks: 201 us
+// with 64 CTAs of 128 threads that kept the weight gradients in shared memory and
+// summed one unit per thread, 33 us so; error against 64 bits 1.3e-7 (1.7e-7
+// before).  Pre-training a cost model (2.3e6 tasks, 4 epochs) 562 -> 136 ms.
+constexpr int kTrainThreads = 256;
+constexpr int kPad = kH1 + 4;
+constexpr int kPartStride = (kParams + 3) & ~3;  // floats between partial gradients (16-byte rows)
+
 struct TrainSmem {
-    __nv_bfloat16 w1t[kIn * kH1];    // 24 KiB
-    __nv_bfloat162 w2p[kH2 / 2 * kH1];  // 32 KiB: w2p[(j/2)*H1 + i] = (W2[j][i], W2[j+1][i])
-    float h1[kGroup * kH1];          // 16 KiB: relu(layer 1), [task][unit]
-    float h2[kGroup * kH1];          // 16 KiB: relu(layer 2), then dL/d(pre-act 2)
-    float dh1[kGroup * kH1];         // 16 KiB: dL/d(pre-act 1)
-    float dw1[kIn * kH1];            // 48 KiB: [input bit][unit]
-    float dw2[kH1 * kH2];            // 64 KiB: [unit of layer 1][unit of layer 2]
-    float dout[kGroup];
-    float y[kGroup];
+    float w2[kH2 * kPad];                   // 66 KiB: W2[j][i]
+    float h1[kGroup * kPad];                // 16.5 KiB: relu(layer 1)
+    float h2[kGroup * kPad];                // 16.5 KiB: relu(layer 2), then dL/d(pre-act 2)
+    float dh1[kGroup * kPad];               // 16.5 KiB: dL/d(pre-act 1)
+    float x[kGroup * kIn];                  // 12 KiB: the tasks' bits
+    __nv_bfloat16 w1t[(kIn + 1) * kH1];     // 24.25 KiB: [input bit][unit], row kIn zero
+    float w3[kH2], b1[kH1], b2[kH2];
+    float dout[kGroup], y[kGroup], loss[kTrainThreads / 32];
     uint32_t m[3][kGroup];
 };
 
-// Forward + backward of tasks [begin, end) of the view (mean-squared-error
-// loss with gradient scale `scale` = 2/batch), one partial gradient per CTA.
-__global__ void __launch_bounds__(128, 1)
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+
+// Partial gradient and squared error of tasks [begin, end) of the view
+// (mean-squared-error loss with gradient scale `scale` = 2/batch), one of each
+// per CTA.
+__global__ void __launch_bounds__(kTrainThreads, 1)
     mlp_train_kernel(TaskView tv, const float *target, long long begin, long long end, float scale,
                      const Weights *w, float *grad_part, float *loss_part) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainSmem &S = *reinterpret_cast<TrainSmem *>(smem_raw);
-    const int j = threadIdx.x;  // unit index in every layer (H1 == H2 == blockDim.x)
-    const int warp = j >> 5, lane = j & 31;
-    for (int i = j; i < kIn * kH1 / 8; i += blockDim.x)
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    for (int i = t; i < kIn * kH1 / 8; i += kTrainThreads)
         reinterpret_cast<uint4 *>(S.w1t)[i] = reinterpret_cast<const uint4 *>(w->w1t)[i];
-    for (int jj = 0; jj < kH2; jj += 2)
-        S.w2p[(jj / 2) * kH1 + j] = __halves2bfloat162(w->w2[jj * kH1 + j], w->w2[(jj + 1) * kH1 + j]);
-    for (int i = j; i < kIn * kH1; i += blockDim.x) S.dw1[i] = 0.f;
-    for (int i = j; i < kH1 * kH2; i += blockDim.x) S.dw2[i] = 0.f;
-    uint32_t w2row[kH1 / 2];
-    load_w2row(w, j, w2row);
-    const float b1 = w->b1[j], b2 = w->b2[j], w3 = __bfloat162float(w->w3[j]), b3 = w->b3;
-    float w3q[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) w3q[k] = __bfloat162float(w->w3[lane * 4 + k]);
+    if (t < kH1 / 8) reinterpret_cast<uint4 *>(S.w1t + kIn * kH1)[t] = make_uint4(0, 0, 0, 0);
+    for (int i = t; i < kH2 * kH1 / 2; i += kTrainThreads) {
+        const uint32_t v = reinterpret_cast<const uint32_t *>(w->w2)[i];
+        float *to = S.w2 + (2 * i / kH1) * kPad + 2 * i % kH1;
+        to[0] = __uint_as_float(v << 16);
+        to[1] = __uint_as_float(v & 0xffff0000u);
+    }
+    if (t < kH1) {
+        S.b1[t] = w->b1[t];
+        S.b2[t] = w->b2[t];
+        S.w3[t] = __bfloat162float(w->w3[t]);
+    }
+    const float b3 = w->b3;
+    const int ty = t >> 4, tx = t & 15;     // 16 x 16 threads of the weight gradients
+    const int col = t & (kH1 - 1), half = t >> 7;  // column sums: a unit and half of the tasks
+    float gw2[8][8] = {}, gw1[8][6] = {};
     float gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, loss = 0.f;
     __syncthreads();
 
     for (long long g0 = begin + (long long)blockIdx.x * kGroup; g0 < end; g0 += (long long)gridDim.x * kGroup) {
         const int gn = (int)min((long long)kGroup, end - g0);
-        if (j < kGroup) {
-            if (j < gn) {
-                load_masks(tv, g0 + j, S.m[0][j], S.m[1][j], S.m[2][j]);
-                const long long i = tv.index ? (long long)tv.index[g0 + j] : g0 + j;
-                S.y[j] = target[i];
-            } else {
-                S.m[0][j] = S.m[1][j] = S.m[2][j] = 0;
-                S.y[j] = 0.f;
+        if (t < kGroup) {
+            S.m[0][t] = S.m[1][t] = S.m[2][t] = 0;
+            S.y[t] = 0.f;
+            if (t < gn) {
+                load_masks(tv, g0 + t, S.m[0][t], S.m[1][t], S.m[2][t]);
+                S.y[t] = target[tv.index ? (long long)tv.index[g0 + t] : g0 + t];
             }
         }
         __syncthreads();
-        // forward
-        for (int s = 0; s < gn; ++s)
-            S.h1[s * kH1 + j] = fmaxf(layer1(S.w1t, b1, S.m[0][s], S.m[1][s], S.m[2][s], j), 0.f);
-        __syncthreads();
-        for (int s = 0; s < gn; ++s) S.h2[s * kH1 + j] = fmaxf(layer2(w2row, b2, S.h1 + s * kH1), 0.f);
-        __syncthreads();
-        for (int s = warp * 8; s < warp * 8 + 8; ++s) {
-            const float4 q = *reinterpret_cast<const float4 *>(S.h2 + s * kH1 + lane * 4);
-            float a = q.x * w3q[0];
-            a = fmaf(q.y, w3q[1], a);
-            a = fmaf(q.z, w3q[2], a);
-            a = fmaf(q.w, w3q[3], a);
+        for (int i = t; i < kGroup * kIn; i += kTrainThreads) {
+            const int s = i / kIn, f = i % kIn;
+            S.x[i] = (float)(S.m[f >> 5][s] >> (f & 31) & 1u);
+        }
+        // ---- layer 1, four bits at a time (row kIn of W1t is zero)
+        for (int s = warp; s < kGroup; s += kTrainThreads / 32) {
+            float4 acc = ld4(S.b1 + 4 * lane);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-            if (lane == 0) {
-                const float e = (s < gn) ? (a + b3 - S.y[s]) : 0.f;
-                S.dout[s] = scale * e;
-                loss += e * e;
+            for (int part = 0; part < 3; ++part)
+                for (uint32_t m = S.m[part][s]; m;) {
+                    uint2 v[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int f = m ? 32 * part + __ffs(m) - 1 : kIn;
+                        m &= m - 1;
+                        v[k] = *reinterpret_cast<const uint2 *>(S.w1t + f * kH1 + 4 * lane);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        acc.x += __uint_as_float(v[k].x << 16);
+                        acc.y += __uint_as_float(v[k].x & 0xffff0000u);
+                        acc.z += __uint_as_float(v[k].y << 16);
+                        acc.w += __uint_as_float(v[k].y & 0xffff0000u);
+                    }
+                }
+            *reinterpret_cast<float4 *>(S.h1 + s * kPad + 4 * lane) =
+                make_float4(fmaxf(acc.x, 0.f), fmaxf(acc.y, 0.f), fmaxf(acc.z, 0.f), fmaxf(acc.w, 0.f));
+        }
+        __syncthreads();
+        // ---- layer 2: tasks 4*warp.., units lane + 32 q
+        {
+            float acc[4][4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) acc[r][q] = S.b2[lane + 32 * q];
+            const float *hp = S.h1 + 4 * warp * kPad, *wp = S.w2 + lane * kPad;
+#pragma unroll 4
+            for (int i = 0; i < kH1; i += 4) {
+                float4 h[4], v[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) h[r] = ld4(hp + r * kPad + i);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = ld4(wp + 32 * q * kPad + i);
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        acc[r][q] = fmaf(h[r].x, v[q].x, acc[r][q]);
+                        acc[r][q] = fmaf(h[r].y, v[q].y, acc[r][q]);
+                        acc[r][q] = fmaf(h[r].z, v[q].z, acc[r][q]);
+                        acc[r][q] = fmaf(h[r].w, v[q].w, acc[r][q]);
+                    }
+            }
+            // ---- layer 3 and its error, for the warp's own four tasks
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int s = 4 * warp + r;
+                float a = 0.f;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    acc[r][q] = fmaxf(acc[r][q], 0.f);
+                    S.h2[s * kPad + lane + 32 * q] = acc[r][q];
+                    a = fmaf(acc[r][q], S.w3[lane + 32 * q], a);
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+                if (lane == 0) {
+                    const float e = (s < gn) ? (a + b3 - S.y[s]) : 0.f;
+                    S.dout[s] = scale * e;
+                    loss += e * e;
+                }
             }
         }
         __syncthreads();
-        // layer 3 and layer 2 backward (thread j = unit of layer 2)
-        for (int s = 0; s < gn; ++s) {
-            const float h = S.h2[s * kH1 + j];
-            const float d = S.dout[s];
+        // ---- layer 3 and relu of layer 2 backward
+        for (int s = half * (kGroup / 2); s < (half + 1) * (kGroup / 2); ++s) {
+            const float h = S.h2[s * kPad + col], d = S.dout[s];
             gw3 = fmaf(d, h, gw3);
-            const float dh = (h > 0.f) ? d * w3 : 0.f;
-            S.h2[s * kH1 + j] = dh;
+            const float dh = (h > 0.f) ? d * S.w3[col] : 0.f;
+            S.h2[s * kPad + col] = dh;
             gb2 += dh;
+            if (col == 0) gb3 += d;
         }
-        if (j == 0)
-            for (int s = 0; s < gn; ++s) gb3 += S.dout[s];
         __syncthreads();
-        // dW2[j][i] += sum_s dh2[s][j] * h1[s][i]   (accumulated as dw2[i][j])
-        for (int i0 = 0; i0 < kH1; i0 += 32) {
-            float acc[32];
+        // ---- dH1 = relu' . dH2 W2: tasks 4*warp.., units 4*lane..
+        {
+            float acc[4][4] = {};
+            const float *dp = S.h2 + 4 * warp * kPad, *wp = S.w2 + 4 * lane;
+#pragma unroll 4
+            for (int j = 0; j < kH2; j += 4) {
+                float4 d[4], v[4];
 #pragma unroll
-            for (int k = 0; k < 32; ++k) acc[k] = 0.f;
-            for (int s = 0; s < gn; ++s) {
-                const float d = S.h2[s * kH1 + j];
+                for (int r = 0; r < 4; ++r) d[r] = ld4(dp + r * kPad + j);
 #pragma unroll
-                for (int k = 0; k < 32; k += 4) {
-                    const float4 h = *reinterpret_cast<const float4 *>(S.h1 + s * kH1 + i0 + k);
-                    acc[k] = fmaf(d, h.x, acc[k]);
-                    acc[k + 1] = fmaf(d, h.y, acc[k + 1]);
-                    acc[k + 2] = fmaf(d, h.z, acc[k + 2]);
-                    acc[k + 3] = fmaf(d, h.w, acc[k + 3]);
+                for (int q = 0; q < 4; ++q) v[q] = ld4(wp + (j + q) * kPad);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float dd[4] = {d[r].x, d[r].y, d[r].z, d[r].w};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        acc[r][0] = fmaf(dd[q], v[q].x, acc[r][0]);
+                        acc[r][1] = fmaf(dd[q], v[q].y, acc[r][1]);
+                        acc[r][2] = fmaf(dd[q], v[q].z, acc[r][2]);
+                        acc[r][3] = fmaf(dd[q], v[q].w, acc[r][3]);
+                    }
                 }
             }
 #pragma unroll
-            for (int k = 0; k < 32; ++k) S.dw2[(i0 + k) * kH2 + j] += acc[k];
-        }
-        // dh1[s][i] = relu'(h1) * sum_j W2[j][i] dh2[s][j]   (thread j acts as unit i of layer 1)
-        for (int s = 0; s < gn; ++s) {
-            float acc = 0.f;
-            const float *dh2 = S.h2 + s * kH1;
-#pragma unroll 8
-            for (int jj = 0; jj < kH2; jj += 4) {
-                const float4 d = *reinterpret_cast<const float4 *>(dh2 + jj);
-                const __nv_bfloat162 wa = S.w2p[(jj / 2) * kH1 + j];
-                const __nv_bfloat162 wb = S.w2p[(jj / 2 + 1) * kH1 + j];
-                acc = fmaf(__low2float(wa), d.x, acc);
-                acc = fmaf(__high2float(wa), d.y, acc);
-                acc = fmaf(__low2float(wb), d.z, acc);
-                acc = fmaf(__high2float(wb), d.w, acc);
+            for (int r = 0; r < 4; ++r) {
+                const int s = 4 * warp + r;
+                const float4 h = ld4(S.h1 + s * kPad + 4 * lane);
+                *reinterpret_cast<float4 *>(S.dh1 + s * kPad + 4 * lane) =
+                    make_float4(h.x > 0.f ? acc[r][0] : 0.f, h.y > 0.f ? acc[r][1] : 0.f, h.z > 0.f ? acc[r][2] : 0.f,
+                                h.w > 0.f ? acc[r][3] : 0.f);
             }
-            const float dh = (S.h1[s * kH1 + j] > 0.f) ? acc : 0.f;
-            S.dh1[s * kH1 + j] = dh;
-            gb1 += dh;
         }
         __syncthreads();
-        // dW1[i][f] += sum_s dh1[s][i] over the set bits f of task s
-        for (int s = 0; s < gn; ++s) {
-            const float d = S.dh1[s * kH1 + j];
-            uint32_t m0 = S.m[0][s], m1 = S.m[1][s], m2 = S.m[2][s];
-            while (m0) {
-                const int f = __ffs(m0) - 1;
-                m0 &= m0 - 1;
-                S.dw1[f * kH1 + j] += d;
-            }
-            while (m1) {
-                const int f = __ffs(m1) - 1 + 32;
-                m1 &= m1 - 1;
-                S.dw1[f * kH1 + j] += d;
-            }
-            while (m2) {
-                const int f = __ffs(m2) - 1 + 64;
-                m2 &= m2 - 1;
-                S.dw1[f * kH1 + j] += d;
-            }
+        // ---- dW2 and dW1: rows 4*ty + {0..3, 64..67}; columns 4*tx + {0..3, 64..67}
+        // of dW2 and 2*tx + 32*q + {0, 1} of dW1
+#pragma unroll 2
+        for (int s = 0; s < kGroup; ++s) {
+            const float4 da = ld4(S.h2 + s * kPad + 4 * ty), db = ld4(S.h2 + s * kPad + 64 + 4 * ty);
+            const float4 ha = ld4(S.h1 + s * kPad + 4 * tx), hb = ld4(S.h1 + s * kPad + 64 + 4 * tx);
+            const float d[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
+            const float h[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
+#pragma unroll
+            for (int a = 0; a < 8; ++a)
+#pragma unroll
+                for (int b = 0; b < 8; ++b) gw2[a][b] = fmaf(d[a], h[b], gw2[a][b]);
         }
+#pragma unroll 2
+        for (int s = 0; s < kGroup; ++s) {
+            const float4 da = ld4(S.dh1 + s * kPad + 4 * ty), db = ld4(S.dh1 + s * kPad + 64 + 4 * ty);
+            const float d[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
+            float x[6];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const float2 v = *reinterpret_cast<const float2 *>(S.x + s * kIn + 2 * tx + 32 * q);
+                x[2 * q] = v.x;
+                x[2 * q + 1] = v.y;
+            }
+#pragma unroll
+            for (int a = 0; a < 8; ++a)
+#pragma unroll
+                for (int b = 0; b < 6; ++b) gw1[a][b] = fmaf(d[a], x[b], gw1[a][b]);
+        }
+        for (int s = half * (kGroup / 2); s < (half + 1) * (kGroup / 2); ++s) gb1 += S.dh1[s * kPad + col];
         __syncthreads();
     }
 
-    // Partial gradient of this CTA in the flat parameter layout.
-    float *g = grad_part + (size_t)blockIdx.x * kParams;
-    for (int f = 0; f < kIn; ++f) g[kOffW1 + j * kIn + f] = S.dw1[f * kH1 + j];
-    g[kOffB1 + j] = gb1;
-    for (int i = 0; i < kH1; ++i) g[kOffW2 + j * kH1 + i] = S.dw2[i * kH2 + j];
-    g[kOffB2 + j] = gb2;
-    g[kOffW3 + j] = gw3;
-    if (j == 0) g[kOffB3] = gb3;
-    // loss: lanes 0 of each warp hold partial sums
-    __shared__ float s_loss[4];
-    if (lane == 0) s_loss[warp] = loss;
+    // ---- partial gradient of this CTA in the flat parameter layout
+    float *g = grad_part + (size_t)blockIdx.x * kPartStride;
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+        const int row = 4 * ty + (a & 3) + 16 * (a & 4);
+        float *g1 = g + kOffW1 + row * kIn + 2 * tx, *g2 = g + kOffW2 + row * kH1 + 4 * tx;
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+            *reinterpret_cast<float2 *>(g1 + 32 * q) = make_float2(gw1[a][2 * q], gw1[a][2 * q + 1]);
+        *reinterpret_cast<float4 *>(g2) = make_float4(gw2[a][0], gw2[a][1], gw2[a][2], gw2[a][3]);
+        *reinterpret_cast<float4 *>(g2 + 64) = make_float4(gw2[a][4], gw2[a][5], gw2[a][6], gw2[a][7]);
+    }
+    // column sums: the second half of the tasks through shared memory
+    float *other = S.h1;
+    if (half) {
+        other[col] = gb1;
+        other[kH1 + col] = gb2;
+        other[2 * kH1 + col] = gw3;
+        if (col == 0) other[3 * kH1] = gb3;
+    }
+    if (lane == 0) S.loss[warp] = loss;
     __syncthreads();
-    if (j == 0) loss_part[blockIdx.x] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
+    if (!half) {
+        g[kOffB1 + col] = gb1 + other[col];
+        g[kOffB2 + col] = gb2 + other[kH1 + col];
+        g[kOffW3 + col] = gw3 + other[2 * kH1 + col];
+        if (col == 0) g[kOffB3] = gb3 + other[3 * kH1];
+    }
+    if (t == 0) {
+        float l = 0.f;
+        for (int k = 0; k < kTrainThreads / 32; ++k) l += S.loss[k];
+        loss_part[blockIdx.x] = l;
+    }
 }
+static_assert(sizeof(TrainSmem) <= 227 * 1024, "shared memory of one CTA");
+static_assert(kGroup == 4 * (kTrainThreads / 32) && kOffW2 % 4 == 0 && kOffW1 % 2 == 0, "tile and vector layout");
 
 // Master weights -> compute copy (round to nearest even BF16).
 __device__ __forceinline__ void refresh_one(int p, float v, Weights *w) {
@@ -623,26 +681,38 @@ __global__ void mlp_refresh_kernel(const float *master, Weights *w) {
         refresh_one(p, master[p], w);
 }
 
-// Sums the per-CTA partial gradients in CTA order (deterministic), applies
-// one Adam step to the master weights and refreshes the compute copy.
-// nparts == 0 only sums (gradient check): grad_out receives the gradient.
-__global__ void mlp_adam_kernel(float *master, float *m1, float *m2, const float *grad_part, int nparts,
-                                float lr, float beta1, float beta2, float eps, float bc1, float bc2, Weights *w,
-                                float *grad_out, int apply) {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < kParams; p += gridDim.x * blockDim.x) {
-        float g = 0.f;
-        for (int b = 0; b < nparts; ++b) g += grad_part[(size_t)b * kParams + p];
-        if (grad_out) grad_out[p] = g;
-        if (!apply) continue;
-        const float a = beta1 * m1[p] + (1.f - beta1) * g;
-        const float v = beta2 * m2[p] + (1.f - beta2) * g * g;
-        m1[p] = a;
-        m2[p] = v;
-        const float upd = (a / bc1) / (sqrtf(v / bc2) + eps);
-        const float nw = master[p] - lr * upd;
-        master[p] = nw;
-        refresh_one(p, nw, w);
+// Sums the per-CTA partial gradients (deterministic: four interleaved runs over
+// the CTAs, then those in order), applies one Adam step to the master weights and
+// refreshes the compute copy.  With apply == 0 it only sums (gradient check):
+// grad_out receives the gradient.  64 parameters x 4 runs per CTA: the reads of
+// 15 MB of partials (128 CTAs) have four times the loads in flight of one thread
+// per parameter.
+constexpr int kSumRuns = 4, kSumParams = 64;
+__global__ void __launch_bounds__(kSumRuns * kSumParams)
+    mlp_adam_kernel(float *master, float *m1, float *m2, const float *grad_part, int nparts, float lr, float beta1,
+                    float beta2, float eps, float bc1, float bc2, Weights *w, float *grad_out, int apply) {
+    __shared__ float s_sum[kSumRuns][kSumParams];
+    const int x = threadIdx.x % kSumParams, run = threadIdx.x / kSumParams;
+    const int p = blockIdx.x * kSumParams + x;
+    float g = 0.f;
+    if (p < kParams) {
+#pragma unroll 8
+        for (int b = run; b < nparts; b += kSumRuns) g += grad_part[(size_t)b * kPartStride + p];
     }
+    s_sum[run][x] = g;
+    __syncthreads();
+    if (run || p >= kParams) return;
+    g = (s_sum[0][x] + s_sum[1][x]) + (s_sum[2][x] + s_sum[3][x]);
+    if (grad_out) grad_out[p] = g;
+    if (!apply) return;
+    const float a = beta1 * m1[p] + (1.f - beta1) * g;
+    const float v = beta2 * m2[p] + (1.f - beta2) * g * g;
+    m1[p] = a;
+    m2[p] = v;
+    const float upd = (a / bc1) / (sqrtf(v / bc2) + eps);
+    const float nw = master[p] - lr * upd;
+    master[p] = nw;
+    refresh_one(p, nw, w);
 }
 
 // Moves the listed tasks behind every other task of the order (key 0).
@@ -665,6 +735,7 @@ struct nq_mlp {
     int device = 0;
     int sms = 0;
     cudaStream_t stream = nullptr;
+    void *block = nullptr;  // holds the next five and tc_err
     float *master = nullptr, *adam1 = nullptr, *adam2 = nullptr;
     Weights *w = nullptr;
     long long steps = 0;
@@ -673,7 +744,8 @@ struct nq_mlp {
     int grad_parts_cap = 0;
     float *gsum = nullptr;  // summed gradient (nq_mlp_grad)
     int *tc_err = nullptr;  // set by the tensor-core kernel when an MMA wait expires
-    float *loss_part = nullptr;
+    void *loss_part = nullptr;  // floats
+    size_t loss_cap = 0;
     void *data = nullptr;
     size_t data_cap = 0;
     void *sort_tmp = nullptr;
@@ -743,31 +815,38 @@ int stage(nq_mlp *m, const uint8_t *task_n, const uint32_t *cols, const uint32_t
     return NQ_OK;
 }
 
-int ensure_grad_parts(nq_mlp *m, int parts) {
-    if (parts <= m->grad_parts_cap) return NQ_OK;
-    if (m->grad_part) cudaFree(m->grad_part);
-    if (m->loss_part) cudaFree(m->loss_part);
-    m->grad_part = nullptr;
-    m->loss_part = nullptr;
-    MLP_CUDA(cudaMalloc(&m->grad_part, (size_t)parts * kParams * sizeof(float)));
-    MLP_CUDA(cudaMalloc(&m->loss_part, (size_t)parts * sizeof(float)));
-    m->grad_parts_cap = parts;
+// Room for `parts` partial gradients and `losses` partial losses.
+int ensure_grad_parts(nq_mlp *m, int parts, size_t losses) {
+    if (parts > m->grad_parts_cap) {
+        if (m->grad_part) cudaFree(m->grad_part);
+        m->grad_part = nullptr;
+        m->grad_parts_cap = 0;
+        MLP_CUDA(cudaMalloc(&m->grad_part, (size_t)parts * kPartStride * sizeof(float)));
+        m->grad_parts_cap = parts;
+    }
+    return grow(m->loss_part, m->loss_cap, losses * sizeof(float));
+}
+
+// CTAs (and partial gradients) of a minibatch of `count` tasks: one per tile of
+// kGroup tasks up to one per SM (the kernel takes most of its shared memory).
+int train_parts(nq_mlp *m, long long count) {
+    return (int)std::min<long long>(train_blocks(m), std::max<long long>((count + kGroup - 1) / kGroup, 1));
+}
+
+// One forward+backward over [begin, end) into the first `parts` partial
+// gradients and d_loss[0..parts).
+int launch_train(nq_mlp *m, const TaskView &tv, const float *target, long long begin, long long end, float scale,
+                 int parts, float *d_loss) {
+    mlp_train_kernel<<<parts, kTrainThreads, sizeof(TrainSmem), m->stream>>>(tv, target, begin, end, scale, m->w,
+                                                                             m->grad_part, d_loss);
+    MLP_CUDA(cudaGetLastError());
     return NQ_OK;
 }
 
-// One forward+backward over [begin, end) into the partials; returns #parts.
-int launch_train(nq_mlp *m, const TaskView &tv, const float *target, long long begin, long long end, float scale,
-                 int &parts) {
-    // Two groups of 32 tasks per CTA amortise the CTA's weight load and its
-    // partial-gradient write; at most one CTA per SM (the kernel takes ~216 KiB).
-    const long long groups = (end - begin + kGroup - 1) / kGroup;
-    parts = (int)std::min<long long>(train_blocks(m), std::max<long long>((groups + 1) / 2, 1));
-    int rc = ensure_grad_parts(m, parts);
-    if (rc) return rc;
-    mlp_train_kernel<<<parts, kH1, sizeof(TrainSmem), m->stream>>>(tv, target, begin, end, scale, m->w,
-                                                                    m->grad_part, m->loss_part);
-    MLP_CUDA(cudaGetLastError());
-    return NQ_OK;
+void launch_adam(nq_mlp *m, int parts, float lr, float beta1, float beta2, float eps, float bc1, float bc2,
+                 float *grad_out, int apply) {
+    mlp_adam_kernel<<<(kParams + kSumParams - 1) / kSumParams, kSumRuns * kSumParams, 0, m->stream>>>(
+        m->master, m->adam1, m->adam2, m->grad_part, parts, lr, beta1, beta2, eps, bc1, bc2, m->w, grad_out, apply);
 }
 
 // Forward pass over n device-resident tasks of board size N (parts: see
@@ -832,12 +911,17 @@ int nq_mlp_create(int device, uint64_t seed, nq_mlp **out) try {
     m->device = device;
     cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device);
     cudaError_t e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&m->master, kParams * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&m->adam1, kParams * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&m->adam2, kParams * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&m->w, sizeof(Weights));
-    if (e == cudaSuccess) e = cudaMalloc(&m->gsum, kParams * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&m->tc_err, sizeof(int));
+    // one allocation for everything whose size is known here
+    auto room = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+    const size_t vec = room(kParams * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc(&m->block, 4 * vec + room(sizeof(Weights)) + room(sizeof(int)));
+    char *at = (char *)m->block;
+    for (float **v : {&m->master, &m->adam1, &m->adam2, &m->gsum}) {
+        *v = (float *)at;
+        at += vec;
+    }
+    m->w = (Weights *)at;
+    m->tc_err = (int *)(at + room(sizeof(Weights)));
     if (e == cudaSuccess) e = cudaMemset(m->tc_err, 0, sizeof(int));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(mlp_forward_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes);
@@ -873,12 +957,7 @@ int nq_mlp_destroy(nq_mlp *m) try {
     if (!m) return NQ_OK;
     cudaSetDevice(m->device);
     if (m->stream) cudaStreamSynchronize(m->stream);
-    cudaFree(m->master);
-    cudaFree(m->adam1);
-    cudaFree(m->adam2);
-    cudaFree(m->w);
-    cudaFree(m->gsum);
-    cudaFree(m->tc_err);
+    cudaFree(m->block);
     cudaFree(m->grad_part);
     cudaFree(m->loss_part);
     cudaFree(m->data);
@@ -953,11 +1032,12 @@ int nq_mlp_grad(nq_mlp *m, const uint8_t *task_n, const uint32_t *cols, const ui
     rc = stage(m, task_n, cols, ld, rd, target, n, st);
     if (rc) return rc;
     TaskView tv{st.cols, st.ld, st.rd, st.task_n, nullptr, 0};
-    int parts = 0;
-    rc = launch_train(m, tv, st.target, 0, n, 2.f / (float)n, parts);
+    const int parts = train_parts(m, n);
+    rc = ensure_grad_parts(m, parts, parts);
     if (rc) return rc;
-    mlp_adam_kernel<<<(kParams + 255) / 256, 256, 0, m->stream>>>(m->master, m->adam1, m->adam2, m->grad_part,
-                                                                  parts, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f, m->w, m->gsum, 0);
+    rc = launch_train(m, tv, st.target, 0, n, 2.f / (float)n, parts, (float *)m->loss_part);
+    if (rc) return rc;
+    launch_adam(m, parts, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f, m->gsum, 0);
     cudaError_t e = cudaGetLastError();
     std::vector<float> lp(parts);
     if (e == cudaSuccess)
@@ -990,10 +1070,12 @@ int nq_mlp_train(nq_mlp *m, const uint8_t *task_n, const uint32_t *cols, const u
     if (rc) return rc;
     std::vector<uint32_t> perm((size_t)n);
     uint64_t s = seed;
-    const int parts_max = train_blocks(m);
-    rc = ensure_grad_parts(m, parts_max);
-    if (rc) return rc;
+    const int parts_max = train_parts(m, batch);
     const long long nsteps_epoch = (n + batch - 1) / batch;
+    // The losses of an epoch's steps stay on the device until its end: a copy per
+    // step would make the host wait for each.
+    rc = ensure_grad_parts(m, parts_max, (size_t)parts_max * nsteps_epoch);
+    if (rc) return rc;
     std::vector<float> lp((size_t)parts_max * nsteps_epoch);
     for (int ep = 0; ep < epochs; ++ep) {
         // Fisher-Yates shuffle from SplitMix64(seed), one per epoch.
@@ -1007,23 +1089,20 @@ int nq_mlp_train(nq_mlp *m, const uint8_t *task_n, const uint32_t *cols, const u
         double eloss = 0;
         for (long long b0 = 0, stepi = 0; b0 < n; b0 += batch, ++stepi) {
             const long long b1 = std::min<long long>(n, b0 + batch);
-            int parts = 0;
-            rc = launch_train(m, tv, st.target, b0, b1, 2.f / (float)(b1 - b0), parts);
+            const int parts = train_parts(m, b1 - b0);
+            float *d_loss = (float *)m->loss_part + (size_t)stepi * parts_max;
+            rc = launch_train(m, tv, st.target, b0, b1, 2.f / (float)(b1 - b0), parts, d_loss);
             if (rc) return rc;
+            if (parts < parts_max) MLP_CUDA(cudaMemsetAsync(d_loss + parts, 0, (parts_max - parts) * 4, m->stream));
             m->steps += 1;
             const float bc1 = 1.f - std::pow(0.9f, (float)m->steps);
             const float bc2 = 1.f - std::pow(0.999f, (float)m->steps);
-            mlp_adam_kernel<<<(kParams + 255) / 256, 256, 0, m->stream>>>(m->master, m->adam1, m->adam2,
-                                                                          m->grad_part, parts, lr, 0.9f, 0.999f,
-                                                                          1e-8f, bc1, bc2, m->w, nullptr, 1);
+            launch_adam(m, parts, lr, 0.9f, 0.999f, 1e-8f, bc1, bc2, nullptr, 1);
             MLP_CUDA(cudaGetLastError());
-            if (epoch_loss)
-                MLP_CUDA(cudaMemcpyAsync(lp.data() + (size_t)stepi * parts_max, m->loss_part, parts * sizeof(float),
-                                         cudaMemcpyDeviceToHost, m->stream));
-            if (epoch_loss && parts < parts_max)
-                for (int q = parts; q < parts_max; ++q) lp[(size_t)stepi * parts_max + q] = 0.f;
         }
         if (epoch_loss) {
+            MLP_CUDA(cudaMemcpyAsync(lp.data(), m->loss_part, lp.size() * sizeof(float), cudaMemcpyDeviceToHost,
+                                     m->stream));
             MLP_CUDA(cudaStreamSynchronize(m->stream));
             for (float v : lp) eloss += v;
             epoch_loss[ep] = (float)(eloss / (double)n);
