@@ -67,12 +67,18 @@ double now_ms() {
 
 typedef void (*KernelFn)(DfsParams);
 
-KernelFn pick_kernel(bool per_owner, bool nodes, bool dih = false) {
+// tight: a count launch without room for kExtraSlots.
+KernelFn pick_kernel(bool per_owner, bool nodes, bool dih = false, bool tight = false) {
     if (dih) return per_owner ? dfs_kernel<true, false, kDihStepVar, kDihUnroll, false, true>
                               : dfs_kernel<false, false, kDihStepVar, kDihUnroll, false, true>;
-    if (per_owner)
-        return nodes ? dfs_kernel<true, true, kNodesStepVar, kNodesUnroll> : dfs_kernel<true, false, kStepVar, kCountUnroll>;
-    return nodes ? dfs_kernel<false, true, kNodesStepVar, kNodesUnroll> : dfs_kernel<false, false, kStepVar, kCountUnroll>;
+    if (nodes)
+        return per_owner ? dfs_kernel<true, true, kNodesStepVar, kNodesUnroll>
+                         : dfs_kernel<false, true, kNodesStepVar, kNodesUnroll>;
+    if (tight)
+        return per_owner ? dfs_kernel<true, false, kTightStepVar, kCountUnroll>
+                         : dfs_kernel<false, false, kTightStepVar, kCountUnroll>;
+    return per_owner ? dfs_kernel<true, false, kStepVar, kCountUnroll>
+                     : dfs_kernel<false, false, kStepVar, kCountUnroll>;
 }
 
 struct DevBuf {
@@ -160,11 +166,14 @@ int ensure_ready(Ctx &c, int dev) {
     NQ_CUDA(cudaStreamSynchronize(c.stream));  // launches may use any stream
     // Dynamic shared memory above 48 KiB needs an opt-in per kernel.
     const int static_smem = kDfsStaticSmem;
-    for (int po = 0; po < 2; ++po)
+    for (int po = 0; po < 2; ++po) {
         for (int nd = 0; nd < 2; ++nd)
             NQ_CUDA(cudaFuncSetAttribute(pick_kernel(po, nd), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          c.smem_optin - static_smem));
-    NQ_CUDA(cudaFuncSetAttribute(dfs_kernel<false, false, kStepVar, kCountUnroll, true>,
+        NQ_CUDA(cudaFuncSetAttribute(pick_kernel(po, false, false, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     c.smem_optin - static_smem));
+    }
+    NQ_CUDA(cudaFuncSetAttribute(dfs_kernel<false, false, kTightStepVar, kCountUnroll, true>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, c.smem_optin - static_smem));
     NQ_CUDA(cudaFuncSetAttribute(dfs_kernel<false, false, kDihResumeStepVar, kUnroll, true, true>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, c.smem_optin - static_smem));
@@ -196,6 +205,8 @@ int lock_device(int dev, Ctx *&out) {
 struct Launch {
     int threads = 0, levels = 0, smem = 0, grid = 0, inner = 0, steal = 1, layout = 0;
     bool dih = false;  // dihedral-decomposition kernel
+    bool tight = false;  // count kernel without its extra slots
+    int slots = 0;     // stack slots per lane of the launch: levels, and the count kernel's extra ones
     bool auto_inner = true;  // inner is the default, not the caller's
 };
 
@@ -203,8 +214,9 @@ struct Launch {
 // resident CTAs per SM as shared memory and registers allow.  Default CTA
 // size: resident_warp_threads (launch.h), the one that keeps the most warps
 // resident per SM for this stack depth.
+// `resumable`: for a resumable kernel, which runs without the extra slots.
 int plan_launch(Ctx &c, const nq_config *cfg, int levels_needed, bool per_owner, bool nodes, Launch &L,
-                bool dih = false) {
+                bool dih = false, bool resumable = false) {
     L.dih = dih;
     L.levels = std::max(1, levels_needed);
     if (cfg && cfg->stack_levels > NQ_MAX_STACK_LEVELS) {
@@ -220,17 +232,23 @@ int plan_launch(Ctx &c, const nq_config *cfg, int levels_needed, bool per_owner,
     }
     const int cap_per_sm = (cfg && cfg->blocks_per_sm > 0) ? std::min(cfg->blocks_per_sm, kMaxBlocksPerSm)
                                                            : kMaxBlocksPerSm;
-    const bool plain = !(cfg && (cfg->block_threads || cfg->blocks_per_sm > 0)) && L.levels <= NQ_MAX_STACK_LEVELS;
+    const bool counts = !nodes && !dih;
+    L.tight = counts && (resumable || (cfg && cfg->block_threads > 0 &&
+                                       !extra_slots_fit(cfg->block_threads, L.levels, c.smem_optin)));
+    L.slots = L.levels + (counts && !L.tight ? kExtraSlots : 0);
+    const KernelFn fn = pick_kernel(per_owner, nodes, dih, L.tight);
+    const bool plain = !(cfg && (cfg->block_threads || cfg->blocks_per_sm > 0)) && !resumable &&
+                       L.levels <= NQ_MAX_STACK_LEVELS;
     Shape *known = plain ? &c.shapes[per_owner][nodes][dih][L.levels] : nullptr;
     int per_sm = 0;
     if (known && known->threads) {
         L.threads = known->threads;
         per_sm = known->per_sm;
-        L.smem = (L.threads / 32) * L.levels * (int)kSlotBytes;
+        L.smem = (L.threads / 32) * L.slots * (int)kSlotBytes;
     } else {
         L.threads = (cfg && cfg->block_threads)
                         ? cfg->block_threads
-                        : resident_warp_threads(pick_kernel(per_owner, nodes, dih), L.levels, c.smem_optin, cap_per_sm);
+                        : resident_warp_threads(fn, L.slots, c.smem_optin, cap_per_sm);
         if (!(cfg && cfg->block_threads) && L.threads == 0) {
             g_last_error = "no CTA size of 64 or more threads fits this stack depth in shared memory";
             return NQ_ERR_DEPTH;
@@ -239,14 +257,13 @@ int plan_launch(Ctx &c, const nq_config *cfg, int levels_needed, bool per_owner,
             g_last_error = "block_threads must be a multiple of 32 in [32, 1024]";
             return NQ_ERR_ARG;
         }
-        const long long smem = (long long)(L.threads / 32) * L.levels * kSlotBytes;
+        const long long smem = (long long)(L.threads / 32) * L.slots * kSlotBytes;
         if (smem + kDfsStaticSmem > c.smem_optin) {
             g_last_error = "per-CTA stack does not fit in shared memory: lower block_threads";
             return NQ_ERR_DEPTH;
         }
         L.smem = (int)smem;
-        NQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_kernel(per_owner, nodes, dih),
-                                                              L.threads, L.smem));
+        NQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, L.threads, L.smem));
         if (per_sm <= 0) {
             g_last_error = "launch configuration cannot be resident";
             return NQ_ERR_ARG;
@@ -277,7 +294,7 @@ void fill_stats_launch(nq_stats *st, const Launch &L) {
 
 // Enqueues queue reset + kernel on stream s.
 int enqueue_dfs(Ctx &c, DfsParams p, const Launch &L, bool per_owner, bool nodes, cudaStream_t s) {
-    p.levels = L.levels;
+    p.levels = L.slots;
     p.inner = L.inner;
     p.steal = L.steal;
     p.layout = L.layout;
@@ -294,7 +311,7 @@ int enqueue_dfs(Ctx &c, DfsParams p, const Launch &L, bool per_owner, bool nodes
     }
     set_shares(p, (long long)L.grid * L.threads);
     if (p.lg_coarse > 0 && L.auto_inner) p.inner = kShareInner;
-    pick_kernel(per_owner, nodes, L.dih)<<<L.grid, L.threads, L.smem, s>>>(p);
+    pick_kernel(per_owner, nodes, L.dih, L.tight)<<<L.grid, L.threads, L.smem, s>>>(p);
     NQ_CUDA(cudaGetLastError());
     return NQ_OK;
 }
@@ -983,9 +1000,9 @@ int count_resumable_impl(int N, int rows, const nq_config *cfg, const char *chec
         NQ_CUDA(cudaMemcpyAsync(d_cont_in, ck.cont.data(), ncont * 16, cudaMemcpyHostToDevice, c.stream));
         if (dih) NQ_CUDA(cudaMemcpyAsync(d_cont_cls, ck.cls.data(), ncont, cudaMemcpyHostToDevice, c.stream));
     }
-    KernelFn fn = dih ? dfs_kernel<false, false, kDihResumeStepVar, kUnroll, true, true> : dfs_kernel<false, false, kStepVar, kCountUnroll, true>;
+    KernelFn fn = dih ? dfs_kernel<false, false, kDihResumeStepVar, kUnroll, true, true> : dfs_kernel<false, false, kTightStepVar, kCountUnroll, true>;
     Launch L;
-    rc = plan_launch(c, cfg, stack_need(N, rows, !dih), false, false, L, dih);
+    rc = plan_launch(c, cfg, stack_need(N, rows, !dih), false, false, L, dih, true);
     if (rc) return rc;
     {
         // the resumable instantiation may fit fewer CTAs per SM

@@ -8,7 +8,7 @@
 //    (cols, ld, rd, avail); only levels that still have untried columns are
 //    pushed to the lane's shared-memory stack, so a pop always resumes a level
 //    with work and every DFS step places exactly one queen.
-//  * The count kernels' step (VAR 4) lists only a level's alive columns --
+//  * The count kernels' step (VAR 6) lists only a level's alive columns --
 //    those whose child still has a free column in the next row -- skips
 //    children whose row two below has none, and counts the completions of a
 //    row N-2 level from its alive columns instead of stepping rows N-2 and N-1
@@ -335,10 +335,6 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "shr.s32 pos, xr, 1;\n\t"                                                         \
     "lop3.and.b32 t|pg, nc, t, pos, 0x01, pg;\n\t"
 
-#define NQB_STEP4_NODES                                                               \
-    "popc.b32 t, na;\n\t"                                                             \
-    "@pb mad.lo.s32 %6, t, %8, %6;\n\t"
-
 #define NQB_STEP4_TAIL                                                                \
     "lop3.and.b32 naf|pd, na, ma, mb, 0xE0, pg;\n\t"                                  \
     "popc.b32 t, naf;\n\t"                                                            \
@@ -356,18 +352,90 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "@pq ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
 
 #define NQB_STEP4 NQB_STEP4_CHILD NQB_STEP4_LOOK NQB_STEP4_TAIL
+#define NQB_STEP4_X4 NQB_STEP4 NQB_STEP4 NQB_STEP4 NQB_STEP4
+#define NQB_STEP4_X16 NQB_STEP4_X4 NQB_STEP4_X4 NQB_STEP4_X4 NQB_STEP4_X4
+
+// VAR 6: VAR 4 in place, the default.  VAR 4 computes a child beside its parent
+// and moves it over (four predicated moves) if it is entered.  Here the parent's
+// remaining columns are pushed first, whether the child lives or not, the child
+// is computed in the level's own registers, and a child that is not entered
+// (dead, or counted on row N-2) is undone by the pop that a finished level needs
+// anyway.  30 operations instead of 34, for more stack traffic: a step pushes
+// whenever columns remain (38 % of the steps, VAR 4 27 %), and one more slot, for
+// the push on row N-3.  A lane without work must stay without: a step that enters
+// nothing clears avail before the pop, which only a lane with a stacked level
+// does.  Bound by issue (82 %; ALU 77 %, FMA 58 %, shared-memory wavefronts 74 %
+// at N=18).  N=19, k=6 145.2 -> 132.1 ms, 1.1e6
+// prefixes of N=18 18.5 -> 17.5 ms, 8 % of N=21's 839 -> 757 ms.
+// Launches whose stated CTA size and stack depth leave no room for that slot run
+// VAR 4, and so do the resumable kernels.
+#define NQB_STEP6_HEAD                                                                \
+    "{\n\t"                                                                           \
+    ".reg .pred pt1, pb, pg, p2, pd, pp, pq;\n\t"                                     \
+    ".reg .b32 t, bit, na, f0, lo, ma, mb, pos, pc;\n\t"                              \
+    "setp.ne.u32 pt1, %8, 0;\n\t"
+
+#define NQB_STEP6_PUSH                                                                \
+    "mul.lo.s32 t, %3, %10;\n\t"                                                      \
+    "lop3.and.b32 bit|pb, t, %3, 0, 0xC0, pt1;\n\t"                                   \
+    "lop3.and.b32 %3|pp, %3, bit, 0, 0x3C, pt1;\n\t"                                  \
+    "@pp st.shared.v4.u32 [%4], {%0, %1, %2, %3};\n\t"                                \
+    "@pp mad.lo.s32 %4, %8, %11, %4;\n\t"                                             \
+    "mad.lo.s32 %0, bit, %8, %0;\n\t"                                                 \
+    "mad.lo.s32 %1, bit, %9, %1;\n\t"                                                 \
+    "shr.u32 t, bit, 1;\n\t"                                                          \
+    "add.u32 %2, t, %2;\n\t"                                                          \
+    "lop3.b32 na, %0, %1, %2, 0x01;\n\t"                                              \
+    "mul.lo.s32 %1, %1, %9;\n\t"                                                      \
+    "shr.s32 %2, %2, 1;\n\t"                                                          \
+    "lop3.b32 f0, %0, %1, %2, 0x01;\n\t"                                              \
+    "popc.b32 pc, %0;\n\t"                                                            \
+    "setp.ne.and.u32 pg, pc, 30, pb;\n\t"                                             \
+    "setp.eq.and.u32 p2, pc, 30, pb;\n\t"
+
+// the masks of the alive columns, from F0
+#define NQB_STEP6_ALIVE                                                               \
+    "neg.s32 t, f0;\n\t"                                                              \
+    "and.b32 lo, t, f0;\n\t"                                                          \
+    "mul.lo.s32 ma, lo, -4;\n\t"                                                      \
+    "bfind.shiftamt.u32 pos, f0;\n\t"                                                 \
+    "shr.b32 mb, 0x3fffffff, pos;\n\t"
+
+#define NQB_STEP6_LOOK                                                                \
+    "mul.lo.s32 t, %1, %9;\n\t"                                                       \
+    "shr.s32 pos, %2, 1;\n\t"                                                         \
+    "lop3.and.b32 t|pg, %0, t, pos, 0x01, pg;\n\t"
+
 // Node counts (%6): a level's placements are its free columns, dead ones
 // included, so a step adds the size of its child's unfiltered list (the root
 // level's is added when a task is loaded), and rows N-2 and N-1 and dead
 // children need no steps of their own.  No look-ahead: a child whose row two
-// below is full still has placements on the row between.  33 operations on 0.63
-// steps per node where VAR 3 takes 21 on one, and 37 % fewer stack accesses,
-// which bound VAR 3 (shared-memory wavefronts 65 %); this form is bound by issue
-// (83 %).  300,007 prefixes of N=17, k=6: kernel 2.12 -> 1.79 ms.
-#define NQB_STEP4N NQB_STEP4_CHILD NQB_STEP4_NODES NQB_STEP4_TAIL
-#define NQB_STEP4N_X4 NQB_STEP4N NQB_STEP4N NQB_STEP4N NQB_STEP4N
-#define NQB_STEP4_X4 NQB_STEP4 NQB_STEP4 NQB_STEP4 NQB_STEP4
-#define NQB_STEP4_X16 NQB_STEP4_X4 NQB_STEP4_X4 NQB_STEP4_X4 NQB_STEP4_X4
+// below is full still has placements on the row between.  29 operations on 0.63
+// steps per node where VAR 3 takes 21 on one, and fewer stack accesses, which
+// bound VAR 3 (shared-memory wavefronts 65 %).  300,007 prefixes of N=17, k=6:
+// the whole call 3.39 ms with VAR 3, 3.01 with VAR 4's form, 2.78 in place.
+#define NQB_STEP6_NODES                                                               \
+    "popc.b32 t, na;\n\t"                                                             \
+    "@pb mad.lo.s32 %6, t, %8, %6;\n\t"
+
+#define NQB_STEP6_CHILD                                                               \
+    "lop3.and.b32 %3|pd, na, ma, mb, 0xE0, pg;\n\t"                                   \
+    "popc.b32 t, %3;\n\t"
+
+#define NQB_STEP6_POP                                                                 \
+    "@!pd mov.b32 %3, 0;\n\t"                                                         \
+    "setp.ne.and.u32 pq, %4, %7, !pd;\n\t"                                            \
+    "@pq mad.lo.s32 %4, %10, %11, %4;\n\t"                                            \
+    "@pq ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
+
+#define NQB_STEP6_COUNT "@p2 mad.lo.s32 %5, t, %8, %5;\n\t"
+#define NQB_STEP6 \
+    NQB_STEP6_PUSH NQB_STEP6_ALIVE NQB_STEP6_LOOK NQB_STEP6_CHILD NQB_STEP6_COUNT NQB_STEP6_POP
+#define NQB_STEP6N \
+    NQB_STEP6_PUSH NQB_STEP6_ALIVE NQB_STEP6_NODES NQB_STEP6_CHILD NQB_STEP6_COUNT NQB_STEP6_POP
+#define NQB_STEP6_X4 NQB_STEP6 NQB_STEP6 NQB_STEP6 NQB_STEP6
+#define NQB_STEP6_X16 NQB_STEP6_X4 NQB_STEP6_X4 NQB_STEP6_X4 NQB_STEP6_X4
+#define NQB_STEP6N_X4 NQB_STEP6N NQB_STEP6N NQB_STEP6N NQB_STEP6N
 
 // Dihedral step: the VAR 1 step plus the class rules of the lane's task.
 //   pc = popc(child cols) = 32 - N + child row
@@ -476,7 +544,8 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
 // 41 operations where the form above has 40, on fewer steps (0.85 at N=11, CPU
 // model; the launch's instructions fall from 111.9e9 to 98.6e9 at N=19, k=6).
 // Bound by issue (84 %, was 79 %) and the ALU pipe (79 %).  N=19, k=6: kernel
-// 122.7 -> 100.7 ms.  Operands as above, with %16 the tie's extra weight dw.
+// 122.7 -> 100.7 ms (in place, as VAR 6, it is no faster: 110.4 against 109.9 ms per
+// call).  Operands as above, with %16 the tie's extra weight dw.
 #define NQB_STEP5_HEAD                                                                \
     "{\n\t"                                                                           \
     ".reg .pred pt1, pb, pg, p2, pd, pk, pp, pq, ps;\n\t"                             \
@@ -539,27 +608,30 @@ struct StepConsts {
     uint32_t one, two, mone, stride;  // stride: bytes between a lane's consecutive stack slots
 };
 
-// Step variant of the count kernels: 4 = filtered children (default), 3 =
-// pre-shifted left diagonal with LOP3 predicate outputs, 1 = the reference's
-// mask form with IMAD-form moves.  Kernels that count DFS nodes run the same
-// variant in its node-counting form; the dihedral kernels run their own
-// filtered step (NQB_STEP_DIH4) with 4, else variant 1.
+// Step variant of the count kernels: 6 = filtered children in place (default),
+// 4 = filtered children, 3 = pre-shifted left diagonal with LOP3 predicate
+// outputs, 1 = the reference's mask form with IMAD-form moves.  Kernels that
+// count DFS nodes run 6 in its node-counting form (3 and 1 themselves); the
+// dihedral kernels run variant 5 (1 with 1 and 3).
 #ifndef NQB_STEP_VAR
-#define NQB_STEP_VAR 4
+#define NQB_STEP_VAR 6
 #endif
 constexpr int kStepVar = NQB_STEP_VAR;
-static_assert(kStepVar == 1 || kStepVar == 3 || kStepVar == 4, "step variant");
-constexpr int kNodesStepVar = kStepVar;
-constexpr int kDihStepVar = kStepVar == 4 ? 5 : 1;
+static_assert(kStepVar == 1 || kStepVar == 3 || kStepVar == 4 || kStepVar == 6, "step variant");
+constexpr int kNodesStepVar = kStepVar == 4 ? 6 : kStepVar;
+constexpr int kDihStepVar = kStepVar >= 4 ? 5 : 1;
+// Count launches without room for variant 6's extra slot, and the resumable
+// kernels, whose stated stack depth leaves none either.
+constexpr int kTightStepVar = kStepVar == 6 ? 4 : kStepVar;
 // The resumable dihedral kernel keeps the form that steps rows N-2 and N-1: its
 // checkpoints hold levels on those rows.
-constexpr int kDihResumeStepVar = kStepVar == 4 ? 4 : 1;
+constexpr int kDihResumeStepVar = kStepVar >= 4 ? 4 : 1;
 
-// Stack rows a step variant never pushes beyond the reference's N-1-rows: the
-// filtered step enters no level on row N-2 or N-1, so the deepest level it
-// pushes is on row N-4.
+// Stack rows a step variant never pushes beyond the reference's N-1-rows: VAR 4
+// and 5 enter no level on row N-2 or N-1 and push what they leave for a child, so
+// the deepest level they push is on row N-4; VAR 6 pushes on row N-3 too.
 template <int VAR>
-constexpr int kStackRowsSpared = VAR == 4 ? 2 : 0;
+constexpr int kStackRowsSpared = VAR == 4 || VAR == 5 ? 2 : VAR == 6 ? 1 : 0;
 
 // Lane registers (ld, rd) from the reference's (left, right) masks of the row
 // a level enumerates, and back (for the checkpoint file, which stores the
@@ -572,10 +644,10 @@ template <int VAR>
 __device__ __forceinline__ uint32_t ref_ld(uint32_t ld) { return VAR >= 3 ? ld >> 1 : ld; }
 template <int VAR>
 __device__ __forceinline__ uint32_t lane_rd(uint32_t right) {
-    return VAR == 4 ? (uint32_t)((int32_t)right >> 1) : right;
+    return VAR >= 4 ? (uint32_t)((int32_t)right >> 1) : right;
 }
 template <int VAR>
-__device__ __forceinline__ uint32_t ref_rd(uint32_t rd) { return VAR == 4 ? rd << 1 : rd; }
+__device__ __forceinline__ uint32_t ref_rd(uint32_t rd) { return VAR >= 4 ? rd << 1 : rd; }
 
 // The alive part of a level's untried columns (VAR 4): drops every column
 // whose child would leave the next row without a free column.  ld and rd in
@@ -645,33 +717,44 @@ __device__ __forceinline__ void dfs_steps3(uint32_t &cols, uint32_t &ld, uint32_
     }
 }
 
-// UNROLL steps of VAR 4, sixteen per asm block where UNROLL allows (0.5 %
-// faster at N=19 than four), else four.  Operand %6, the node counter, is used
-// by the NODES form only.
-template <bool NODES, int UNROLL>
+// UNROLL steps of VAR 4 (no NODES form), four per asm block.  Operand %6 is
+// unused (it stands where the node counter sits in the other forms).
+template <int UNROLL>
 __device__ __forceinline__ void dfs_steps4(uint32_t &cols, uint32_t &ld, uint32_t &rd, uint32_t &avail, uint32_t &sp,
+                                           uint32_t &cnt, uint32_t bot, const StepConsts &k) {
+    static_assert(UNROLL % 4 == 0, "VAR 4 unrolls in groups of 4");
+#pragma unroll
+    for (int g = 0; g < UNROLL / 4; ++g)
+        asm volatile(NQB_STEP4_HEAD NQB_STEP4_X4 "}\n\t"
+                     : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt)
+                     : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(0x3fffffffu),
+                       "r"(0xfffffffcu), "r"(30u)
+                     : "memory");
+}
+
+// UNROLL steps of VAR 6, sixteen per asm block where UNROLL allows, else four.
+// Operand %6, the node counter, is used by the NODES form only.
+template <bool NODES, int UNROLL>
+__device__ __forceinline__ void dfs_steps6(uint32_t &cols, uint32_t &ld, uint32_t &rd, uint32_t &avail, uint32_t &sp,
                                            uint32_t &cnt, uint32_t &it, uint32_t bot, const StepConsts &k) {
-    static_assert(UNROLL % 4 == 0, "VAR 4 unrolls in groups of 4 or 16");
+    static_assert(UNROLL % 4 == 0, "VAR 6 unrolls in groups of 4 or 16");
     constexpr int kGroup = UNROLL % 16 == 0 && !NODES ? 16 : 4;
 #pragma unroll
     for (int g = 0; g < UNROLL / kGroup; ++g) {
         if constexpr (NODES)
-            asm volatile(NQB_STEP4_HEAD NQB_STEP4N_X4 "}\n\t"
+            asm volatile(NQB_STEP6_HEAD NQB_STEP6N_X4 "}\n\t"
                          : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt), "+r"(it)
-                         : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(0x3fffffffu),
-                           "r"(0xfffffffcu), "r"(30u)
+                         : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride)
                          : "memory");
         else if constexpr (kGroup == 16)
-            asm volatile(NQB_STEP4_HEAD NQB_STEP4_X16 "}\n\t"
+            asm volatile(NQB_STEP6_HEAD NQB_STEP6_X16 "}\n\t"
                          : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt)
-                         : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(0x3fffffffu),
-                           "r"(0xfffffffcu), "r"(30u)
+                         : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride)
                          : "memory");
         else
-            asm volatile(NQB_STEP4_HEAD NQB_STEP4_X4 "}\n\t"
+            asm volatile(NQB_STEP6_HEAD NQB_STEP6_X4 "}\n\t"
                          : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt)
-                         : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(0x3fffffffu),
-                           "r"(0xfffffffcu), "r"(30u)
+                         : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride)
                          : "memory");
     }
 }
@@ -707,14 +790,14 @@ __device__ __forceinline__ void load_class(const DfsParams &p, long long t, DihL
 }
 
 // DFS nodes (placements on rows before N-1) from a lane's counters: VAR 1 and 3
-// count every placement, of which a completion is the one on row N-1; VAR 4
+// count every placement, of which a completion is the one on row N-1; VAR 6
 // counts the nodes themselves.
 template <int VAR>
 __device__ __forceinline__ uint32_t node_count(uint32_t it, uint32_t cnt) {
-    return VAR == 4 ? it : it - cnt;
+    return VAR >= 4 ? it : it - cnt;
 }
 
-// VAR 4 keeps only levels on rows 0..N-3, with their alive columns.  A level
+// VAR 4 and 6 keep only levels on rows 0..N-3, with their alive columns.  A level
 // on row N-1 (one column left) completes once per free column; on row N-2
 // once per alive column.  Returns those completions and leaves avail = 0 for
 // such levels; otherwise filters avail and returns 0.
@@ -757,7 +840,7 @@ __device__ __forceinline__ uint32_t settle_level_dih(int n, uint32_t cols, uint3
 // (1 for an already-complete board) and leaves avail == 0 when the task has
 // no free column.  A column mask with off-board bits can never equal `last`,
 // so such a task counts 0, exactly as the reference recursion does.
-// VAR 4: `placed` receives the columns whose placements the nodes of the task's
+// VAR 4 and 6: `placed` receives the columns whose placements the nodes of the task's
 // own row are (its free columns on rows before N-1).
 template <int VAR, bool SETTLE = true>
 __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, uint32_t &cols, uint32_t &ld,
@@ -782,7 +865,7 @@ __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, u
     ld = lane_ld<VAR>(l);
     rd = lane_rd<VAR>(r);
     avail = ~(cols | l | r);
-    if (VAR == 4 && SETTLE) {
+    if (VAR >= 4 && SETTLE) {
         placed = __popc(c) < n - 1 ? avail : 0u;
         return settle_level(n, cols, ld, rd, avail);
     }
@@ -980,12 +1063,15 @@ __device__ __forceinline__ uint32_t post_mail(const DfsParams &p, uint32_t lane,
 // (it measurably changed the code generated for the DFS loop).
 // DIH runs the dihedral decomposition: every task carries a class (rules and
 // weights, see DfsParams::cls_tab) and the step is dfs_step_dih.
+// The count kernels are held to 32 registers (2 x 1024 threads): left to itself
+// the compiler takes 42 for one of them, and the loop's code is worse (N=19 133.6
+// -> 136.2 ms); the others spill at 32.
 template <bool PER_OWNER, bool NODES, int VAR, int UNROLL, bool RESUME = false, bool DIH = false>
-__global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
+__global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kernel(DfsParams p) {
     static_assert(DIH ? VAR == 1 || VAR == 4 || VAR == 5 : VAR != 5, "dihedral step variants: 1, 4 and 5");
-    // Lane registers of the step: the dihedral VAR 4 keeps VAR 3's form, VAR 5
-    // has VAR 4's.
-    constexpr int LVAR = (DIH && VAR == 4) ? 3 : VAR == 5 ? 4 : VAR;
+    static_assert(!(VAR == 4 && NODES), "node counts run variant 6");
+    // Lane registers of the step: the dihedral VAR 4 keeps VAR 3's form.
+    constexpr int LVAR = (DIH && VAR == 4) ? 3 : VAR;
     constexpr bool MAIL = !RESUME;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned long long red_cnt[32];
@@ -1125,7 +1211,7 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                                 if (avail) owner = own;
                             }
                             tot += done;
-                            if (NODES && VAR == 4) {
+                            if (NODES && VAR >= 4) {
                                 const uint32_t here = __popc(placed & share_mask(lg, way));
                                 if (PER_OWNER && here) atomicAdd(p.out_nodes + own, (unsigned long long)here);
                                 tot_nodes += here;
@@ -1208,8 +1294,10 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                         dfs_steps5<UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
                     else if constexpr (DIH)
                         dfs_step_dih<VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
+                    else if constexpr (VAR == 6)
+                        dfs_steps6<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
                     else if constexpr (VAR == 4)
-                        dfs_steps4<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
+                        dfs_steps4<UNROLL>(cols, ld, rd, avail, sp, cnt, bot, kc);
                     else if constexpr (VAR == 3)
                         dfs_steps3<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
                     else
@@ -1225,8 +1313,10 @@ __global__ void __launch_bounds__(1024) dfs_kernel(DfsParams p) {
                         dfs_steps5<UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
                     else if constexpr (DIH)
                         dfs_step_dih<VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
+                    else if constexpr (VAR == 6)
+                        dfs_steps6<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
                     else if constexpr (VAR == 4)
-                        dfs_steps4<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
+                        dfs_steps4<UNROLL>(cols, ld, rd, avail, sp, cnt, bot, kc);
                     else if constexpr (VAR == 3)
                         dfs_steps3<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
                     else

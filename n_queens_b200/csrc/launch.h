@@ -36,7 +36,7 @@ constexpr int kUnroll = NQB_UNROLL;
 #endif
 constexpr int kNodesUnroll = NQB_NODES_UNROLL;
 constexpr int kDihUnroll = NQB_DIH_UNROLL;
-constexpr int kCountUnroll = kStepVar == 4 ? NQB_COUNT_UNROLL : NQB_UNROLL;
+constexpr int kCountUnroll = kStepVar >= 4 ? NQB_COUNT_UNROLL : NQB_UNROLL;
 static_assert(kUnroll % 4 == 0 && kCountUnroll % 4 == 0, "inner_steps are rounded to multiples of 4");
 
 // DFS steps a warp runs between visits to the queue (the fold of its 32-bit
@@ -50,11 +50,19 @@ constexpr int kDfsStaticSmem = 2 * 32 * 8 + 16;
 constexpr int kMinAutoThreads = 64;
 constexpr int kMaxAutoThreads = 512;
 
+// Slots a count launch gets beyond stack_need(): variant 6 pushes on one more row
+// than the stated depth (nq_stack_levels) covers.  A launch with a stated CTA size
+// that has no room for it runs kTightStepVar, which needs none.
+constexpr int kExtraSlots = kStepVar == 6 ? 1 : 0;
+inline bool extra_slots_fit(int threads, int levels, int smem_optin) {
+    return (long long)(threads / 32) * (levels + kExtraSlots) * kSlotBytes + kDfsStaticSmem <= smem_optin;
+}
+
 // Stack slots per lane that a launch over prefixes with `placed` queens needs:
 // N-1-placed for the kernels that step every row (node counts, the dihedral
 // decomposition), two fewer for the filtered count step.  At least 1.
 inline int stack_need(int N, int placed, bool filtered) {
-    const int need = N - 1 - placed - (filtered && kStepVar == 4 ? kStackRowsSpared<4> : 0);
+    const int need = N - 1 - placed - (filtered && kStepVar >= 4 ? kStackRowsSpared<4> : 0);
     return need < 1 ? 1 : need;
 }
 

@@ -63,8 +63,11 @@ std::mutex g_noalloc_mu;
 NoAllocDev g_noalloc_dev[kNoAllocMaxDevices];
 
 typedef void (*NoAllocKernel)(DfsParams);
-// The same instantiation the allocating device entry runs for a plain count.
-NoAllocKernel noalloc_kernel() { return dfs_kernel<false, false, kStepVar, kCountUnroll>; }
+// The same instantiations the allocating device entry runs for a plain count.
+NoAllocKernel noalloc_kernel(bool tight) {
+    return tight ? dfs_kernel<false, false, kTightStepVar, kCountUnroll>
+                 : dfs_kernel<false, false, kStepVar, kCountUnroll>;
+}
 
 int noalloc_fail(cudaError_t e, const char *what) {
     set_last_error((std::string(what) + ": " + cudaGetErrorString(e)).c_str());
@@ -120,9 +123,11 @@ int noalloc_setup(int dev, NoAllocDev &d) {
     if (e != cudaSuccess) return noalloc_fail(e, "cudaDeviceGetAttribute");
     e = cudaDeviceGetAttribute(&d.smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return noalloc_fail(e, "cudaDeviceGetAttribute");
-    e = cudaFuncSetAttribute(noalloc_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             d.smem_optin - kDfsStaticSmem);
-    if (e != cudaSuccess) return noalloc_fail(e, "cudaFuncSetAttribute");
+    for (const bool tight : {false, true}) {
+        e = cudaFuncSetAttribute(noalloc_kernel(tight), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 d.smem_optin - kDfsStaticSmem);
+        if (e != cudaSuccess) return noalloc_fail(e, "cudaFuncSetAttribute");
+    }
     d.ready = true;
     return NQ_OK;
 }
@@ -175,22 +180,26 @@ extern "C" int nq_count_tasks_device_noalloc(int N, const uint32_t *d_cols, cons
     const int levels = (cfg && cfg->stack_levels > 0) ? cfg->stack_levels : stack_need(N, 0, true);
     int cap_per_sm = std::min(kNoAllocMaxBlocksPerSm, std::max(1, kNoAllocMaxCtas / d.sms));
     if (cfg && cfg->blocks_per_sm > 0) cap_per_sm = std::min(cap_per_sm, cfg->blocks_per_sm);
+    const bool tight =
+        cfg && cfg->block_threads > 0 && !extra_slots_fit(cfg->block_threads, levels, d.smem_optin);
+    const int slots = levels + (tight ? 0 : kExtraSlots);
+    const NoAllocKernel fn = noalloc_kernel(tight);
     const int threads = (cfg && cfg->block_threads)
                             ? cfg->block_threads
-                            : resident_warp_threads(noalloc_kernel(), levels, d.smem_optin, cap_per_sm);
+                            : resident_warp_threads(fn, slots, d.smem_optin, cap_per_sm);
     if (threads == 0) {
         set_last_error("no CTA size of 64 or more threads fits this stack depth in shared memory");
         return NQ_ERR_DEPTH;
     }
     if (threads < 32 || threads > 1024 || (threads & 31)) return NQ_ERR_ARG;
-    const long long smem64 = (long long)(threads / 32) * levels * kSlotBytes;
+    const long long smem64 = (long long)(threads / 32) * slots * kSlotBytes;
     if (smem64 + kDfsStaticSmem > d.smem_optin) {
         set_last_error("per-CTA stack does not fit in shared memory: lower block_threads or stack_levels");
         return NQ_ERR_DEPTH;
     }
     const int smem = (int)smem64;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, noalloc_kernel(), threads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
     if (e != cudaSuccess) return noalloc_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     if (per_sm <= 0) {
         set_last_error("launch configuration cannot be resident");
@@ -213,7 +222,7 @@ extern "C" int nq_count_tasks_device_noalloc(int N, const uint32_t *d_cols, cons
         p.nqueue = (long long)cfg->queue_len;
     }
     p.N = N;
-    p.levels = levels;
+    p.levels = slots;
     if (cfg && cfg->inner_steps > NQ_MAX_INNER_STEPS) {
         set_last_error("inner_steps is above NQ_MAX_INNER_STEPS");
         return NQ_ERR_ARG;
@@ -241,7 +250,7 @@ extern "C" int nq_count_tasks_device_noalloc(int N, const uint32_t *d_cols, cons
     // ticket, error and timeout words): clear all of them.
     e = cudaMemsetAsync(d.scratch, 0, kCtlWords * sizeof(unsigned long long), s);
     if (e != cudaSuccess) return noalloc_fail(e, "cudaMemsetAsync");
-    noalloc_kernel()<<<grid, threads, smem, s>>>(p);
+    fn<<<grid, threads, smem, s>>>(p);
     e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(e, "dfs_kernel launch");
     return NQ_OK;

@@ -67,3 +67,16 @@ def test_time_limit_still_stops(gpu):
         gpu.count(19, 3, config=dict(time_limit_ms=3))
     assert e.value.status == gpu.NQ_ERR_TIMEOUT
     assert gpu.count(15, 2).total == 2279184
+
+
+# 1024 threads and 14 slots fill the SM's shared memory, so the in-place step's
+# extra slot does not fit; 13 leave room for it; 32 is the deepest stack.
+@pytest.mark.parametrize("threads,levels", [(1024, 14), (1024, 13), (448, 32), (416, 32), (32, 8)])
+def test_stack_shapes_with_and_without_the_extra_slot(gpu, threads, levels):
+    N, k = 13, 2
+    c, l, r = oracle.expand(N, k)
+    want = oracle.count_tasks(N, c, l, r)
+    cfg = dict(block_threads=threads, stack_levels=levels)
+    assert np.array_equal(gpu.count_tasks(N, c, l, r, per_task=True, config=cfg)["per_task"], want)
+    res = gpu.count(N, k, config=cfg)
+    assert res.total == 2 * int(want.sum()) and res.stats["stack_levels"] == levels
