@@ -924,8 +924,16 @@ constexpr unsigned long long kMailPatienceNs = 20ull * 1000 * 1000;
 constexpr int kMailPolls = 1 << 16;   // second limit on a wait, in polls
 constexpr int kMailRootRows = 13;      // rows left in the deepest task from which a launch uses the mailbox
 constexpr uint32_t kMailMinRows = 12;  // rows left below which a level is not worth posting
-constexpr uint32_t kGiveMinRows = 6;   // the same for a level given to a lane of the same warp
-constexpr int kShortTrip = 48;         // DFS steps of a warp with idle lanes before it looks again
+constexpr uint32_t kGiveMinRows = 8;   // the same for a level given to a lane of the same warp
+// Once the queue is empty a warp looks at its idle lanes after kTailTrip DFS
+// steps, or as soon as kTailIdle lanes are idle: a look (donation, mailbox) costs
+// about 290 instructions, ten steps, and with one at every newly idle lane they
+// were a quarter of all instructions of a batch.  512 boards of N=12..17
+// 9.65 ms with a look per idle lane, 8.9 at 8 lanes and 64 steps, 8.1 at 12 and
+// 96; 60,001 prefixes of N=16 538, 491, 489 us (496 at 16 lanes).  The loop of a
+// live queue keeps its plain any-vote: counting the lanes there costs 6 % (N=19).
+constexpr int kTailTrip = 96;
+constexpr int kTailIdle = 12;
 
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *a) {
     uint32_t v;
@@ -1285,6 +1293,8 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
             }
         }
 
+        if (!RESUME) check_idle &= queue_live;
+
         // ---- DFS steps
         if (check_idle) {
             for (int s = 0; s < p.inner; s += UNROLL) {
@@ -1306,7 +1316,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                 if (__any_sync(kFull, avail == 0)) break;
             }
         } else {
-            for (int s = 0; s < kShortTrip; s += UNROLL) {
+            for (int s = 0; s < kTailTrip; s += UNROLL) {
 #pragma unroll
                 for (int u = 0; u < ((VAR >= 3 && !DIH) || VAR == 5 ? 1 : UNROLL); ++u) {
                     if constexpr (VAR == 5)
@@ -1322,7 +1332,8 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                     else
                         dfs_step<NODES, VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
                 }
-                if (__all_sync(kFull, avail == 0)) break;
+                const unsigned idle_now = __ballot_sync(kFull, avail == 0);
+                if (RESUME ? idle_now == kFull : (p.steal && __popc(idle_now) >= kTailIdle)) break;
             }
         }
     }
