@@ -80,10 +80,13 @@ typedef struct nq_config {
     int blocks_per_sm;      /* resident CTAs per SM for the persistent grid */
     int stack_levels;       /* per-lane DFS stack slots (>= nq_stack_levels(N, rows, nodes), at most
                                NQ_MAX_STACK_LEVELS) */
-    int steal;              /* 0 = default (on), 1 = on, -1 = off: in-warp work donation */
+    int steal;              /* 0 = default (on), 1 = on, -1 = off: work sharing (tasks dealt out in shares,
+                               donation inside a warp, levels handed between warps) */
     int inner_steps;        /* DFS steps between warp refill checks: 1..NQ_MAX_INNER_STEPS (larger values
                                are NQ_ERR_ARG), rounded up to a multiple of the kernel's steps per warp
-                               vote (16 for counts, 8 for node counts and the dihedral kernels) */
+                               vote (16 for counts, 8 for the dihedral kernels); 0 = 1024, or 256 where
+                               there are fewer than four tasks per lane.  Once the queue is empty a
+                               warp looks at its idle lanes at least every 96 steps */
     int order_kind;         /* NQ_ORDER_PLAIN or NQ_ORDER_GIVEN */
     const uint32_t *order;  /* NQ_ORDER_GIVEN: queue position -> task index (host or device
                                pointer, matching the entry's other task arrays) */
@@ -114,9 +117,9 @@ typedef struct nq_stats {
     int smem_bytes;     /* dynamic shared memory per CTA */
     int reserved[5];
     /* With nq_config.timing: kernel span from the first CTA start to the last
-     * CTA end, the mean CTA busy time, and the idle fraction of the grid
-     * (1 - sum of CTA busy times / (CTAs x span)) -- the tail left by uneven
-     * tasks. */
+     * CTA end, the mean CTA busy time (its span less the time its warps waited
+     * for work), and the idle fraction of the grid (1 - sum of CTA busy times /
+     * (CTAs x span)) -- the tail left by uneven tasks. */
     double makespan_ms;
     double cta_busy_mean_ms;
     double tail_idle_frac;
@@ -205,7 +208,7 @@ int nq_count_tasks(int N, const uint32_t *cols, const uint32_t *ld, const uint32
  * d_nodes needs d_per_task).  d_sum is a device array of 2 uint64: [0]
  * receives the plain sum of the counts, [1] status bits (1: a task needed
  * more stack levels than the launch had and was skipped; 2: the time limit
- * stopped the kernel).  Without a host view of the tasks the stack covers
+ * stopped the kernel; 8: internal error, the sum is not to be used).  Without a host view of the tasks the stack covers
  * the deepest possible task (nq_stack_levels(N, 0, d_nodes != NULL) levels)
  * unless cfg->stack_levels says otherwise.  Returns after enqueueing;
  * the caller synchronises the stream.  Uses the library's device scratch for the
@@ -241,7 +244,8 @@ int nq_count_tasks_device_noalloc(int N, const uint32_t *d_cols, const uint32_t 
  * counted once; a mirror-symmetric board counts its left-half children twice
  * (the reference's half-board rule, src/n_queens.cpp:74-113, applied to any
  * symmetric board).  Every distinct board is split split_rows rows deeper
- * (0 = 3).  nq_count_batch = nq_batch_create + nq_batch_run + destroy. */
+ * (0 = 3).  The same counts as nq_batch_create + nq_batch_run + destroy, without
+ * building a plan (the subtasks go through the device's kept buffers). */
 int nq_count_batch(const nq_instance *inst, int64_t n, int split_rows, uint64_t *out, const nq_config *cfg,
                    nq_stats *stats);
 
@@ -296,13 +300,13 @@ int nq_mlp_destroy(nq_mlp *m);
 /* FP32 master weights in the flat layout; set also resets Adam's moments. */
 int nq_mlp_get_params(nq_mlp *m, float *out);
 int nq_mlp_set_params(nq_mlp *m, const float *in);
-/* Predicted log2(1 + nodes) of n tasks of board size N (host arrays). */
+/* Predicted log2(1 + nodes) of n tasks of board size N (host arrays), on the
+ * tensor cores with the layer-1 outputs in FP32 (three BF16 parts). */
 int nq_mlp_predict(nq_mlp *m, int N, const uint32_t *cols, const uint32_t *ld, const uint32_t *rd, int64_t n,
                    float *out);
-/* The same forward on the tensor cores (tcgen05.mma, BF16 operands, FP32
- * accumulators in TMEM), as nq_schedule_device runs it: the layer-1 outputs
- * are rounded to BF16 before layer 2, so results differ from nq_mlp_predict
- * by that rounding. */
+/* The same forward as nq_schedule_device runs it: the layer-1 outputs are
+ * rounded to BF16 before layer 2, so results differ from nq_mlp_predict by
+ * that rounding. */
 int nq_mlp_predict_tensor(nq_mlp *m, int N, const uint32_t *cols, const uint32_t *ld, const uint32_t *rd, int64_t n,
                           float *out);
 /* Gradient of the mean squared error over n tasks (per-task board sizes in
