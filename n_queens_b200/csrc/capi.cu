@@ -483,11 +483,11 @@ int count_resident(Ctx &c, int N, const uint32_t *d_cols, const uint32_t *d_ld, 
     NQ_CUDA(cudaEventRecord(c.ev[2], c.stream));
     const bool want_cnt = per_owner && h_per_task, want_nodes = per_owner && nodes && h_nodes_task;
     const bool staged = ((size_t)want_cnt + want_nodes) * (size_t)n * 8 <= kStageBytes;
-    rc = c.h_out.grow(64 + (staged ? 2 * (size_t)n * 8 : 0));
+    rc = c.h_out.grow(64 + (staged ? ((size_t)want_cnt + want_nodes) * (size_t)n * 8 : 0));
     if (rc) return rc;
     unsigned long long *res = (unsigned long long *)c.h_out.p;
     uint64_t *to_cnt = staged ? (uint64_t *)res + 8 : h_per_task;
-    uint64_t *to_nodes = staged ? (uint64_t *)res + 8 + n : h_nodes_task;
+    uint64_t *to_nodes = staged ? (uint64_t *)res + 8 + (want_cnt ? n : 0) : h_nodes_task;
     NQ_CUDA(cudaMemcpyAsync(res, c.d_ctl + kWordSum, 3 * sizeof(*res), cudaMemcpyDeviceToHost, c.stream));
     if (want_cnt) NQ_CUDA(cudaMemcpyAsync(to_cnt, p.out_cnt, (size_t)n * 8, cudaMemcpyDeviceToHost, c.stream));
     if (want_nodes) NQ_CUDA(cudaMemcpyAsync(to_nodes, p.out_nodes, (size_t)n * 8, cudaMemcpyDeviceToHost, c.stream));
@@ -653,6 +653,7 @@ int write_checkpoint(const char *path, const Checkpoint &ck) {
 }
 
 constexpr int kDefaultSplit = 3;
+constexpr size_t kDirectBatchBytes = 16u << 20;  // about a million subtasks
 
 // Reverses the low N bits (column j -> N-1-j).
 uint32_t rev_bits(uint32_t x, int N) {
@@ -852,9 +853,9 @@ void destroy_batch(nq_batch &b) {
     b.h_res = nullptr;
 }
 
-int build_batch(Ctx &c, const nq_instance *inst, int64_t n, int split, const nq_config *cfg, nq_batch &B) {
+// Builds the plan of the subtasks in B.t.
+int build_batch(Ctx &c, const nq_config *cfg, nq_batch &B) {
     B.device = device_of(cfg);
-    batch_tasks(inst, n, split, B.t);
     const int64_t m = (int64_t)B.t.tc.size();
     B.m_tasks = m;
     int rc = plan_launch(c, cfg, B.t.levels, true, false, B.L);
@@ -1516,7 +1517,8 @@ int nq_batch_create(const nq_instance *inst, int64_t n, int split_rows, const nq
     rc = ensure_ready(c, device_of(cfg));
     if (rc) return rc;
     nq_batch *b = new nq_batch();
-    rc = build_batch(c, inst, n, split_rows ? split_rows : kDefaultSplit, cfg, *b);
+    batch_tasks(inst, n, split_rows ? split_rows : kDefaultSplit, b->t);
+    rc = build_batch(c, cfg, *b);
     if (rc) {
         destroy_batch(*b);
         delete b;
@@ -1730,7 +1732,9 @@ int nq_count_batch(const nq_instance *inst, int64_t n, int split_rows, uint64_t 
     if (n == 0) return (n < 0 || split_rows < 0 || split_rows > 8) ? NQ_ERR_ARG : NQ_OK;
     // One pass needs no plan of its own: the subtasks go through the device's
     // buffers and the launch is issued directly (an allocation, a graph capture
-    // and their release cost 2-4 ms, against some 20 us for a small board).
+    // and their release cost 2-4 ms, against some 20 us for a small board).  A
+    // list above kDirectBatchBytes, whose run is long against that, still gets a
+    // plan, so that its memory is given back.
     const double t0 = now_ms();
     int rc = check_instances(inst, n, split_rows);
     if (rc) return rc;
@@ -1742,8 +1746,20 @@ int nq_count_batch(const nq_instance *inst, int64_t n, int split_rows, uint64_t 
     std::lock_guard<std::mutex> lock(c.mu);
     rc = ensure_ready(c, device_of(cfg));
     if (rc) return rc;
-    BatchTasks t;
+    nq_batch plan;
+    BatchTasks &t = plan.t;
     batch_tasks(inst, n, split_rows ? split_rows : kDefaultSplit, t);
+    if (t.task_bytes() > kDirectBatchBytes) {
+        rc = build_batch(c, cfg, plan);
+        if (!rc) rc = run_batch(c, plan, stats);
+        if (!rc) {
+            t.gather(plan.h_res + 3, out);
+            if (stats) stats->total_ms = now_ms() - t0;
+            rc = status_from_bits(plan.h_res[2]);
+        }
+        destroy_batch(plan);
+        return rc;
+    }
     Launch L;
     rc = plan_launch(c, cfg, t.levels, true, false, L);
     if (rc) return rc;
