@@ -67,7 +67,7 @@ double now_ms() {
 
 typedef void (*KernelFn)(DfsParams);
 
-// tight: a count launch without room for kExtraSlots.
+// tight: a count launch without room for extra_slots().
 KernelFn pick_kernel(bool per_owner, bool nodes, bool dih = false, bool tight = false) {
     if (dih) return per_owner ? dfs_kernel<true, false, kDihStepVar, kDihUnroll, false, true>
                               : dfs_kernel<false, false, kDihStepVar, kDihUnroll, false, true>;
@@ -77,7 +77,7 @@ KernelFn pick_kernel(bool per_owner, bool nodes, bool dih = false, bool tight = 
     if (tight)
         return per_owner ? dfs_kernel<true, false, kTightStepVar, kCountUnroll>
                          : dfs_kernel<false, false, kTightStepVar, kCountUnroll>;
-    return per_owner ? dfs_kernel<true, false, kStepVar, kCountUnroll>
+    return per_owner ? dfs_kernel<true, false, kOwnerStepVar, kCountUnroll>
                      : dfs_kernel<false, false, kStepVar, kCountUnroll>;
 }
 
@@ -233,9 +233,10 @@ int plan_launch(Ctx &c, const nq_config *cfg, int levels_needed, bool per_owner,
     const int cap_per_sm = (cfg && cfg->blocks_per_sm > 0) ? std::min(cfg->blocks_per_sm, kMaxBlocksPerSm)
                                                            : kMaxBlocksPerSm;
     const bool counts = !nodes && !dih;
+    const int extra = counts ? extra_slots(per_owner) : 0;
     L.tight = counts && (resumable || (cfg && cfg->block_threads > 0 &&
-                                       !extra_slots_fit(cfg->block_threads, L.levels, c.smem_optin)));
-    L.slots = L.levels + (counts && !L.tight ? kExtraSlots : 0);
+                                       !slots_fit(cfg->block_threads, L.levels + extra, c.smem_optin)));
+    L.slots = L.levels + (L.tight ? 0 : extra);
     const KernelFn fn = pick_kernel(per_owner, nodes, dih, L.tight);
     const bool plain = !(cfg && (cfg->block_threads || cfg->blocks_per_sm > 0)) && !resumable &&
                        L.levels <= NQ_MAX_STACK_LEVELS;

@@ -390,8 +390,10 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "shr.s32 %2, %2, 1;\n\t"                                                          \
     "lop3.b32 f0, %0, %1, %2, 0x01;\n\t"                                              \
     "popc.b32 pc, %0;\n\t"                                                            \
-    "setp.ne.and.u32 pg, pc, 30, pb;\n\t"                                             \
     "setp.eq.and.u32 p2, pc, 30, pb;\n\t"
+
+// a child on row N-2 is counted and not entered
+#define NQB_STEP6_GATE "setp.ne.and.u32 pg, pc, 30, pb;\n\t"
 
 // the masks of the alive columns, from F0
 #define NQB_STEP6_ALIVE                                                               \
@@ -405,6 +407,19 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "mul.lo.s32 t, %1, %9;\n\t"                                                       \
     "shr.s32 pos, %2, 1;\n\t"                                                         \
     "lop3.and.b32 t|pg, %0, t, pos, 0x01, pg;\n\t"
+
+// VAR 7, the count kernels with per-owner outputs: VAR 6 without the gate.  A
+// counted child on row N-2 is entered too when its row two below (there is none)
+// looks free; its level finds no alive column and ends.  One ALU operation fewer
+// on every step for about 1 % more steps, and a second extra slot (for the push on
+// row N-2).  1.1e6 prefixes of N=18 with per-task counts 17.24 -> 16.69 ms, 1.8e6 of N=19
+// 128.2 -> 125.6 ms; in the kernel without per-owner outputs the same step issues
+// 80.9 instead of 84.4 % of the slots and is slower (126.8 -> 129.8 ms), so that
+// one keeps the gate.
+#define NQB_STEP7_LOOK                                                                \
+    "mul.lo.s32 t, %1, %9;\n\t"                                                       \
+    "shr.s32 pos, %2, 1;\n\t"                                                         \
+    "lop3.and.b32 t|pg, %0, t, pos, 0x01, pb;\n\t"
 
 // Node counts (%6): a level's placements are its free columns, dead ones
 // included, so a step adds the size of its child's unfiltered list (the root
@@ -430,11 +445,15 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
 
 #define NQB_STEP6_COUNT "@p2 mad.lo.s32 %5, t, %8, %5;\n\t"
 #define NQB_STEP6 \
-    NQB_STEP6_PUSH NQB_STEP6_ALIVE NQB_STEP6_LOOK NQB_STEP6_CHILD NQB_STEP6_COUNT NQB_STEP6_POP
+    NQB_STEP6_PUSH NQB_STEP6_GATE NQB_STEP6_ALIVE NQB_STEP6_LOOK NQB_STEP6_CHILD NQB_STEP6_COUNT NQB_STEP6_POP
 #define NQB_STEP6N \
-    NQB_STEP6_PUSH NQB_STEP6_ALIVE NQB_STEP6_NODES NQB_STEP6_CHILD NQB_STEP6_COUNT NQB_STEP6_POP
+    NQB_STEP6_PUSH NQB_STEP6_GATE NQB_STEP6_ALIVE NQB_STEP6_NODES NQB_STEP6_CHILD NQB_STEP6_COUNT NQB_STEP6_POP
+#define NQB_STEP7 \
+    NQB_STEP6_PUSH NQB_STEP6_ALIVE NQB_STEP7_LOOK NQB_STEP6_CHILD NQB_STEP6_COUNT NQB_STEP6_POP
 #define NQB_STEP6_X4 NQB_STEP6 NQB_STEP6 NQB_STEP6 NQB_STEP6
 #define NQB_STEP6_X16 NQB_STEP6_X4 NQB_STEP6_X4 NQB_STEP6_X4 NQB_STEP6_X4
+#define NQB_STEP7_X4 NQB_STEP7 NQB_STEP7 NQB_STEP7 NQB_STEP7
+#define NQB_STEP7_X16 NQB_STEP7_X4 NQB_STEP7_X4 NQB_STEP7_X4 NQB_STEP7_X4
 #define NQB_STEP6N_X4 NQB_STEP6N NQB_STEP6N NQB_STEP6N NQB_STEP6N
 
 // Dihedral step: the VAR 1 step plus the class rules of the lane's task.
@@ -608,7 +627,8 @@ struct StepConsts {
     uint32_t one, two, mone, stride;  // stride: bytes between a lane's consecutive stack slots
 };
 
-// Step variant of the count kernels: 6 = filtered children in place (default),
+// Step variant of the count kernels: 6 = filtered children in place (default; 7,
+// its form for per-owner outputs),
 // 4 = filtered children, 3 = pre-shifted left diagonal with LOP3 predicate
 // outputs, 1 = the reference's mask form with IMAD-form moves.  Kernels that
 // count DFS nodes run 6 in its node-counting form (3 and 1 themselves); the
@@ -618,9 +638,11 @@ struct StepConsts {
 #endif
 constexpr int kStepVar = NQB_STEP_VAR;
 static_assert(kStepVar == 1 || kStepVar == 3 || kStepVar == 4 || kStepVar == 6, "step variant");
+// ... with per-owner outputs
+constexpr int kOwnerStepVar = kStepVar == 6 ? 7 : kStepVar;
 constexpr int kNodesStepVar = kStepVar == 4 ? 6 : kStepVar;
 constexpr int kDihStepVar = kStepVar >= 4 ? 5 : 1;
-// Count launches without room for variant 6's extra slot, and the resumable
+// Count launches without room for the extra slots of 6 and 7, and the resumable
 // kernels, whose stated stack depth leaves none either.
 constexpr int kTightStepVar = kStepVar == 6 ? 4 : kStepVar;
 // The resumable dihedral kernel keeps the form that steps rows N-2 and N-1: its
@@ -629,7 +651,8 @@ constexpr int kDihResumeStepVar = kStepVar >= 4 ? 4 : 1;
 
 // Stack rows a step variant never pushes beyond the reference's N-1-rows: VAR 4
 // and 5 enter no level on row N-2 or N-1 and push what they leave for a child, so
-// the deepest level they push is on row N-4; VAR 6 pushes on row N-3 too.
+// the deepest level they push is on row N-4; VAR 6 pushes on row N-3 too, VAR 7 on
+// row N-2.
 template <int VAR>
 constexpr int kStackRowsSpared = VAR == 4 || VAR == 5 ? 2 : VAR == 6 ? 1 : 0;
 
@@ -732,12 +755,17 @@ __device__ __forceinline__ void dfs_steps4(uint32_t &cols, uint32_t &ld, uint32_
                      : "memory");
 }
 
-// UNROLL steps of VAR 6, sixteen per asm block where UNROLL allows, else four.
-// Operand %6, the node counter, is used by the NODES form only.
-template <bool NODES, int UNROLL>
+// UNROLL steps of VAR 6 or 7, sixteen per asm block where UNROLL allows, else
+// four.  Operand %6, the node counter, is used by the NODES form (VAR 6) only.
+#define NQB_RUN_STEPS(TEXT)                                                                                     \
+    asm volatile(NQB_STEP6_HEAD TEXT "}\n\t"                                                                    \
+                 : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt)                             \
+                 : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride)                        \
+                 : "memory")
+template <int VAR, bool NODES, int UNROLL>
 __device__ __forceinline__ void dfs_steps6(uint32_t &cols, uint32_t &ld, uint32_t &rd, uint32_t &avail, uint32_t &sp,
                                            uint32_t &cnt, uint32_t &it, uint32_t bot, const StepConsts &k) {
-    static_assert(UNROLL % 4 == 0, "VAR 6 unrolls in groups of 4 or 16");
+    static_assert(UNROLL % 4 == 0, "VAR 6 and 7 unroll in groups of 4 or 16");
     constexpr int kGroup = UNROLL % 16 == 0 && !NODES ? 16 : 4;
 #pragma unroll
     for (int g = 0; g < UNROLL / kGroup; ++g) {
@@ -746,18 +774,17 @@ __device__ __forceinline__ void dfs_steps6(uint32_t &cols, uint32_t &ld, uint32_
                          : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt), "+r"(it)
                          : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride)
                          : "memory");
+        else if constexpr (VAR == 7 && kGroup == 16)
+            NQB_RUN_STEPS(NQB_STEP7_X16);
+        else if constexpr (VAR == 7)
+            NQB_RUN_STEPS(NQB_STEP7_X4);
         else if constexpr (kGroup == 16)
-            asm volatile(NQB_STEP6_HEAD NQB_STEP6_X16 "}\n\t"
-                         : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt)
-                         : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride)
-                         : "memory");
+            NQB_RUN_STEPS(NQB_STEP6_X16);
         else
-            asm volatile(NQB_STEP6_HEAD NQB_STEP6_X4 "}\n\t"
-                         : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt)
-                         : "r"(0u), "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride)
-                         : "memory");
+            NQB_RUN_STEPS(NQB_STEP6_X4);
     }
 }
+#undef NQB_RUN_STEPS
 
 // UNROLL steps of VAR 5, four per asm block.
 template <int UNROLL>
@@ -1077,7 +1104,7 @@ __device__ __forceinline__ uint32_t post_mail(const DfsParams &p, uint32_t lane,
 template <bool PER_OWNER, bool NODES, int VAR, int UNROLL, bool RESUME = false, bool DIH = false>
 __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kernel(DfsParams p) {
     static_assert(DIH ? VAR == 1 || VAR == 4 || VAR == 5 : VAR != 5, "dihedral step variants: 1, 4 and 5");
-    static_assert(!(VAR == 4 && NODES), "node counts run variant 6");
+    static_assert(!(NODES && (VAR == 4 || VAR == 7)), "node counts run variant 6");
     // Lane registers of the step: the dihedral VAR 4 keeps VAR 3's form.
     constexpr int LVAR = (DIH && VAR == 4) ? 3 : VAR;
     constexpr bool MAIL = !RESUME;
@@ -1304,8 +1331,8 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                         dfs_steps5<UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
                     else if constexpr (DIH)
                         dfs_step_dih<VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
-                    else if constexpr (VAR == 6)
-                        dfs_steps6<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
+                    else if constexpr (VAR == 6 || VAR == 7)
+                        dfs_steps6<VAR, NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
                     else if constexpr (VAR == 4)
                         dfs_steps4<UNROLL>(cols, ld, rd, avail, sp, cnt, bot, kc);
                     else if constexpr (VAR == 3)
@@ -1323,8 +1350,8 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                         dfs_steps5<UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
                     else if constexpr (DIH)
                         dfs_step_dih<VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
-                    else if constexpr (VAR == 6)
-                        dfs_steps6<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
+                    else if constexpr (VAR == 6 || VAR == 7)
+                        dfs_steps6<VAR, NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
                     else if constexpr (VAR == 4)
                         dfs_steps4<UNROLL>(cols, ld, rd, avail, sp, cnt, bot, kc);
                     else if constexpr (VAR == 3)

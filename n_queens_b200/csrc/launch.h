@@ -51,11 +51,12 @@ constexpr int kMinAutoThreads = 64;
 constexpr int kMaxAutoThreads = 512;
 
 // Slots a count launch gets beyond stack_need(): variant 6 pushes on one more row
-// than the stated depth (nq_stack_levels) covers.  A launch with a stated CTA size
-// that has no room for it runs kTightStepVar, which needs none.
-constexpr int kExtraSlots = kStepVar == 6 ? 1 : 0;
-inline bool extra_slots_fit(int threads, int levels, int smem_optin) {
-    return (long long)(threads / 32) * (levels + kExtraSlots) * kSlotBytes + kDfsStaticSmem <= smem_optin;
+// than the stated depth (nq_stack_levels) covers, variant 7 (per-owner outputs) on
+// two.  A launch with a stated CTA size that has no room for them runs
+// kTightStepVar, which needs none.
+inline int extra_slots(bool per_owner) { return kStepVar != 6 ? 0 : per_owner ? 2 : 1; }
+inline bool slots_fit(int threads, int slots, int smem_optin) {
+    return (long long)(threads / 32) * slots * kSlotBytes + kDfsStaticSmem <= smem_optin;
 }
 
 // Stack slots per lane that a launch over prefixes with `placed` queens needs:

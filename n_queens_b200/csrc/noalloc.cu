@@ -181,8 +181,8 @@ extern "C" int nq_count_tasks_device_noalloc(int N, const uint32_t *d_cols, cons
     int cap_per_sm = std::min(kNoAllocMaxBlocksPerSm, std::max(1, kNoAllocMaxCtas / d.sms));
     if (cfg && cfg->blocks_per_sm > 0) cap_per_sm = std::min(cap_per_sm, cfg->blocks_per_sm);
     const bool tight =
-        cfg && cfg->block_threads > 0 && !extra_slots_fit(cfg->block_threads, levels, d.smem_optin);
-    const int slots = levels + (tight ? 0 : kExtraSlots);
+        cfg && cfg->block_threads > 0 && !slots_fit(cfg->block_threads, levels + extra_slots(false), d.smem_optin);
+    const int slots = levels + (tight ? 0 : extra_slots(false));
     const NoAllocKernel fn = noalloc_kernel(tight);
     const int threads = (cfg && cfg->block_threads)
                             ? cfg->block_threads

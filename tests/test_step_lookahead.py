@@ -8,6 +8,8 @@ the smallest the step enters and on arbitrary 32-bit masks:
 * ``NQB_STEP6``: the same in place -- the parent's remaining columns are pushed
   before the child is computed over it, and a child that is not entered is
   undone by a pop -- with one stack slot more;
+* ``NQB_STEP7``: the same without the gate on row N-2 -- a counted child may be
+  entered, finds no alive column and ends -- with a second extra slot;
 * ``NQB_STEP6N``: its node-count form (the size of each child's unfiltered list
   instead of the look-ahead, plus the root level's)."""
 import numpy as np
@@ -65,6 +67,7 @@ class LookAheadLanes(Lanes):
 
 class InPlaceLanes(LookAheadLanes):
     spared = 1  # one slot more than need_slots
+    gate = True
 
     def step(self):
         cols, ld, rd, avail = self.cols, self.ld, self.rd, self.avail
@@ -77,7 +80,7 @@ class InPlaceLanes(LookAheadLanes):
         ld, rd = ld * TWO, sar1(rd)
         f0 = ~(cols | ld | rd)
         pc = popc(cols)
-        pg, p2 = (pc != 30) & pb, (pc == 30) & pb
+        pg, p2 = ((pc != 30) | (not self.gate)) & pb, (pc == 30) & pb
         if self.count_nodes:
             self.nodes += np.where(pb, popc(na), 0).astype(np.uint64)
         else:
@@ -92,8 +95,13 @@ class InPlaceLanes(LookAheadLanes):
         self.cols, self.ld, self.rd, self.avail = cols, ld, rd, avail
 
 
+class UngatedLanes(InPlaceLanes):
+    spared = 2
+    gate = False
+
+
 @pytest.mark.parametrize("N,k", [(4, 1), (5, 1), (6, 2), (7, 2), (8, 3), (10, 4), (11, 6)])
-@pytest.mark.parametrize("model", [LookAheadLanes, InPlaceLanes])
+@pytest.mark.parametrize("model", [LookAheadLanes, InPlaceLanes, UngatedLanes])
 def test_whole_board_prefixes(N, k, model):
     c, l, r = oracle.expand(N, k)
     lanes = model(N, c, l, r)
@@ -102,7 +110,7 @@ def test_whole_board_prefixes(N, k, model):
 
 
 @pytest.mark.parametrize("N", [6, 9, 11])
-@pytest.mark.parametrize("model", [LookAheadLanes, InPlaceLanes])
+@pytest.mark.parametrize("model", [LookAheadLanes, InPlaceLanes, UngatedLanes])
 def test_arbitrary_32bit_tasks(N, model):
     rng = np.random.default_rng(N)
     rand = lambda: rng.integers(0, 1 << 32, 2500, dtype=np.uint64).astype(np.uint32)
