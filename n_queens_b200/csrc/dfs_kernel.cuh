@@ -560,11 +560,12 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
 //  * Weights: each completion weighs w, and the one whose row N-1 queen stands
 //    at the tie column weighs w + dw; there is one when the tie column is unused
 //    and a column other than it is alive.
-// 41 operations where the form above has 40, on fewer steps (0.85 at N=11, CPU
-// model; the launch's instructions fall from 111.9e9 to 98.6e9 at N=19, k=6).
-// Bound by issue (84 %, was 79 %) and the ALU pipe (79 %).  N=19, k=6: kernel
-// 122.7 -> 100.7 ms (in place, as VAR 6, it is no faster: 110.4 against 109.9 ms per
-// call).  Operands as above, with %16 the tie's extra weight dw.
+// A counted child on row N-2 may be entered too (see VAR 7); its level finds no
+// alive column and ends.  40 operations, as the form above, on fewer steps (0.85 at N=11, CPU
+// model).  Bound by issue (84 %, was 79 %) and the ALU pipe.  N=19, k=6, a whole
+// call: 132.1 ms with the form above, 108.7 with the compare that keeps row N-2
+// out, 106.2 without it (in place, as VAR 6, it is no faster).  Operands as above,
+// with %16 the tie's extra weight dw.
 #define NQB_STEP5_HEAD                                                                \
     "{\n\t"                                                                           \
     ".reg .pred pt1, pb, pg, p2, pd, pk, pp, pq, ps;\n\t"                             \
@@ -584,7 +585,6 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "lop3.b32 f0, nc, xl, xr, 0x01;\n\t"                                              \
     "popc.b32 pc, nc;\n\t"                                                            \
     "setp.eq.and.u32 p2, pc, 30, pb;\n\t"                                             \
-    "setp.ne.and.u32 pg, pc, 30, pb;\n\t"                                             \
     "setp.gt.u32 ps, pc, %12;\n\t"                                                    \
     "lop3.and.b32 t|ps, nc, %17, 0, 0x03, ps;\n\t"                                    \
     "@ps mul.lo.s32 na, na, 0;\n\t"                                                   \
@@ -596,7 +596,7 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
     "shr.b32 mb, 0x3fffffff, pos;\n\t"                                                \
     "mul.lo.s32 t, xl, %9;\n\t"                                                       \
     "shr.s32 pos, xr, 1;\n\t"                                                         \
-    "lop3.and.b32 t|pg, nc, t, pos, 0x01, pg;\n\t"                                    \
+    "lop3.and.b32 t|pg, nc, t, pos, 0x01, pb;\n\t"                                    \
     "lop3.and.b32 naf|pd, na, ma, mb, 0xE0, pg;\n\t"                                  \
     "popc.b32 t, naf;\n\t"                                                            \
     "@p2 mad.lo.s32 %5, t, %15, %5;\n\t"                                              \
@@ -650,11 +650,11 @@ constexpr int kTightStepVar = kStepVar == 6 ? 4 : kStepVar;
 constexpr int kDihResumeStepVar = kStepVar >= 4 ? 4 : 1;
 
 // Stack rows a step variant never pushes beyond the reference's N-1-rows: VAR 4
-// and 5 enter no level on row N-2 or N-1 and push what they leave for a child, so
-// the deepest level they push is on row N-4; VAR 6 pushes on row N-3 too, VAR 7 on
+// enters no level on row N-2 or N-1 and pushes what it leaves for a child, so the
+// deepest level it pushes is on row N-4; VAR 5 and 6 push on row N-3 too, VAR 7 on
 // row N-2.
 template <int VAR>
-constexpr int kStackRowsSpared = VAR == 4 || VAR == 5 ? 2 : VAR == 6 ? 1 : 0;
+constexpr int kStackRowsSpared = VAR == 4 ? 2 : VAR == 5 || VAR == 6 ? 1 : 0;
 
 // Lane registers (ld, rd) from the reference's (left, right) masks of the row
 // a level enumerates, and back (for the checkpoint file, which stores the

@@ -42,7 +42,7 @@ class CountingDihLanes(DihLanes):
         ma = ((U(0) - f0) & f0) * U(0xFFFFFFFC)
         mb = shr_clamp(U(0x3FFFFFFF), shiftamt(f0))
         naf = na & (ma | mb)
-        pd = (naf != 0) & (pc != 30) & pb & (~(nc | xl * U(2) | sar1(xr)) != 0)
+        pd = (naf != 0) & pb & (~(nc | xl * U(2) | sar1(xr)) != 0)  # row N-2 is not kept out
         tie = p2 & ((self.tie_bit & ~nc) != 0) & ((naf & ~self.tie_bit) != 0)
         add = np.where(p2, popc(naf) * self.w, U(0)) + np.where(tie, self.w_tie - self.w, U(0))
         self.cnt += add.astype(np.uint64)
