@@ -306,9 +306,13 @@ int nq_mlp_predict(nq_mlp *m, int N, const uint32_t *cols, const uint32_t *ld, c
                    float *out);
 /* The same forward as nq_schedule_device runs it: the layer-1 outputs are
  * rounded to BF16 before layer 2, so results differ from nq_mlp_predict by
- * that rounding. */
+ * that rounding.  Both return NQ_ERR_TIMEOUT when a wait for the tensor cores
+ * expires (nq_mlp_set_wait_limit). */
 int nq_mlp_predict_tensor(nq_mlp *m, int N, const uint32_t *cols, const uint32_t *ld, const uint32_t *rd, int64_t n,
                           float *out);
+/* Polls after which a wait for the tensor cores counts as expired: at most, and
+ * by default, 2^22 (seconds).  For tests of what follows an expired wait. */
+int nq_mlp_set_wait_limit(nq_mlp *m, uint64_t polls);
 /* Gradient of the mean squared error over n tasks (per-task board sizes in
  * task_n, targets in log2(1 + nodes)) with respect to the BF16 compute
  * weights, in the flat layout, and the loss.  Changes nothing. */
@@ -325,7 +329,9 @@ int nq_mlp_train(nq_mlp *m, const uint8_t *task_n, const uint32_t *cols, const u
  * and stable inside a bin; d_pred (optional, n floats) the predictions.
  * Stream-ordered on `stream` (a cudaStream_t; NULL = legacy default stream).
  * The model's prediction scratch is in use until that work completes: call no
- * other entry of the same model before it has. */
+ * other entry of the same model before it has.  Should a wait for the tensor
+ * cores expire, the tasks without a prediction go last, in index order: d_order
+ * is a permutation in any case. */
 int nq_schedule_device(nq_mlp *m, int N, const uint32_t *d_cols, const uint32_t *d_ld, const uint32_t *d_rd,
                        int64_t n, uint32_t *d_order, float *d_pred, void *stream);
 /* nq_schedule_device with the n_last tasks listed in d_last (device u32 task
@@ -337,7 +343,9 @@ int nq_schedule_device_last(nq_mlp *m, int N, const uint32_t *d_cols, const uint
                             void *stream);
 /* nq_count with the queue ordered by the model: expand, upload, schedule on
  * the device, count.  The same total as nq_count; stats->schedule_ms holds the
- * prediction + sort time.  The model must live on cfg->device. */
+ * prediction + sort time.  The model must live on cfg->device.  NQ_ERR_TIMEOUT
+ * with the right *total: a wait for the tensor cores expired, so the queue was
+ * not ordered by the model throughout. */
 int nq_count_learned(int N, int rows, nq_mlp *m, const nq_config *cfg, uint64_t *total, nq_stats *stats);
 /* nq_count_learned for a board part of whose tasks was already counted --
  * typically the cost model's fine-tuning and hold-out samples, which the

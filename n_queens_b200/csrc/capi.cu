@@ -1291,6 +1291,11 @@ int nq_count_dihedral_resumable(int N, int rows, const nq_config *cfg, const cha
 }  // extern "C"
 
 namespace nqb {
+
+// The scheduler's expired MMA waits (defined in mlp.cu).
+void clear_schedule_error(nq_mlp *m);
+bool schedule_error(nq_mlp *m);
+
 namespace {
 
 // nq_count_learned and nq_count_learned_reuse: expand, upload, order the
@@ -1359,6 +1364,7 @@ int count_learned_impl(int N, int rows, nq_mlp *m, const int64_t *done_idx, int6
     NQ_CUDA(cudaEventCreate(&e_sched0));
     NQ_CUDA(cudaEventCreate(&e_sched1));
     NQ_CUDA(cudaEventRecord(e_sched0, c.stream));
+    clear_schedule_error(m);
     rc = nq_schedule_device_last(m, N, d, d + n, d + 2 * n, n, d_done, n_done, d_order, nullptr, c.stream);
     if (rc) {
         cudaEventDestroy(e_sched0);
@@ -1382,7 +1388,8 @@ int count_learned_impl(int N, int rows, nq_mlp *m, const int64_t *done_idx, int6
     // The reference doubles every per-prefix sum for the mirror image
     // (src/n_queens_cuda.cu:181-183).
     *total = 2 * (sum + done_sum);
-    return rc;
+    // an order cut short by an expired wait is still a permutation: the count holds
+    return rc ? rc : schedule_error(m) ? NQ_ERR_TIMEOUT : NQ_OK;
 }
 
 }  // namespace

@@ -107,8 +107,10 @@ __device__ __forceinline__ void load_masks(const TaskView &tv, long long t, uint
 // 16-byte core matrices, LBO = 128 B between the two core matrices of one
 // K=16 step, SBO = K/8 * 128 B between 8-row groups.  One thread of a group
 // issues its MMAs; completion is signalled through the group's mbarrier
-// (tcgen05.commit) and every wait on it is bounded (on expiry the kernel sets
-// *err and stops).
+// (tcgen05.commit) and every wait on it is bounded: on expiry the group sets
+// *err, gives its remaining tasks the lowest key and their own index (so that a
+// sorted order stays a permutation), waits once more, again bounded, for the
+// MMAs in flight and stops.
 //
 // What bounds it: the latency of a tile's chain (X build, MMA, epilogue, MMA,
 // epilogue), then issue in the epilogues (52 % at 1.9e6 tasks, tensor pipe 38 %).
@@ -134,7 +136,7 @@ constexpr uint32_t kTmemCols = 512;
 // Instruction descriptor, kind::f16: D F32, A and B BF16, both K-major,
 // N = 128 (N>>3 at bit 17), M = 128 (M>>4 at bit 24).
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-constexpr unsigned long long kWaitLimit = 1ull << 22;  // a few seconds at most
+constexpr unsigned long long kWaitLimit = 1ull << 22;  // polls: a few seconds at most
 
 static_assert(off_kmajor(127, 95, kSbo1) < kOffB2 - kOffB1, "W1 tile bounds");
 static_assert(off_kmajor(127, 127, kSbo2) < kOffA - kOffB2, "W2 tile bounds");
@@ -157,9 +159,9 @@ __device__ __forceinline__ void commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// Bounded wait for the mbarrier phase with the given parity; false on expiry.
-__device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity) {
-    for (unsigned long long i = 0; i < kWaitLimit; ++i) {
+// Bounded wait (`limit` polls) for the mbarrier phase with the given parity; false on expiry.
+__device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, unsigned long long limit) {
+    for (unsigned long long i = 0; i < limit; ++i) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
@@ -208,10 +210,12 @@ __device__ __forceinline__ uint16_t order_key(float pred) {
 }
 
 // out (optional): predictions.  key and idx (both or neither): sort keys and the
-// identity permutation for the scheduler.
+// identity permutation for the scheduler.  err: a host word, written only when a
+// wait of `limit` polls expires.
 template <int PARTS>
 __global__ void __launch_bounds__(PARTS == 1 ? 512 : 256, 1)
-    mlp_forward_kernel(TaskView tv, long long n, const Weights *w, float *out, uint16_t *key, uint32_t *idx, int *err) {
+    mlp_forward_kernel(TaskView tv, long long n, const Weights *w, float *out, uint16_t *key, uint32_t *idx,
+                       volatile int *err, unsigned long long limit) {
     constexpr uint32_t kGroups = PARTS == 1 ? 4 : 2;
     constexpr uint32_t kBufs = 4 / kGroups;  // operand buffers of a group
     extern __shared__ __align__(1024) unsigned char tc_smem[];
@@ -265,7 +269,7 @@ __global__ void __launch_bounds__(PARTS == 1 ? 512 : 256, 1)
 
     // Waits for the group's MMAs; false when the wait expired for some thread.
     auto mma_done = [&]() -> bool {
-        if (!tc::wait_phase(bar, phase)) *fail = 1;
+        if (!tc::wait_phase(bar, phase, limit)) *fail = 1;
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         group_sync(g);
@@ -382,7 +386,21 @@ __global__ void __launch_bounds__(PARTS == 1 ? 512 : 256, 1)
         group_sync(g);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
-    if (*fail && t == 0) atomicExch(err, 1);
+    if (*fail) {
+        tc::wait_phase(bar, phase ^ 1u, tc::kWaitLimit);  // MMAs still in flight read this CTA's shared memory
+        if (key)
+            for (; tile < tiles; tile += step) {
+                const long long task = tile * 128 + t;
+                if (task < n) {
+                    key[task] = 1;
+                    idx[task] = (uint32_t)task;
+                }
+            }
+        if (t == 0) {
+            *err = 1;
+            __threadfence_system();
+        }
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -735,7 +753,7 @@ struct nq_mlp {
     int device = 0;
     int sms = 0;
     cudaStream_t stream = nullptr;
-    void *block = nullptr;  // holds the next five and tc_err
+    void *block = nullptr;  // holds the next five
     float *master = nullptr, *adam1 = nullptr, *adam2 = nullptr;
     Weights *w = nullptr;
     long long steps = 0;
@@ -743,7 +761,11 @@ struct nq_mlp {
     float *grad_part = nullptr;
     int grad_parts_cap = 0;
     float *gsum = nullptr;  // summed gradient (nq_mlp_grad)
-    int *tc_err = nullptr;  // set by the tensor-core kernel when an MMA wait expires
+    // Set by the forward kernel when an MMA wait expires: [0] nq_mlp_predict*, [1] the
+    // scheduler.  In host memory, so that reading them costs a call neither a memset
+    // nor a copy.
+    volatile int *err = nullptr;
+    unsigned long long wait_limit = tc::kWaitLimit;
     void *loss_part = nullptr;  // floats
     size_t loss_cap = 0;
     void *data = nullptr;
@@ -856,11 +878,20 @@ int launch_forward(nq_mlp *m, int parts, const TaskView &tv, long long n, float 
                    cudaStream_t s) {
     const int grid = (int)std::min<long long>((n + 127) / 128, m->sms);
     if (parts == 1)
-        mlp_forward_kernel<1><<<grid, 512, tc::kSmemBytes, s>>>(tv, n, m->w, d_out, key, idx, m->tc_err);
+        mlp_forward_kernel<1>
+            <<<grid, 512, tc::kSmemBytes, s>>>(tv, n, m->w, d_out, key, idx, m->err + (key ? 1 : 0), m->wait_limit);
     else
-        mlp_forward_kernel<3><<<grid, 256, tc::kSmemBytes, s>>>(tv, n, m->w, d_out, key, idx, m->tc_err);
+        mlp_forward_kernel<3><<<grid, 256, tc::kSmemBytes, s>>>(tv, n, m->w, d_out, key, idx, m->err, m->wait_limit);
     MLP_CUDA(cudaGetLastError());
     return NQ_OK;
+}
+
+// Whether an MMA wait expired since the last look (the kernels have finished).
+bool take_wait_error(volatile int *err) {
+    if (!*err) return false;
+    *err = 0;
+    set_last_error("tensor-core MMA completion wait expired");
+    return true;
 }
 
 // Predictions of n host tasks into a host array.
@@ -870,18 +901,11 @@ int predict_host(nq_mlp *m, int parts, int N, const uint32_t *cols, const uint32
     int rc = stage(m, nullptr, cols, ld, rd, nullptr, n, st);
     if (rc) return rc;
     TaskView tv{st.cols, st.ld, st.rd, nullptr, nullptr, N};
-    MLP_CUDA(cudaMemsetAsync(m->tc_err, 0, sizeof(int), m->stream));
     rc = launch_forward(m, parts, tv, n, st.target, nullptr, nullptr, m->stream);
     if (rc) return rc;
-    int err = 0;
     MLP_CUDA(cudaMemcpyAsync(out, st.target, (size_t)n * 4, cudaMemcpyDeviceToHost, m->stream));
-    MLP_CUDA(cudaMemcpyAsync(&err, m->tc_err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
     MLP_CUDA(cudaStreamSynchronize(m->stream));
-    if (err) {
-        set_last_error("tensor-core MMA completion wait expired");
-        return NQ_ERR_TIMEOUT;
-    }
-    return NQ_OK;
+    return take_wait_error(m->err) ? NQ_ERR_TIMEOUT : NQ_OK;
 }
 
 int check_model(nq_mlp *m) {
@@ -891,6 +915,13 @@ int check_model(nq_mlp *m) {
 }
 
 }  // namespace
+
+// For nq_count_learned (capi.cu): forgets the scheduler's expired waits, and
+// tells whether one has expired since (its stream synchronised).
+namespace nqb {
+void clear_schedule_error(nq_mlp *m) { m->err[1] = 0; }
+bool schedule_error(nq_mlp *m) { return take_wait_error(m->err + 1); }
+}  // namespace nqb
 
 extern "C" {
 
@@ -914,15 +945,15 @@ int nq_mlp_create(int device, uint64_t seed, nq_mlp **out) try {
     // one allocation for everything whose size is known here
     auto room = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
     const size_t vec = room(kParams * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&m->block, 4 * vec + room(sizeof(Weights)) + room(sizeof(int)));
+    if (e == cudaSuccess) e = cudaMalloc(&m->block, 4 * vec + room(sizeof(Weights)));
+    if (e == cudaSuccess) e = cudaHostAlloc((void **)&m->err, 2 * sizeof(int), cudaHostAllocDefault);
     char *at = (char *)m->block;
     for (float **v : {&m->master, &m->adam1, &m->adam2, &m->gsum}) {
         *v = (float *)at;
         at += vec;
     }
     m->w = (Weights *)at;
-    m->tc_err = (int *)(at + room(sizeof(Weights)));
-    if (e == cudaSuccess) e = cudaMemset(m->tc_err, 0, sizeof(int));
+    if (e == cudaSuccess) m->err[0] = m->err[1] = 0;
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(mlp_forward_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes);
     if (e == cudaSuccess)
@@ -962,6 +993,7 @@ int nq_mlp_destroy(nq_mlp *m) try {
     cudaFree(m->loss_part);
     cudaFree(m->data);
     cudaFree(m->sort_tmp);
+    cudaFreeHost((void *)m->err);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
     return NQ_OK;
@@ -993,6 +1025,15 @@ int nq_mlp_set_params(nq_mlp *m, const float *in) try {
     MLP_CUDA(cudaGetLastError());
     MLP_CUDA(cudaStreamSynchronize(m->stream));
     m->steps = 0;
+    return NQ_OK;
+} catch (...) {
+    return status_of_exception();
+}
+
+int nq_mlp_set_wait_limit(nq_mlp *m, uint64_t polls) try {
+    if (!m) return NQ_ERR_ARG;
+    std::lock_guard<std::mutex> lock(m->mu);
+    m->wait_limit = std::min<uint64_t>(polls, tc::kWaitLimit);
     return NQ_OK;
 } catch (...) {
     return status_of_exception();

@@ -45,6 +45,8 @@ def _declare():
     L.nq_mlp_get_params.argtypes = [_mlpp, _f32p]
     L.nq_mlp_set_params.restype = ctypes.c_int
     L.nq_mlp_set_params.argtypes = [_mlpp, _f32p]
+    L.nq_mlp_set_wait_limit.restype = ctypes.c_int
+    L.nq_mlp_set_wait_limit.argtypes = [_mlpp, ctypes.c_uint64]
     L.nq_mlp_predict.restype = ctypes.c_int
     L.nq_mlp_predict.argtypes = [_mlpp, ctypes.c_int, _u32p, _u32p, _u32p, ctypes.c_int64, _f32p]
     L.nq_mlp_predict_tensor.restype = ctypes.c_int

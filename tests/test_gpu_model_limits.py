@@ -1,0 +1,64 @@
+"""The cost model at its limits, on the GPU: waits for the tensor cores that expire."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle
+from oracle import mlp_ref
+
+pytestmark = pytest.mark.gpu
+POLLS = 1 << 22  # the default limit
+
+
+def _params(seed):
+    p = np.random.default_rng(seed).uniform(-0.12, 0.12, mlp_ref.NPARAMS).astype(np.float32)
+    p[mlp_ref.OFF_B3] = 12.0
+    return p
+
+
+def _schedule(learned, m, N, tasks, last=None):
+    import torch
+    t = [torch.from_numpy(np.ascontiguousarray(a).view(np.int32)).cuda() for a in tasks]
+    order = torch.full((t[0].numel(),), -1, dtype=torch.int32, device="cuda")
+    d_last = None if last is None else torch.tensor(last, dtype=torch.int32, device="cuda")
+    rc = learned.lib.nq_schedule_device_last(m._m, N, *(a.data_ptr() for a in t), order.numel(),
+                                             d_last.data_ptr() if last else None, len(last or ()), order.data_ptr(),
+                                             None, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    torch.cuda.synchronize()
+    return order.cpu().numpy()
+
+
+# one task; a ragged tile; more tiles than the 148 x 4 groups, so that a group leaves several unfinished
+@pytest.mark.parametrize("n", [1, 300, 75_777, 200_001])
+def test_expired_wait_leaves_a_permutation_and_is_reported(gpu, n):
+    from n_queens_b200 import learned
+    N = 17
+    tasks = [a[:n] for a in oracle.expand(N, 6)]
+    m = learned.CostModel(seed=3)
+    m.set_params(_params(3))
+    pred, order = m.predict(N, *tasks), _schedule(learned, m, N, tasks)
+    learned.lib.nq_mlp_set_wait_limit(m._m, 0)
+    assert np.array_equal(_schedule(learned, m, N, tasks), np.arange(n))
+    last = [0, n // 2] if n > 2 else []
+    want = np.concatenate([np.setdiff1d(np.arange(n), last), np.array(last, np.int64)])
+    assert np.array_equal(_schedule(learned, m, N, tasks, last), want)
+    for f in (m.predict, m.predict_tensor):
+        with pytest.raises(gpu.NQError) as e:
+            f(N, *tasks)
+        assert e.value.status == gpu.NQ_ERR_TIMEOUT
+    learned.lib.nq_mlp_set_wait_limit(m._m, POLLS)
+    assert np.array_equal(m.predict(N, *tasks), pred) and np.array_equal(_schedule(learned, m, N, tasks), order)
+    m.close()
+
+
+def test_learned_count_reports_an_expired_wait_with_the_right_total(gpu):
+    from n_queens_b200 import learned
+    m = learned.CostModel(seed=3)
+    for polls, status in ((0, gpu.NQ_ERR_TIMEOUT), (POLLS, gpu.NQ_OK), (0, gpu.NQ_ERR_TIMEOUT)):
+        learned.lib.nq_mlp_set_wait_limit(m._m, polls)
+        total = ctypes.c_uint64(0)
+        assert learned.lib.nq_count_learned(14, 4, m._m, None, ctypes.byref(total), None) == status
+        assert total.value == 365596
+    m.close()
