@@ -301,7 +301,8 @@ int nq_mlp_destroy(nq_mlp *m);
 int nq_mlp_get_params(nq_mlp *m, float *out);
 int nq_mlp_set_params(nq_mlp *m, const float *in);
 /* Predicted log2(1 + nodes) of n tasks of board size N (host arrays), on the
- * tensor cores with the layer-1 outputs in FP32 (three BF16 parts). */
+ * tensor cores with the layer-1 outputs in FP32 (three BF16 parts); with weights
+ * of 2^32 or more, infinite or NaN, in FP32 on the CUDA cores. */
 int nq_mlp_predict(nq_mlp *m, int N, const uint32_t *cols, const uint32_t *ld, const uint32_t *rd, int64_t n,
                    float *out);
 /* The same forward as nq_schedule_device runs it: the layer-1 outputs are

@@ -12,6 +12,7 @@
 // FP32 master copies for Adam; biases are FP32; every sum accumulates in
 // FP32.  Kernels (all hand-written):
 //   mlp_forward_kernel  forward for many tasks on the tensor cores
+//   mlp_predict_kernel  the same in FP32 on the CUDA cores, for weights of any size
 //   mlp_train_kernel    forward + backward of a minibatch slice; per-CTA
 //                       partial gradients (no atomics: deterministic)
 //   mlp_adam_kernel     sums the partials in CTA order, Adam step, refreshes
@@ -92,6 +93,95 @@ __device__ __forceinline__ void load_masks(const TaskView &tv, long long t, uint
     m2 = tv.rd[i] & last;
 }
 
+// Layer 1 for one task and hidden unit j: b1[j] + sum of W1 columns of the
+// set input bits.  Every thread of the CTA walks the same bits (uniform).
+__device__ __forceinline__ float layer1(const __nv_bfloat16 *w1t, float b, uint32_t m0, uint32_t m1, uint32_t m2,
+                                        int j) {
+    float acc = b;
+    while (m0) {
+        const int f = __ffs(m0) - 1;
+        m0 &= m0 - 1;
+        acc += __bfloat162float(w1t[f * kH1 + j]);
+    }
+    while (m1) {
+        const int f = __ffs(m1) - 1 + 32;
+        m1 &= m1 - 1;
+        acc += __bfloat162float(w1t[f * kH1 + j]);
+    }
+    while (m2) {
+        const int f = __ffs(m2) - 1 + 64;
+        m2 &= m2 - 1;
+        acc += __bfloat162float(w1t[f * kH1 + j]);
+    }
+    return acc;
+}
+
+// Layer 2 pre-activation of unit j for one task: w2row holds W2[j][:] as
+// 64 packed BF16 pairs, h1 the task's 128 layer-1 outputs (broadcast reads).
+__device__ __forceinline__ float layer2(const uint32_t (&w2row)[kH1 / 2], float b, const float *h1) {
+    float acc = b;
+#pragma unroll
+    for (int i = 0; i < kH1; i += 4) {
+        const float4 h = *reinterpret_cast<const float4 *>(h1 + i);
+        const __nv_bfloat162 wa = *reinterpret_cast<const __nv_bfloat162 *>(&w2row[i / 2]);
+        const __nv_bfloat162 wb = *reinterpret_cast<const __nv_bfloat162 *>(&w2row[i / 2 + 1]);
+        acc = fmaf(__low2float(wa), h.x, acc);
+        acc = fmaf(__high2float(wa), h.y, acc);
+        acc = fmaf(__low2float(wb), h.z, acc);
+        acc = fmaf(__high2float(wb), h.w, acc);
+    }
+    return acc;
+}
+
+__device__ __forceinline__ void load_w2row(const Weights *w, int j, uint32_t (&w2row)[kH1 / 2]) {
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(w->w2 + j * kH1);
+#pragma unroll
+    for (int i = 0; i < kH1 / 2; ++i) w2row[i] = src[i];
+}
+
+// The general forward of nq_mlp_predict, in FP32 on the CUDA cores: out[t] =
+// predicted log2(1 + nodes).  128 threads, thread j = hidden unit j.  Runs where
+// the split form's products of zeros and of BF16 parts would differ from FP32's
+// (see kWideWeight); elsewhere the split form is faster (200,000 tasks 889 us
+// against 55).
+__global__ void __launch_bounds__(128) mlp_predict_kernel(TaskView tv, long long n, const Weights *w, float *out) {
+    __shared__ __align__(16) __nv_bfloat16 s_w1t[kIn * kH1];
+    __shared__ __align__(16) float s_h[kGroup * kH1];
+    __shared__ uint32_t s_m[3][kGroup];
+    const int j = threadIdx.x;
+    for (int i = j; i < kIn * kH1 / 8; i += blockDim.x)
+        reinterpret_cast<uint4 *>(s_w1t)[i] = reinterpret_cast<const uint4 *>(w->w1t)[i];
+    uint32_t w2row[kH1 / 2];
+    load_w2row(w, j, w2row);
+    const float b1 = w->b1[j], b2 = w->b2[j], w3 = __bfloat162float(w->w3[j]), b3 = w->b3;
+    const int warp = j >> 5, lane = j & 31;
+    __syncthreads();
+    for (long long g0 = (long long)blockIdx.x * kGroup; g0 < n; g0 += (long long)gridDim.x * kGroup) {
+        const int gn = (int)min((long long)kGroup, n - g0);
+        if (j < gn) load_masks(tv, g0 + j, s_m[0][j], s_m[1][j], s_m[2][j]);
+        __syncthreads();
+        for (int s = 0; s < gn; ++s)
+            s_h[s * kH1 + j] = fmaxf(layer1(s_w1t, b1, s_m[0][s], s_m[1][s], s_m[2][s], j), 0.f);
+        __syncthreads();
+        float v[kGroup];
+#pragma unroll
+        for (int s = 0; s < kGroup; ++s) v[s] = (s < gn) ? fmaxf(layer2(w2row, b2, s_h + s * kH1), 0.f) * w3 : 0.f;
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < kGroup; ++s) s_h[s * kH1 + j] = v[s];
+        __syncthreads();
+        // layer 3: warp w reduces tasks 8w..8w+7, each lane summing 4 units
+        for (int s = warp * 8; s < warp * 8 + 8; ++s) {
+            const float4 q = *reinterpret_cast<const float4 *>(s_h + s * kH1 + lane * 4);
+            float a = (q.x + q.y) + (q.z + q.w);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (lane == 0 && s < gn) out[g0 + s] = a + b3;
+        }
+        __syncthreads();
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Forward pass on the tensor cores (tcgen05).  A CTA runs GROUPS groups of 128
 // threads, each on its own tiles of 128 tasks (thread t of a group = task row t
@@ -142,6 +232,18 @@ static_assert(off_kmajor(127, 95, kSbo1) < kOffB2 - kOffB1, "W1 tile bounds");
 static_assert(off_kmajor(127, 127, kSbo2) < kOffA - kOffB2, "W2 tile bounds");
 static_assert(off_kmajor(127, 127, kSbo2) < kABytes, "A tile bounds");
 static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
+
+// PARTS 3 runs when every weight and bias of the three layers (b3 is added last)
+// is below 2^32 in magnitude: then layer 1 stays below 2^39 and layer 2 below
+// 2^79, so no part of the split overflows, and no zero input or zero part meets an
+// infinity or a NaN (0 * inf), which FP32 over the set bits alone would not have.
+// Trained weights are far below; others go to mlp_predict_kernel.
+constexpr float kWideWeight = 4294967296.f;
+constexpr uint32_t kWideBf16 = 0x4F80u;  // the same in BF16
+__device__ __forceinline__ bool wide(uint32_t two_bf16) {
+    return (two_bf16 & 0x7fffu) >= kWideBf16 || (two_bf16 >> 16 & 0x7fffu) >= kWideBf16;
+}
+__device__ __forceinline__ bool wide(const uint4 &v) { return wide(v.x) || wide(v.y) || wide(v.z) || wide(v.w); }
 
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
@@ -210,8 +312,10 @@ __device__ __forceinline__ uint16_t order_key(float pred) {
 }
 
 // out (optional): predictions.  key and idx (both or neither): sort keys and the
-// identity permutation for the scheduler.  err: a host word, written only when a
-// wait of `limit` polls expires.
+// identity permutation for the scheduler.  err: a host word, left alone unless a wait
+// of `limit` polls expires (kErrWait) or the weights are out of PARTS 3's range
+// (kErrWide: nothing was computed).
+enum : int { kErrWait = 1, kErrWide = 2 };
 template <int PARTS>
 __global__ void __launch_bounds__(PARTS == 1 ? 512 : 256, 1)
     mlp_forward_kernel(TaskView tv, long long n, const Weights *w, float *out, uint16_t *key, uint32_t *idx,
@@ -231,13 +335,30 @@ __global__ void __launch_bounds__(PARTS == 1 ? 512 : 256, 1)
         const uint4 *src1 = reinterpret_cast<const uint4 *>(w->w1c), *src2 = reinterpret_cast<const uint4 *>(w->w2c);
         uint4 *dst1 = reinterpret_cast<uint4 *>(tc_smem + tc::kOffB1);
         uint4 *dst2 = reinterpret_cast<uint4 *>(tc_smem + tc::kOffB2);
-        for (uint32_t i = tid; i < kIn * kH1 / 8; i += blockDim.x) dst1[i] = src1[i];
-        for (uint32_t i = tid; i < kH2 * kH1 / 8; i += blockDim.x) dst2[i] = src2[i];
+        bool wide = false;
+        auto copy = [&](uint4 *dst, const uint4 *src, uint32_t count) {
+            for (uint32_t i = tid; i < count; i += blockDim.x) {
+                const uint4 v = src[i];
+                dst[i] = v;
+                if (PARTS == 3) wide |= tc::wide(v);
+            }
+        };
+        copy(dst1, src1, kIn * kH1 / 8);
+        copy(dst2, src2, kH2 * kH1 / 8);
         float *b = reinterpret_cast<float *>(tc_smem + tc::kOffBias);
         if (tid < 128) {
             b[tid] = w->b1[tid];
             b[128 + tid] = w->b2[tid];
             b[256 + tid] = __bfloat162float(w->w3[tid]);
+            if (PARTS == 3)
+                for (int k = 0; k < 3; ++k) wide |= !(fabsf(b[128 * k + tid]) < tc::kWideWeight);
+        }
+        if (PARTS == 3 && __syncthreads_or(wide)) {
+            if (tid == 0) {
+                *err = kErrWide;
+                __threadfence_system();
+            }
+            return;
         }
         if (tid < 16) {
             uint32_t *lut = reinterpret_cast<uint32_t *>(tc_smem + tc::kOffLut) + 2 * tid;
@@ -397,7 +518,7 @@ __global__ void __launch_bounds__(PARTS == 1 ? 512 : 256, 1)
                 }
             }
         if (t == 0) {
-            *err = 1;
+            *err = kErrWait;
             __threadfence_system();
         }
     }
@@ -761,8 +882,8 @@ struct nq_mlp {
     float *grad_part = nullptr;
     int grad_parts_cap = 0;
     float *gsum = nullptr;  // summed gradient (nq_mlp_grad)
-    // Set by the forward kernel when an MMA wait expires: [0] nq_mlp_predict*, [1] the
-    // scheduler.  In host memory, so that reading them costs a call neither a memset
+    // kErr* words of the forward kernels: [0] nq_mlp_predict*, [1] the scheduler.  In
+    // host memory, so that reading them costs a call neither a memset
     // nor a copy.
     volatile int *err = nullptr;
     unsigned long long wait_limit = tc::kWaitLimit;
@@ -886,12 +1007,12 @@ int launch_forward(nq_mlp *m, int parts, const TaskView &tv, long long n, float 
     return NQ_OK;
 }
 
-// Whether an MMA wait expired since the last look (the kernels have finished).
-bool take_wait_error(volatile int *err) {
-    if (!*err) return false;
+// What the forward kernels reported since the last look (they have finished).
+int take_error(volatile int *err) {
+    const int e = *err;
     *err = 0;
-    set_last_error("tensor-core MMA completion wait expired");
-    return true;
+    if (e == kErrWait) set_last_error("tensor-core MMA completion wait expired");
+    return e;
 }
 
 // Predictions of n host tasks into a host array.
@@ -905,7 +1026,15 @@ int predict_host(nq_mlp *m, int parts, int N, const uint32_t *cols, const uint32
     if (rc) return rc;
     MLP_CUDA(cudaMemcpyAsync(out, st.target, (size_t)n * 4, cudaMemcpyDeviceToHost, m->stream));
     MLP_CUDA(cudaStreamSynchronize(m->stream));
-    return take_wait_error(m->err) ? NQ_ERR_TIMEOUT : NQ_OK;
+    const int e = take_error(m->err);
+    if (e == kErrWide) {
+        const int grid = (int)std::min<long long>((n + kGroup - 1) / kGroup, (long long)m->sms * 8);
+        mlp_predict_kernel<<<grid, kH1, 0, m->stream>>>(tv, n, m->w, st.target);
+        MLP_CUDA(cudaGetLastError());
+        MLP_CUDA(cudaMemcpyAsync(out, st.target, (size_t)n * 4, cudaMemcpyDeviceToHost, m->stream));
+        MLP_CUDA(cudaStreamSynchronize(m->stream));
+    }
+    return e == kErrWait ? NQ_ERR_TIMEOUT : NQ_OK;
 }
 
 int check_model(nq_mlp *m) {
@@ -920,7 +1049,7 @@ int check_model(nq_mlp *m) {
 // tells whether one has expired since (its stream synchronised).
 namespace nqb {
 void clear_schedule_error(nq_mlp *m) { m->err[1] = 0; }
-bool schedule_error(nq_mlp *m) { return take_wait_error(m->err + 1); }
+bool schedule_error(nq_mlp *m) { return take_error(m->err + 1) == kErrWait; }
 }  // namespace nqb
 
 extern "C" {

@@ -1,4 +1,4 @@
-"""The cost model at its limits, on the GPU: waits for the tensor cores that expire."""
+"""The cost model at its limits, on the GPU: waits for the tensor cores that expire, infinite and huge weights."""
 import ctypes
 
 import numpy as np
@@ -61,4 +61,36 @@ def test_learned_count_reports_an_expired_wait_with_the_right_total(gpu):
         total = ctypes.c_uint64(0)
         assert learned.lib.nq_count_learned(14, 4, m._m, None, ctypes.byref(total), None) == status
         assert total.value == 365596
+    m.close()
+
+
+def _forward_over_set_bits(p, X):
+    """Float64 forward that adds only the W1 columns of the set bits, ReLU of NaN = 0 (CUDA's fmaxf)."""
+    W1, b1, W2, b2, W3, b3 = mlp_ref.unpack(p)
+    with np.errstate(all="ignore"):
+        h1 = np.stack([np.fmax(b1 + W1[:, x > 0].sum(1), 0) for x in X])
+        h2 = np.fmax((h1[:, None, :] * W2[None]).sum(2) + b2, 0)
+        return (h2 * W3).sum(1) + b3
+
+
+# Column 20 is off the N=14 board (no input bit), column 3 is on it.  2^32 is where
+# the general forward takes over.  FP32 sums of 96 and 128 terms: 1e-5 of the largest output.
+@pytest.mark.parametrize("where,value", [
+    (5 * 96 + 20, np.inf), (5 * 96 + 20, np.nan), (5 * 96 + 20, 3e38), (5 * 96 + 3, np.inf), (5 * 96 + 3, -np.inf),
+    (5 * 96 + 3, np.nan), (5 * 96 + 3, 1e37), (5 * 96 + 3, 2.0**32), (5 * 96 + 3, 2.0**31), (mlp_ref.OFF_B1 + 5, 3.395e38),
+    (mlp_ref.OFF_B1 + 5, np.inf), (mlp_ref.OFF_W2 + 7, np.inf), (mlp_ref.OFF_W2 + 7, -np.inf), (mlp_ref.OFF_W2 + 7, 1e30),
+    (mlp_ref.OFF_B2 + 7, np.nan), (mlp_ref.OFF_B2 + 7, 1e33), (mlp_ref.OFF_W3 + 7, np.inf), (mlp_ref.OFF_B3, np.inf)])
+@pytest.mark.parametrize("n", [1, 300])
+def test_predictions_with_infinite_and_huge_weights(gpu, where, value, n):
+    from n_queens_b200 import learned
+    p = _params(1)
+    p[where] = value
+    c, l, r = (a[:n] for a in oracle.expand(14, 5))
+    m = learned.CostModel(seed=3)
+    m.set_params(p)
+    got, want = m.predict(14, c, l, r), _forward_over_set_bits(p, mlp_ref.features(14, c, l, r))
+    finite = np.isfinite(want)
+    assert np.array_equal(got[~finite], want[~finite].astype(np.float32), equal_nan=True)
+    if finite.any():
+        assert np.abs(got[finite] - want[finite]).max() <= 1e-5 * np.abs(want[finite]).max()
     m.close()
