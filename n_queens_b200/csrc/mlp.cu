@@ -538,15 +538,18 @@ __global__ void __launch_bounds__(PARTS == 1 ? 512 : 256, 1)
 //   out, dout                a warp per task
 //   dH2 = relu' . dout w3    (over H2)
 //   dH1 = relu' . dH2 W2     4 x 4 a thread
-//   dW2 += dH2^T H1          8 x 8 a thread, accumulated in registers
+//   dW2 += dH2^T H1          8 x 8 a thread, a tile's sum in registers, the tiles'
+//                            sum in shared memory
 //   dW1 += dH1^T X           8 x 6 a thread, accumulated in registers
 // The products read rows of 16-byte vectors; rows are padded to 132 floats, so
 // the eight lanes of a quarter-warp that read eight rows cover the banks once.
 // What bounds it: the shared-memory reads of the two 32 x 128 x 128 products (5
 // wavefronts for 16 multiply-adds of a warp), then FMA issue.  4096 tasks: 201 us
 // with 64 CTAs of 128 threads that kept the weight gradients in shared memory and
-// summed one unit per thread, 33 us so; error against 64 bits 1.3e-7 (1.7e-7
-// before).  Pre-training a cost model (2.3e6 tasks, 4 epochs) 562 -> 136 ms.
+// summed one unit per thread, 33 us so.  Relative error of dW2 against 64 bits, two
+// seeds: 3.5e-7 and 3.0e-7 before, 3.3e-7 and 2.5e-7 so at 4096 tasks; 3.9e-7 and
+// 1.9e-7 before, 3.8e-7 and 0.9e-7 so at 200,000 (4.3e-7 and 1.4e-7 with one running
+// sum over the tiles, which took 1.08 ms a call instead of 1.11).  Pre-training a cost model (2.3e6 tasks, 4 epochs) 562 -> 136 ms.
 constexpr int kTrainThreads = 256;
 constexpr int kPad = kH1 + 4;
 constexpr int kPartStride = (kParams + 3) & ~3;  // floats between partial gradients (16-byte rows)
@@ -561,6 +564,9 @@ struct TrainSmem {
     float w3[kH2], b1[kH1], b2[kH2];
     float dout[kGroup], y[kGroup], loss[kTrainThreads / 32];
     uint32_t m[3][kGroup];
+    // 64 KiB: dW2 of the tiles before the current one, [vector of a thread][thread].
+    // One running sum over all tiles of a CTA would be 1350 terms long at 200,000 tasks.
+    float4 dw2[16][kTrainThreads];
 };
 
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
@@ -595,7 +601,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     float gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, loss = 0.f;
     __syncthreads();
 
-    for (long long g0 = begin + (long long)blockIdx.x * kGroup; g0 < end; g0 += (long long)gridDim.x * kGroup) {
+    const long long first = begin + (long long)blockIdx.x * kGroup, second = first + (long long)gridDim.x * kGroup;
+    for (long long g0 = first; g0 < end; g0 += (long long)gridDim.x * kGroup) {
         const int gn = (int)min((long long)kGroup, end - g0);
         if (t < kGroup) {
             S.m[0][t] = S.m[1][t] = S.m[2][t] = 0;
@@ -724,6 +731,19 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             }
         }
         __syncthreads();
+        // ---- the last tile's dW2 joins those before it
+        if (g0 != first) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                float *r = &gw2[q >> 1][(q & 1) * 4];
+                if (g0 != second) {
+                    const float4 v = S.dw2[q][t];
+                    r[0] += v.x, r[1] += v.y, r[2] += v.z, r[3] += v.w;
+                }
+                S.dw2[q][t] = make_float4(r[0], r[1], r[2], r[3]);
+                r[0] = r[1] = r[2] = r[3] = 0.f;
+            }
+        }
         // ---- dW2 and dW1: rows 4*ty + {0..3, 64..67}; columns 4*tx + {0..3, 64..67}
         // of dW2 and 2*tx + 32*q + {0, 1} of dW1
 #pragma unroll 2
@@ -757,6 +777,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
         __syncthreads();
     }
 
+    if (second < end) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            float *r = &gw2[q >> 1][(q & 1) * 4];
+            const float4 v = S.dw2[q][t];
+            r[0] += v.x, r[1] += v.y, r[2] += v.z, r[3] += v.w;
+        }
+    }
     // ---- partial gradient of this CTA in the flat parameter layout
     float *g = grad_part + (size_t)blockIdx.x * kPartStride;
 #pragma unroll

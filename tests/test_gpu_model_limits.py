@@ -94,3 +94,28 @@ def test_predictions_with_infinite_and_huge_weights(gpu, where, value, n):
     if finite.any():
         assert np.abs(got[finite] - want[finite]).max() <= 1e-5 * np.abs(want[finite]).max()
     m.close()
+
+
+def test_weight_gradient_sums_tile_by_tile(gpu):
+    # Weights and labels on binary grids, so that the forward pass and every factor of
+    # dW2 are exact in FP32 and only the order of its sums shows; labels around the
+    # prediction, so that the terms cancel.  131072 tasks are 28 tiles for each of 148
+    # CTAs: a CPU emulation of both orders gives an error of 2.2e-7 with a sum per tile
+    # and 5.7e-7 with one running sum over a CTA's tiles.
+    from n_queens_b200 import learned
+    n, rng = 1 << 17, np.random.default_rng(1)
+    p = np.zeros(mlp_ref.NPARAMS, np.float32)
+    p[:mlp_ref.OFF_W3] = rng.integers(-8, 9, mlp_ref.OFF_W3) / 64
+    p[mlp_ref.OFF_B1:mlp_ref.OFF_W2] = rng.integers(-512, 513, mlp_ref.H1) / 4096
+    p[mlp_ref.OFF_W3:mlp_ref.OFF_B3] = rng.choice([-0.125, 0.125], mlp_ref.H2)
+    tasks = [a[:n] for a in oracle.expand(17, 6)]
+    X = mlp_ref.features(17, *tasks)
+    out = mlp_ref.forward(p, X)[0]
+    y = ((np.round(out * 2**20) + rng.integers(-2**22, 2**22, n)) / 2**20).astype(np.float32)
+    want = mlp_ref.loss_and_grad(p, X, y)[1]
+    m = learned.CostModel(seed=3)
+    m.set_params(p)
+    got = m.grad(np.full(n, 17, np.uint8), *tasks, y)[0]
+    m.close()
+    w2 = slice(mlp_ref.OFF_W2, mlp_ref.OFF_B2)
+    assert np.linalg.norm(got[w2] - want[w2]) <= 3.5e-7 * np.linalg.norm(want[w2])
