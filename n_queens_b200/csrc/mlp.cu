@@ -617,7 +617,9 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             const int s = i / kIn, f = i % kIn;
             S.x[i] = (float)(S.m[f >> 5][s] >> (f & 31) & 1u);
         }
-        // ---- layer 1, four bits at a time (row kIn of W1t is zero)
+        // ---- layer 1, four bits at a time (row kIn of W1t is zero).  The rows that fill a
+        // tile up are zero in every layer: they have no error, but 0 times an infinite
+        // activation would be NaN.
         for (int s = warp; s < kGroup; s += kTrainThreads / 32) {
             float4 acc = ld4(S.b1 + 4 * lane);
 #pragma unroll
@@ -638,6 +640,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
                         acc.w += __uint_as_float(v[k].y & 0xffff0000u);
                     }
                 }
+            if (s >= gn) acc = make_float4(0.f, 0.f, 0.f, 0.f);
             *reinterpret_cast<float4 *>(S.h1 + s * kPad + 4 * lane) =
                 make_float4(fmaxf(acc.x, 0.f), fmaxf(acc.y, 0.f), fmaxf(acc.z, 0.f), fmaxf(acc.w, 0.f));
         }
@@ -674,7 +677,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
                 float a = 0.f;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    acc[r][q] = fmaxf(acc[r][q], 0.f);
+                    acc[r][q] = s < gn ? fmaxf(acc[r][q], 0.f) : 0.f;
                     S.h2[s * kPad + lane + 32 * q] = acc[r][q];
                     a = fmaf(acc[r][q], S.w3[lane + 32 * q], a);
                 }
@@ -699,6 +702,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
         }
         __syncthreads();
         // ---- dH1 = relu' . dH2 W2: tasks 4*warp.., units 4*lane..
+        bool unbounded = false;  // an infinite or NaN dH1
         {
             float acc[4][4] = {};
             const float *dp = S.h2 + 4 * warp * kPad, *wp = S.w2 + 4 * lane;
@@ -725,12 +729,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             for (int r = 0; r < 4; ++r) {
                 const int s = 4 * warp + r;
                 const float4 h = ld4(S.h1 + s * kPad + 4 * lane);
-                *reinterpret_cast<float4 *>(S.dh1 + s * kPad + 4 * lane) =
+                const float4 d =
                     make_float4(h.x > 0.f ? acc[r][0] : 0.f, h.y > 0.f ? acc[r][1] : 0.f, h.z > 0.f ? acc[r][2] : 0.f,
                                 h.w > 0.f ? acc[r][3] : 0.f);
+                *reinterpret_cast<float4 *>(S.dh1 + s * kPad + 4 * lane) = d;
+                unbounded |= !(fabsf((d.x + d.y) + (d.z + d.w)) <= 3.4e38f);
             }
         }
-        __syncthreads();
+        unbounded = __syncthreads_or(unbounded);
         // ---- the last tile's dW2 joins those before it
         if (g0 != first) {
 #pragma unroll
@@ -745,7 +751,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             }
         }
         // ---- dW2 and dW1: rows 4*ty + {0..3, 64..67}; columns 4*tx + {0..3, 64..67}
-        // of dW2 and 2*tx + 32*q + {0, 1} of dW1
+        // of dW2 and 2*tx + 32*q + {0, 1} of dW1.  dW1 is the sum of dH1 over the tasks
+        // that have the bit set: a product with the bits, unless dH1 is unbounded.
 #pragma unroll 2
         for (int s = 0; s < kGroup; ++s) {
             const float4 da = ld4(S.h2 + s * kPad + 4 * ty), db = ld4(S.h2 + s * kPad + 64 + 4 * ty);
@@ -757,22 +764,28 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
 #pragma unroll
                 for (int b = 0; b < 8; ++b) gw2[a][b] = fmaf(d[a], h[b], gw2[a][b]);
         }
+        auto dw1 = [&](auto add) {
 #pragma unroll 2
-        for (int s = 0; s < kGroup; ++s) {
-            const float4 da = ld4(S.dh1 + s * kPad + 4 * ty), db = ld4(S.dh1 + s * kPad + 64 + 4 * ty);
-            const float d[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
-            float x[6];
+            for (int s = 0; s < kGroup; ++s) {
+                const float4 da = ld4(S.dh1 + s * kPad + 4 * ty), db = ld4(S.dh1 + s * kPad + 64 + 4 * ty);
+                const float d[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
+                float x[6];
 #pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const float2 v = *reinterpret_cast<const float2 *>(S.x + s * kIn + 2 * tx + 32 * q);
-                x[2 * q] = v.x;
-                x[2 * q + 1] = v.y;
+                for (int q = 0; q < 3; ++q) {
+                    const float2 v = *reinterpret_cast<const float2 *>(S.x + s * kIn + 2 * tx + 32 * q);
+                    x[2 * q] = v.x;
+                    x[2 * q + 1] = v.y;
+                }
+#pragma unroll
+                for (int a = 0; a < 8; ++a)
+#pragma unroll
+                    for (int b = 0; b < 6; ++b) gw1[a][b] = add(d[a], x[b], gw1[a][b]);
             }
-#pragma unroll
-            for (int a = 0; a < 8; ++a)
-#pragma unroll
-                for (int b = 0; b < 6; ++b) gw1[a][b] = fmaf(d[a], x[b], gw1[a][b]);
-        }
+        };
+        if (unbounded)
+            dw1([](float d, float x, float sum) { return x != 0.f ? sum + d : sum; });
+        else
+            dw1([](float d, float x, float sum) { return fmaf(d, x, sum); });
         for (int s = half * (kGroup / 2); s < (half + 1) * (kGroup / 2); ++s) gb1 += S.dh1[s * kPad + col];
         __syncthreads();
     }

@@ -1,4 +1,5 @@
-"""The cost model at its limits, on the GPU: waits for the tensor cores that expire, infinite and huge weights."""
+"""The cost model at its limits, on the GPU: waits for the tensor cores that expire, infinite and huge weights,
+the order of the gradient's sums."""
 import ctypes
 
 import numpy as np
@@ -119,3 +120,45 @@ def test_weight_gradient_sums_tile_by_tile(gpu):
     m.close()
     w2 = slice(mlp_ref.OFF_W2, mlp_ref.OFF_B2)
     assert np.linalg.norm(got[w2] - want[w2]) <= 3.5e-7 * np.linalg.norm(want[w2])
+
+
+def _gradient_over_set_bits(p, X, y):
+    """Float64 gradient by the sums that the model states: layer 1 and dW1 over set bits only."""
+    W1, b1, W2, b2, W3, b3 = mlp_ref.unpack(p)
+    with np.errstate(all="ignore"):
+        h1 = np.stack([np.fmax(b1 + W1[:, x > 0].sum(1), 0) for x in X])
+        h2 = np.fmax((h1[:, None, :] * W2[None]).sum(2) + b2, 0)
+        e = (h2 * W3).sum(1) + b3 - y
+        d = 2.0 / len(y) * e
+        dh2 = np.where(h2 > 0, d[:, None] * W3, 0.0)
+        dh1 = np.where(h1 > 0, (dh2[:, :, None] * W2[None]).sum(1), 0.0)
+        dw1 = np.stack([dh1[X[:, f] > 0].sum(0) for f in range(mlp_ref.IN)], 1)
+        parts = (dw1, dh1.sum(0), (dh2[:, :, None] * h1[:, None, :]).sum(0), dh2.sum(0), (d[:, None] * h2).sum(0),
+                 [d.sum()])
+        return (e * e).mean(), np.concatenate([np.asarray(q).ravel() for q in parts])
+
+
+# One task (31 rows of the tile unused), one more than a tile, ragged tiles.  where < 0: the label of task 0.
+@pytest.mark.parametrize("n", [1, 33, 300])
+@pytest.mark.parametrize("where,value", [
+    (-1, np.nan), (-1, np.inf), (5 * 96 + 20, np.inf), (5 * 96 + 3, np.inf), (5 * 96 + 3, np.nan),
+    (mlp_ref.OFF_B1 + 5, np.inf), (mlp_ref.OFF_W2 + 7, np.inf), (mlp_ref.OFF_B2 + 7, np.inf),
+    (mlp_ref.OFF_W3 + 7, np.inf), (mlp_ref.OFF_W3 + 7, np.nan), (mlp_ref.OFF_B3, np.inf)])
+def test_gradient_with_infinities(gpu, where, value, n):
+    from n_queens_b200 import learned
+    p, y = _params(1), np.random.default_rng(2).normal(12, 1.5, n).astype(np.float32)
+    if where < 0:
+        y[0] = value
+    else:
+        p[where] = value
+    tasks = [a[:n] for a in oracle.expand(14, 5)]
+    m = learned.CostModel(seed=3)
+    m.set_params(p)
+    got, loss = m.grad(np.full(n, 14, np.uint8), *tasks, y)
+    m.close()
+    want_loss, want = _gradient_over_set_bits(p, mlp_ref.features(14, *tasks), y.astype(np.float64))
+    finite = np.isfinite(want)
+    assert np.array_equal(got[~finite], want[~finite].astype(np.float32), equal_nan=True)
+    # FP32 sums of up to 300 terms, after layers of 96 and 128
+    assert np.abs(got[finite] - want[finite]).max() <= 1e-5 * np.abs(want[finite]).max()
+    assert np.isfinite(loss) == np.isfinite(want_loss)
