@@ -44,6 +44,8 @@ constexpr int kWordSum = kCtlWords + 0;
 constexpr int kWordNodes = kCtlWords + 1;
 constexpr int kWordStatus = kCtlWords + 2;
 constexpr int kWordBlocks = 16;
+constexpr size_t kGateWords = 32;        // 256 B of their own behind the per-CTA words
+constexpr size_t kCtlEnd(int sms) { return kWordBlocks + 5 * (size_t)sms * kMaxBlocksPerSm + kGateWords; }
 constexpr uint32_t kMailCap = 1u << 15;  // mailbox slots (256 B each)
 
 thread_local std::string g_last_error;
@@ -158,7 +160,7 @@ int ensure_ready(Ctx &c, int dev) {
     c.smem_optin = (int)prop.sharedMemPerBlockOptin;
     NQ_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     for (auto &e : c.ev) NQ_CUDA(cudaEventCreate(&e));
-    const size_t ctl_words = kWordBlocks + 5 * (size_t)c.sms * kMaxBlocksPerSm;
+    const size_t ctl_words = kCtlEnd(c.sms);
     NQ_CUDA(cudaMalloc(&c.d_ctl, ctl_words * sizeof(unsigned long long)));
     NQ_CUDA(cudaMemset(c.d_ctl, 0, ctl_words * sizeof(unsigned long long)));
     NQ_CUDA(cudaMalloc(&c.d_mail, kMailCap * sizeof(MailSlot)));
@@ -208,6 +210,8 @@ struct Launch {
     bool tight = false;  // count kernel without its extra slots
     int slots = 0;     // stack slots per lane of the launch: levels, and the count kernel's extra ones
     bool auto_inner = true;  // inner is the default, not the caller's
+    int rows = 0;      // rows left in the deepest task; with `look`: at most
+    bool look = false;  // the tasks' depth is not known on the host
 };
 
 // Chooses the persistent grid: CTA size, stack slots per lane and as many
@@ -219,6 +223,8 @@ int plan_launch(Ctx &c, const nq_config *cfg, int levels_needed, bool per_owner,
                 bool dih = false, bool resumable = false) {
     L.dih = dih;
     L.levels = std::max(1, levels_needed);
+    // its stack slots and the rows never stacked
+    L.rows = L.levels + (nodes || dih ? 1 : 3);
     if (cfg && cfg->stack_levels > NQ_MAX_STACK_LEVELS) {
         g_last_error = "stack_levels is above NQ_MAX_STACK_LEVELS";
         return NQ_ERR_ARG;
@@ -293,6 +299,26 @@ void fill_stats_launch(nq_stats *st, const Launch &L) {
     st->smem_bytes = L.smem;
 }
 
+// Rows left in the deepest task of a device-resident list, into a zeroed word.
+// Bound by its launch (300,000 tasks: 1.2 MB).
+__global__ void __launch_bounds__(256) deepest_task_kernel(const uint32_t *cols, long long n, int N,
+                                                           uint32_t *rows) {
+    const uint32_t last = (1u << N) - 1u;
+    uint32_t most = 0;
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += gridDim.x * 256ll) {
+        const uint32_t c = __ldg(cols + i);
+        if (!(c & ~last)) most = max(most, (uint32_t)N - __popc(c));
+    }
+    most = __reduce_max_sync(kFull, most);
+    __shared__ uint32_t s_most[8];
+    if ((threadIdx.x & 31u) == 0) s_most[threadIdx.x >> 5] = most;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 0; w < 8; ++w) most = max(most, s_most[w]);
+        if (most) atomicMax(rows, most);
+    }
+}
+
 // Enqueues queue reset + kernel on stream s.
 int enqueue_dfs(Ctx &c, DfsParams p, const Launch &L, bool per_owner, bool nodes, cudaStream_t s) {
     p.levels = L.slots;
@@ -305,10 +331,17 @@ int enqueue_dfs(Ctx &c, DfsParams p, const Launch &L, bool per_owner, bool nodes
         p.cta_wait = c.d_ctl + kWordBlocks + 4 * (size_t)c.sms * kMaxBlocksPerSm;
         NQ_CUDA(cudaMemsetAsync(p.cta_wait, 0, (size_t)L.grid * sizeof(unsigned long long), s));
     }
-    // rows left in the deepest task = its stack slots + the rows never stacked
-    if (L.levels + (nodes || L.dih ? 1 : 3) >= kMailRootRows) {
+    if (L.rows >= kMailRootRows && p.ntasks > 0) {
         p.mail = c.d_mail;
         p.mail_cap = kMailCap;
+        if (L.look) {
+            const int grid = (int)std::min<long long>((p.ntasks + 1023) / 1024, 2 * c.sms);
+            uint32_t *rows = (uint32_t *)(c.d_ctl + kCtlEnd(c.sms) - kGateWords);
+            NQ_CUDA(cudaMemsetAsync(rows, 0, sizeof(*rows), s));
+            deepest_task_kernel<<<grid, 256, 0, s>>>(p.cols, p.ntasks, p.N, rows);
+            NQ_CUDA(cudaGetLastError());
+            p.mail_gate = rows;
+        }
     }
     set_shares(p, (long long)L.grid * L.threads);
     if (p.lg_coarse > 0 && L.auto_inner) p.inner = kShareInner;
@@ -1488,6 +1521,7 @@ int nq_count_tasks_device(int N, const uint32_t *d_cols, const uint32_t *d_ld, c
     Launch L;
     rc = plan_launch(c, cfg, need, per_owner, want_nodes, L);
     if (rc) return rc;
+    L.look = !(cfg && cfg->stack_levels > 0);
     DfsParams p = base_params(c, N, n, cfg);
     long long qlen = n;
     rc = queue_len_of(cfg, n, qlen);

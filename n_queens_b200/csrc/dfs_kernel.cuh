@@ -134,6 +134,11 @@ struct DfsParams {
     // kMailEmpty at the start of a launch and again at its end.
     MailSlot *mail;
     uint32_t mail_cap;
+    // Where the host does not know the tasks' depth: the rows left in the deepest
+    // task; the mailbox is used only if they are kMailRootRows or more.  The word is
+    // not written during the launch and shares no cache line with the control words,
+    // whose atomics would hold up its load.  nullptr: used.
+    const uint32_t *mail_gate;
     // With cta_times: per-CTA sum over warps of the time spent waiting for mail.
     unsigned long long *cta_wait;
 };
@@ -940,8 +945,11 @@ __device__ __forceinline__ uint32_t share_mask(uint32_t lg, uint32_t way) {
 // more to hand over (a ticket, a post and a poll, about 3 us, then a warp that
 // starts with a few lanes) than they hold: with 10 instead of 12 the N=18 list
 // was 6 % slower.  For the same reason launches whose deepest task has fewer
-// than kMailRootRows rows left run without (60,001 prefixes of N=16, k=5: 0.60 ms
-// without, 0.82 with).
+// than kMailRootRows rows left run without (60,001 prefixes of N=16, k=5: 0.51 ms
+// without, 0.65 with).  A list in device memory whose depth is not stated is looked
+// through first (deepest_task_kernel, 2-3 us).  With the stack depth, an empty
+// board's, in its place 8000 prefixes of N=13, k=5 took 99 us a call instead of 74,
+// 300,007 of N=17, k=6 1.52 ms instead of 1.31.
 //
 // No count depends on the waiting: a waiter only watches its own slot, gives
 // up after kMailPatienceNs (it marks the slot kMailGone, so the supplier keeps
@@ -972,6 +980,11 @@ __device__ __forceinline__ MailSlot *mail_slot(const DfsParams &p, uint32_t t) {
 }
 __device__ __forceinline__ uint32_t mail_tag(const DfsParams &p, uint32_t t, uint32_t st) {
     return (t / p.mail_cap) << 2 | st;
+}
+
+// Whether this launch uses the mailbox (the same answer in all of its warps).
+__device__ __forceinline__ bool mail_on(const DfsParams &p) {
+    return p.mail && p.steal && (!p.mail_gate || __ldg(p.mail_gate) >= (uint32_t)kMailRootRows);
 }
 
 // Counts this warp as out of work; the last one to be so ends every wait.
@@ -1136,6 +1149,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                                   : (p.coarse << p.lg_coarse) +
                                         (((p.nqueue > 0 ? p.nqueue : p.ntasks) - p.coarse) << p.lg_fine);
     bool queue_live = qlen > 0;
+    const bool mail = MAIL && mail_on(p);
     unsigned looks = 0;           // trips, for the looks at the mailbox
     bool timed_out = false;
     unsigned long long deadline = 0;
@@ -1172,7 +1186,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
             if (now > deadline) {
                 if (lane == 0) atomicExch(p.ctl + kCtlTimeout, 1ull);
                 if (RESUME) timed_out = true;
-                if (MAIL && p.mail && p.steal) out_of_work(p, lane);
+                if (MAIL && mail) out_of_work(p, lane);
                 break;
             }
         }
@@ -1301,7 +1315,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                     check_idle = npair == __popc(idle);
                 } else if (idle == kFull) {
                     // whole warp idle, queue empty
-                    if (!MAIL || !p.mail || !p.steal) break;
+                    if (!MAIL || !mail) break;
                     if (!take_mail<DIH>(p, lane, cols, ld, rd, avail, owner, dih)) break;
                     sp = bot = my_base;
                     check_idle = false;
@@ -1312,7 +1326,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
         }
         // Other warps may be out of work (and the queue empty): offer them
         // stacked levels.
-        if (MAIL && p.mail && p.steal) {
+        if (MAIL && mail) {
             looks += check_idle ? 4u : 1u;
             if (looks >= 4u) {
                 looks = 0;
@@ -1465,7 +1479,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
             const unsigned long long err = *((volatile unsigned long long *)(p.ctl + kCtlError));
             const unsigned long long tmo = *((volatile unsigned long long *)(p.ctl + kCtlTimeout));
             // Every warp is out of work and no posted level was left behind.
-            const bool mail_ok = !MAIL || !p.mail || !p.steal || tmo ||
+            const bool mail_ok = !MAIL || !mail || tmo ||
                                  (long long)*((volatile unsigned long long *)(p.ctl + kCtlWork)) +
                                          (long long)gridDim.x * (blockDim.x >> 5) == 0;
             *p.status_out = ((err & kErrDepth) ? kStatDepth : 0ull) | (tmo ? kStatTimeout : 0ull) |
