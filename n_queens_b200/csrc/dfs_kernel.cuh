@@ -874,7 +874,8 @@ __device__ __forceinline__ uint32_t settle_level_dih(int n, uint32_t cols, uint3
 // so such a task counts 0, exactly as the reference recursion does.
 // VAR 4 and 6: `placed` receives the columns whose placements the nodes of the task's
 // own row are (its free columns on rows before N-1).
-template <int VAR, bool SETTLE = true>
+// SPARED: the rows by which the launch's stack may fall short of N-1-popc(cols).
+template <int VAR, bool SETTLE, int SPARED>
 __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, uint32_t &cols, uint32_t &ld,
                                               uint32_t &rd, uint32_t &avail, uint32_t &placed) {
     const int n = p.task_n ? (int)p.task_n[t] : p.N;
@@ -885,10 +886,7 @@ __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, u
     avail = 0;
     if (c & ~last) return 0;
     if (c == last) return 1;
-    // Stack slots this task can use: one per level that still has a sibling,
-    // at most N-1-popc(cols) -- N-3-popc(cols) for the filtered step, which
-    // never enters rows N-2 and N-1.
-    const int need = n - 1 - __popc(c) - kStackRowsSpared<VAR>;
+    const int need = n - 1 - __popc(c) - SPARED;
     if (need > p.levels) {
         atomicOr(p.ctl + kCtlError, kErrDepth);
         return 0;
@@ -1121,6 +1119,9 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
     // Lane registers of the step: the dihedral VAR 4 keeps VAR 3's form.
     constexpr int LVAR = (DIH && VAR == 4) ? 3 : VAR;
     constexpr bool MAIL = !RESUME;
+    // Node counts and the dihedral kernels take a stack of N-1-rows slots as
+    // nq_stack_levels states it (one more than their step uses), and refuse less.
+    constexpr int kSpared = NODES || DIH ? 0 : kStackRowsSpared<LVAR>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned long long red_cnt[32];
     __shared__ unsigned long long red_nodes[32];
@@ -1239,7 +1240,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                         if (t >= 0 && t < p.ntasks) {
                             sp = bot = my_base;
                             uint32_t placed = 0;
-                            uint32_t done = load_task<LVAR, !DIH>(p, t, cols, ld, rd, avail, placed);
+                            uint32_t done = load_task<LVAR, !DIH, kSpared>(p, t, cols, ld, rd, avail, placed);
                             if (DIH) {
                                 load_class(p, t, dih);
                                 done *= dih.w;
