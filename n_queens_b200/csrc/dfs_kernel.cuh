@@ -1150,7 +1150,8 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                                   : (p.coarse << p.lg_coarse) +
                                         (((p.nqueue > 0 ? p.nqueue : p.ntasks) - p.coarse) << p.lg_fine);
     bool queue_live = qlen > 0;
-    const bool mail = MAIL && mail_on(p);
+    const bool gate = !DIH && mail_on(p);  // (a dihedral list's depth is always known)
+    const auto mail = [&] { return MAIL && (DIH ? p.mail && p.steal : gate); };
     unsigned looks = 0;           // trips, for the looks at the mailbox
     bool timed_out = false;
     unsigned long long deadline = 0;
@@ -1187,7 +1188,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
             if (now > deadline) {
                 if (lane == 0) atomicExch(p.ctl + kCtlTimeout, 1ull);
                 if (RESUME) timed_out = true;
-                if (MAIL && mail) out_of_work(p, lane);
+                if (mail()) out_of_work(p, lane);
                 break;
             }
         }
@@ -1316,7 +1317,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                     check_idle = npair == __popc(idle);
                 } else if (idle == kFull) {
                     // whole warp idle, queue empty
-                    if (!MAIL || !mail) break;
+                    if (!mail()) break;
                     if (!take_mail<DIH>(p, lane, cols, ld, rd, avail, owner, dih)) break;
                     sp = bot = my_base;
                     check_idle = false;
@@ -1327,7 +1328,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
         }
         // Other warps may be out of work (and the queue empty): offer them
         // stacked levels.
-        if (MAIL && mail) {
+        if (mail()) {
             looks += check_idle ? 4u : 1u;
             if (looks >= 4u) {
                 looks = 0;
@@ -1480,7 +1481,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
             const unsigned long long err = *((volatile unsigned long long *)(p.ctl + kCtlError));
             const unsigned long long tmo = *((volatile unsigned long long *)(p.ctl + kCtlTimeout));
             // Every warp is out of work and no posted level was left behind.
-            const bool mail_ok = !MAIL || !mail || tmo ||
+            const bool mail_ok = !mail() || tmo ||
                                  (long long)*((volatile unsigned long long *)(p.ctl + kCtlWork)) +
                                          (long long)gridDim.x * (blockDim.x >> 5) == 0;
             *p.status_out = ((err & kErrDepth) ? kStatDepth : 0ull) | (tmo ? kStatTimeout : 0ull) |
