@@ -244,8 +244,9 @@ int nq_count_tasks_device_noalloc(int N, const uint32_t *d_cols, const uint32_t 
  * counted once; a mirror-symmetric board counts its left-half children twice
  * (the reference's half-board rule, src/n_queens.cpp:74-113, applied to any
  * symmetric board).  Every distinct board is split split_rows rows deeper
- * (0 = 3).  The same counts as nq_batch_create + nq_batch_run + destroy, without
- * building a plan (the subtasks go through the device's kept buffers). */
+ * (0 = 3).  The same counts as nq_batch_create + nq_batch_run + destroy.  Up to
+ * 16 MiB of subtasks and results go through the device's kept buffers, without a
+ * plan; a larger list builds one and gives its memory back. */
 int nq_count_batch(const nq_instance *inst, int64_t n, int split_rows, uint64_t *out, const nq_config *cfg,
                    nq_stats *stats);
 

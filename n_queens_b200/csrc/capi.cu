@@ -687,7 +687,7 @@ int write_checkpoint(const char *path, const Checkpoint &ck) {
 }
 
 constexpr int kDefaultSplit = 3;
-constexpr size_t kDirectBatchBytes = 16u << 20;  // about a million subtasks
+constexpr size_t kDirectBatchBytes = 16u << 20;  // a million subtasks, or boards without any
 
 // Reverses the low N bits (column j -> N-1-j).
 uint32_t rev_bits(uint32_t x, int N) {
@@ -1791,7 +1791,7 @@ int nq_count_batch(const nq_instance *inst, int64_t n, int split_rows, uint64_t 
     nq_batch plan;
     BatchTasks &t = plan.t;
     batch_tasks(inst, n, split_rows ? split_rows : kDefaultSplit, t);
-    if (t.task_bytes() > kDirectBatchBytes) {
+    if (t.task_bytes() + t.out_bytes() > kDirectBatchBytes) {
         rc = build_batch(c, cfg, plan);
         if (!rc) rc = run_batch(c, plan, stats);
         if (!rc) {
