@@ -271,8 +271,10 @@ typedef struct nq_tune_entry {
 
 /* Sweeps split depth 3..7, CTA size 64/128/256/512 and both stack layouts on
  * the given instances (other launch fields from `base`), then queue chunking
- * -- 256, 1024 (the default) and 4096 DFS steps between a warp's queue
- * refills -- at the fastest of those; replays each plan's graph and writes up
+ * -- 256, 1024 and 4096 DFS steps between a warp's queue refills -- at the
+ * fastest of those.  The sweep runs at base's interval, or at the one that each
+ * plan takes by itself (256 or 1024, see nq_config.inner_steps); the entries
+ * state the interval that was run.  Replays each plan's graph and writes up
  * to table_cap measured entries (40 + 2), their number and the fastest.  Each
  * plan's stack depth is the least its subtasks need (a deeper split needs
  * fewer slots), so the split sweep also sweeps the stack depth and the

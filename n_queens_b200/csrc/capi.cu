@@ -319,12 +319,18 @@ __global__ void __launch_bounds__(256) deepest_task_kernel(const uint32_t *cols,
     }
 }
 
+// Deals the queue of a launch out in shares and sets its DFS steps between visits.
+void set_queue(DfsParams &p, const Launch &L) {
+    p.steal = L.steal;
+    set_shares(p, (long long)L.grid * L.threads);
+    p.inner = p.lg_coarse > 0 && L.auto_inner ? kShareInner : L.inner;
+}
+
 // Enqueues queue reset + kernel on stream s.
 int enqueue_dfs(Ctx &c, DfsParams p, const Launch &L, bool per_owner, bool nodes, cudaStream_t s) {
     p.levels = L.slots;
-    p.inner = L.inner;
-    p.steal = L.steal;
     p.layout = L.layout;
+    set_queue(p, L);
     NQ_CUDA(cudaMemsetAsync(p.ctl, 0, kCtlWords * sizeof(unsigned long long), s));
     if (p.cta_times) {
         NQ_CUDA(cudaMemsetAsync(p.cta_times, 0, 2 * (size_t)L.grid * sizeof(unsigned long long), s));
@@ -343,8 +349,6 @@ int enqueue_dfs(Ctx &c, DfsParams p, const Launch &L, bool per_owner, bool nodes
             p.mail_gate = rows;
         }
     }
-    set_shares(p, (long long)L.grid * L.threads);
-    if (p.lg_coarse > 0 && L.auto_inner) p.inner = kShareInner;
     pick_kernel(per_owner, nodes, L.dih, L.tight)<<<L.grid, L.threads, L.smem, s>>>(p);
     NQ_CUDA(cudaGetLastError());
     return NQ_OK;
@@ -871,6 +875,7 @@ struct nq_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     nqb::Launch L;
+    int inner = 0;                         // DFS steps between visits of that launch
 };
 
 namespace nqb {
@@ -908,7 +913,9 @@ int build_batch(Ctx &c, const nq_config *cfg, nq_batch &B) {
         NQ_CUDA(cudaMemcpyAsync(d + 4 * m, B.t.tn.data(), (size_t)m, cudaMemcpyHostToDevice, c.stream));
     }
     NQ_CUDA(cudaStreamSynchronize(c.stream));
-    const DfsParams p = B.t.params(c, cfg, B.d_buf, B.d_out);
+    DfsParams p = B.t.params(c, cfg, B.d_buf, B.d_out);
+    set_queue(p, B.L);
+    B.inner = p.inner;
     for (auto *v : {&B.t.tc, &B.t.tl, &B.t.tr, &B.t.own}) std::vector<uint32_t>().swap(*v);  // uploaded
     std::vector<uint8_t>().swap(B.t.tn);
     // 4. one graph: reset, count, copy back (result words and per-owner sums)
@@ -1609,13 +1616,15 @@ int nq_batch_autotune(const nq_instance *inst, int64_t n, int repeats, const nq_
     static const int kSplits[] = {3, 4, 5, 6, 7};
     static const int kThreads[] = {64, 128, 256, 512};
     static const int kLayouts[] = {NQ_LAYOUT_INTERLEAVED, NQ_LAYOUT_LANE_MAJOR};
-    static const int kInner[] = {256, 4096};  // queue chunking tried beside the default
+    static const int kInner[] = {kShareInner, kDefaultInner, 4096};  // queue chunking tried beside the first
     nq_config cfg;
     if (base)
         cfg = *base;
     else
         memset(&cfg, 0, sizeof(cfg));
-    const int inner0 = cfg.inner_steps > 0 ? ((cfg.inner_steps + 3) & ~3) : kDefaultInner;
+    // The sweep runs at the caller's interval, or at the one that the list's own launch
+    // takes (0); the table states what was run.
+    const int inner0 = cfg.inner_steps > 0 ? ((cfg.inner_steps + 3) & ~3) : 0;
     int count = 0;
     best->ms = -1.0;
     // Measures one configuration; NQ_ERR_DEPTH (the CTA cannot hold the
@@ -1636,13 +1645,14 @@ int nq_batch_autotune(const nq_instance *inst, int64_t n, int repeats, const nq_
             rc = nq_batch_run(b, outv.data(), &st);
             sum_ms += st.kernel_ms;
         }
+        const int ran = b->inner;
         nq_batch_destroy(b);
         if (rc) return rc;
         nq_tune_entry e;
         e.split_rows = split;
         e.block_threads = threads;
         e.layout = layout;
-        e.inner_steps = inner;
+        e.inner_steps = ran;
         e.ms = sum_ms / repeats;
         if (count < table_cap) table[count] = e;
         ++count;
@@ -1658,7 +1668,7 @@ int nq_batch_autotune(const nq_instance *inst, int64_t n, int repeats, const nq_
     if (best->ms < 0) return NQ_ERR_ARG;
     const nq_tune_entry first = *best;
     for (int inner : kInner) {
-        if (inner == inner0) continue;
+        if (inner == first.inner_steps || (inner0 && inner == kDefaultInner)) continue;
         const int rc = measure(first.split_rows, first.block_threads, first.layout, inner);
         if (rc) return rc;
     }
