@@ -927,7 +927,10 @@ __device__ __forceinline__ uint32_t share_mask(uint32_t lg, uint32_t way) {
 // slot t % mail_cap as its (t / mail_cap)-th use, which the state word carries
 // above the kMail* value; its taker readies the slot for the next use.  A warp
 // holds one open ticket and claims one number at a time, so fewer than twice
-// the grid's warps are live at once, which is below mail_cap.
+// the grid's warps are live at once, which is below mail_cap.  Should a slot come
+// round while its last taker still reads (a warp that stood still for a whole
+// round), its next waiter stays until that is over, so that no level is posted to
+// a ticket that was given up unseen (tests/test_mailbox_model.py).
 //
 // kCtlWork counts, as a signed number, slots posted and not yet taken minus
 // warps out of work; with the grid's warps added it is the number of parties
@@ -1024,7 +1027,7 @@ __device__ __forceinline__ bool take_mail(const DfsParams &p, uint32_t lane, uin
         unsigned nap = 100;
         for (int i = 0; i < kMailPolls; ++i) {
             st = ld_acquire(&s->state);
-            if (st > none || globaltimer_ns() > until) break;
+            if (st > none || (st == none && globaltimer_ns() > until)) break;
             __nanosleep(nap);
             nap = min(nap * 2, 1000u);
         }
