@@ -99,7 +99,9 @@ typedef struct nq_config {
                                instead of on the host + H2D copy */
     uint32_t queue_len;     /* queue positions to run, 0 = all n (must be <= n): the count covers only the
                                tasks at positions 0 .. queue_len-1 (order[i] with NQ_ORDER_GIVEN, else i) */
-    int reserved[2];
+    int reserved[2];        /* 0.  For tests of the mailbox between warps: [0] 1 + microseconds that a warp
+                               waits for mail (up to 20,000, the default), [1] slots of its ring (a power
+                               of two above twice the launch's warps); other values change nothing */
 } nq_config;
 
 /* Timings and sizes of one call (all optional outputs). */
@@ -115,7 +117,7 @@ typedef struct nq_stats {
     int block_threads;  /* threads per CTA */
     int stack_levels;   /* stack slots per lane */
     int smem_bytes;     /* dynamic shared memory per CTA */
-    int reserved[5];
+    int reserved[5];    /* [0], [1]: mailbox tickets drawn and posts made or tried (host entries) */
     /* With nq_config.timing: kernel span from the first CTA start to the last
      * CTA end, the mean CTA busy time (its span less the time its warps waited
      * for work), and the idle fraction of the grid (1 - sum of CTA busy times /

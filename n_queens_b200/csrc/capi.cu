@@ -210,6 +210,7 @@ struct Launch {
     bool tight = false;  // count kernel without its extra slots
     int slots = 0;     // stack slots per lane of the launch: levels, and the count kernel's extra ones
     bool auto_inner = true;  // inner is the default, not the caller's
+    uint32_t mail_cap = kMailCap, mail_patience_ns = kMailPatienceNs;
     int rows = 0;      // rows left in the deepest task; with `look`: at most
     bool look = false;  // the tasks' depth is not known on the host
 };
@@ -288,6 +289,10 @@ int plan_launch(Ctx &c, const nq_config *cfg, int levels_needed, bool per_owner,
     L.auto_inner = !(cfg && cfg->inner_steps > 0);
     L.steal = (cfg && cfg->steal < 0) ? 0 : 1;
     L.layout = (cfg && cfg->layout == NQ_LAYOUT_LANE_MAJOR) ? 1 : 0;
+    if (cfg && cfg->reserved[0] > 0 && cfg->reserved[0] <= (int)(kMailPatienceNs / 1000))
+        L.mail_patience_ns = 1000u * (uint32_t)(cfg->reserved[0] - 1);
+    const long long ring = cfg ? cfg->reserved[1] : 0, warps = (long long)L.grid * (L.threads / 32);
+    if (ring > 2 * warps && ring < kMailCap && (ring & (ring - 1)) == 0) L.mail_cap = (uint32_t)ring;
     return NQ_OK;
 }
 
@@ -339,7 +344,8 @@ int enqueue_dfs(Ctx &c, DfsParams p, const Launch &L, bool per_owner, bool nodes
     }
     if (L.rows >= kMailRootRows && p.ntasks > 0) {
         p.mail = c.d_mail;
-        p.mail_cap = kMailCap;
+        p.mail_cap = L.mail_cap;
+        p.mail_patience_ns = L.mail_patience_ns;
         if (L.look) {
             const int grid = (int)std::min<long long>((p.ntasks + 1023) / 1024, 2 * c.sms);
             uint32_t *rows = (uint32_t *)(c.d_ctl + kCtlEnd(c.sms) - kGateWords);
@@ -526,7 +532,11 @@ int count_resident(Ctx &c, int N, const uint32_t *d_cols, const uint32_t *d_ld, 
     unsigned long long *res = (unsigned long long *)c.h_out.p;
     uint64_t *to_cnt = staged ? (uint64_t *)res + 8 : h_per_task;
     uint64_t *to_nodes = staged ? (uint64_t *)res + 8 + (want_cnt ? n : 0) : h_nodes_task;
-    NQ_CUDA(cudaMemcpyAsync(res, c.d_ctl + kWordSum, 3 * sizeof(*res), cudaMemcpyDeviceToHost, c.stream));
+    // mailbox tickets, open work, then the three result words
+    NQ_CUDA(cudaMemcpyAsync(res, c.d_ctl + kCtlMail, 5 * sizeof(*res), cudaMemcpyDeviceToHost, c.stream));
+    static_assert(kWordSum == kCtlMail + 2, "read back in one piece");
+    const unsigned long long *mail = res;
+    res += 2;
     if (want_cnt) NQ_CUDA(cudaMemcpyAsync(to_cnt, p.out_cnt, (size_t)n * 8, cudaMemcpyDeviceToHost, c.stream));
     if (want_nodes) NQ_CUDA(cudaMemcpyAsync(to_nodes, p.out_nodes, (size_t)n * 8, cudaMemcpyDeviceToHost, c.stream));
     NQ_CUDA(cudaEventRecord(c.ev[3], c.stream));
@@ -549,6 +559,8 @@ int count_resident(Ctx &c, int N, const uint32_t *d_cols, const uint32_t *d_ld, 
         cudaEventElapsedTime(&ms, c.ev[2], c.ev[3]);
         st->d2h_ms = ms;
         if (nodes) st->nodes = res[1];
+        st->reserved[0] = (int)(uint32_t)*mail;
+        st->reserved[1] = (int)(uint32_t)(*mail >> 32);
     }
     if (sum) *sum = res[0];
     if (nodes_total) *nodes_total = res[1];

@@ -134,6 +134,7 @@ struct DfsParams {
     // kMailEmpty at the start of a launch and again at its end.
     MailSlot *mail;
     uint32_t mail_cap;
+    uint32_t mail_patience_ns;  // how long a warp waits for mail, at most kMailPatienceNs
     // Where the host does not know the tasks' depth: the rows left in the deepest
     // task; the mailbox is used only if they are kMailRootRows or more.  The word is
     // not written during the launch and shares no cache line with the control words,
@@ -953,10 +954,10 @@ __device__ __forceinline__ uint32_t share_mask(uint32_t lg, uint32_t way) {
 // 300,007 of N=17, k=6 1.52 ms instead of 1.31.
 //
 // No count depends on the waiting: a waiter only watches its own slot, gives
-// up after kMailPatienceNs (it marks the slot kMailGone, so the supplier keeps
+// up after mail_patience_ns (it marks the slot kMailGone, so the supplier keeps
 // its levels) and then just ends.  CTAs that have not started count as working
 // and, when they start, find the queue as any other warp does.
-constexpr unsigned long long kMailPatienceNs = 20ull * 1000 * 1000;
+constexpr uint32_t kMailPatienceNs = 20u * 1000 * 1000;
 constexpr int kMailPolls = 1 << 16;   // second limit on a wait, in polls
 constexpr int kMailRootRows = 13;      // rows left in the deepest task from which a launch uses the mailbox
 constexpr uint32_t kMailMinRows = 12;  // rows left below which a level is not worth posting
@@ -1022,7 +1023,7 @@ __device__ __forceinline__ bool take_mail(const DfsParams &p, uint32_t lane, uin
     MailSlot *s = mail_slot(p, t);
     const uint32_t none = mail_tag(p, t, kMailEmpty);
     if (lane == 0) {
-        const unsigned long long until = globaltimer_ns() + kMailPatienceNs;
+        const unsigned long long until = globaltimer_ns() + p.mail_patience_ns;
         uint32_t st = none;
         unsigned nap = 100;
         for (int i = 0; i < kMailPolls; ++i) {
