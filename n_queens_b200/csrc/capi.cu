@@ -177,7 +177,7 @@ int ensure_ready(Ctx &c, int dev) {
     }
     NQ_CUDA(cudaFuncSetAttribute(dfs_kernel<false, false, kTightStepVar, kCountUnroll, true>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, c.smem_optin - static_smem));
-    NQ_CUDA(cudaFuncSetAttribute(dfs_kernel<false, false, kDihResumeStepVar, kUnroll, true, true>,
+    NQ_CUDA(cudaFuncSetAttribute(dfs_kernel<false, false, kDihResumeStepVar, kDihUnroll, true, true>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, c.smem_optin - static_smem));
     for (int po = 0; po < 2; ++po)
         NQ_CUDA(cudaFuncSetAttribute(pick_kernel(po, false, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1054,7 +1054,7 @@ int count_resumable_impl(int N, int rows, const nq_config *cfg, const char *chec
         NQ_CUDA(cudaMemcpyAsync(d_cont_in, ck.cont.data(), ncont * 16, cudaMemcpyHostToDevice, c.stream));
         if (dih) NQ_CUDA(cudaMemcpyAsync(d_cont_cls, ck.cls.data(), ncont, cudaMemcpyHostToDevice, c.stream));
     }
-    KernelFn fn = dih ? dfs_kernel<false, false, kDihResumeStepVar, kUnroll, true, true> : dfs_kernel<false, false, kTightStepVar, kCountUnroll, true>;
+    KernelFn fn = dih ? dfs_kernel<false, false, kDihResumeStepVar, kDihUnroll, true, true> : dfs_kernel<false, false, kTightStepVar, kCountUnroll, true>;
     Launch L;
     rc = plan_launch(c, cfg, stack_need(N, rows, !dih), false, false, L, dih, true);
     if (rc) return rc;
@@ -1793,7 +1793,7 @@ int nq_count_dihedral_tasks(int N, int rows, const uint32_t *cols, const uint32_
 int nq_count_batch(const nq_instance *inst, int64_t n, int split_rows, uint64_t *out, const nq_config *cfg,
                    nq_stats *stats) try {
     if (stats) memset(stats, 0, sizeof(*stats));
-    if (n == 0) return (n < 0 || split_rows < 0 || split_rows > 8) ? NQ_ERR_ARG : NQ_OK;
+    if (n == 0) return (split_rows < 0 || split_rows > 8) ? NQ_ERR_ARG : NQ_OK;
     // One pass needs no plan of its own: the subtasks go through the device's
     // buffers and the launch is issued directly (an allocation, a graph capture
     // and their release cost 2-4 ms, against some 20 us for a small board).  A

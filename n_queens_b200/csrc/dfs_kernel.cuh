@@ -175,99 +175,16 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
 // (node statistics), %7 bot, %8 = 1, %9 = 2, %10 = -1, %11 the slot stride
 // (512 B interleaved, 16 B lane-major).  The constants arrive as kernel
 // parameters, so the compiler cannot fold the multiply-adds below back into
-// ALU adds/moves.
+// ALU adds/moves: adds, left shifts and register moves are issued in multiply-add
+// form (the FMA pipe), which leaves LOP3, right shifts and compares to the ALU
+// pipe (an all-ALU form was 20 % slower).  Predicates come from LOP3's predicate
+// output (p = (result != 0) op q); four or sixteen steps share one asm block, whose
+// head sets the constant predicate `pt1` (true) once.
 //
-// VAR 1 issues the adds, the left shift and the four register moves in
-// multiply-add form (the FMA pipe), leaving the LOP3/shift/compare work on the
-// ALU pipe: about 11 instructions on each pipe per step (an all-ALU form ran
-// ~17 ALU + 7 FMA and was 20 % slower).
-#define NQB_STEP_HEAD                                                                 \
-    "{\n\t"                                                                           \
-    ".reg .pred pb, pd, pp, pe, pq;\n\t"                                              \
-    ".reg .b32 t, bit, nc, nl, nr, na;\n\t"
-
-#define NQB_STEP_CHILD_VAR1                                                           \
-    "mul.lo.s32 t, %3, %10;\n\t"                                                      \
-    "and.b32 bit, t, %3;\n\t"                                                         \
-    "setp.ne.u32 pb, bit, 0;\n\t"                                                     \
-    "mad.lo.s32 %3, bit, %10, %3;\n\t"                                                \
-    "mad.lo.s32 nc, bit, %8, %0;\n\t"                                                 \
-    "or.b32 nl, %1, bit;\n\t"                                                         \
-    "mul.lo.s32 nl, nl, %9;\n\t"                                                      \
-    "or.b32 nr, %2, bit;\n\t"                                                         \
-    "shr.s32 nr, nr, 1;\n\t"                                                          \
-    "lop3.b32 na, nc, nl, nr, 0x01;\n\t"                                              \
-    "setp.eq.u32 pe, nc, 0xffffffff;\n\t"                                             \
-    "@pe mad.lo.s32 %5, %8, %8, %5;\n\t"
-
-#define NQB_STEP_NODES_VAR1 "@pb mad.lo.s32 %6, %8, %8, %6;\n\t"
-
-#define NQB_STEP_TAIL_VAR1                                                            \
-    "setp.ne.and.u32 pd, na, 0, pb;\n\t"                                              \
-    "setp.ne.and.u32 pp, %3, 0, pd;\n\t"                                              \
-    "@pp st.shared.v4.u32 [%4], {%0, %1, %2, %3};\n\t"                                \
-    "@pp mad.lo.s32 %4, %8, %11, %4;\n\t"                                             \
-    "@pd mul.lo.s32 %0, nc, %8;\n\t"                                                  \
-    "@pd mul.lo.s32 %1, nl, %8;\n\t"                                                  \
-    "@pd mul.lo.s32 %2, nr, %8;\n\t"                                                  \
-    "@pd mul.lo.s32 %3, na, %8;\n\t"                                                  \
-    "setp.eq.u32 pq, %3, 0;\n\t"                                                      \
-    "setp.ne.and.u32 pq, %4, %7, pq;\n\t"                                             \
-    "@pq mad.lo.s32 %4, %10, %11, %4;\n\t"                                            \
-    "@pq ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"                                \
-    "}\n\t"
-
-// VAR 3 keeps a level's left-diagonal mask pre-shifted for its children
-// (register ld holds left << 1), so a child's left mask is one multiply-add,
-// (left | bit) << 1 = ld + 2*bit (bit is free, so | equals +), and the shift
-// for the grandchildren rides on the descend move (x 2 instead of x 1).  The
-// right diagonal stays in the reference's form: a right shift has no
-// multiply-add form, and a multiply-high in its place loaded the FMA pipe
-// more than the two ALU operations it saved (measured 5-7 % slower).  The
-// predicates come from LOP3's predicate output (p = (result != 0) op q)
-// instead of separate compares:
-//   lop3.and bit|pb      bit = avail & -avail,  pb = bit != 0
-//   lop3.and na|pd       na = ~(c|l|r),         pd = na != 0 && pb    (descend)
-//   lop3.or  avail|pk    avail ^= bit,          pk = avail != 0 || pd (level goes on)
-//   setp pp = avail != 0 && pd (push),  setp pq = sp != bot && !pk (pop)
-// 20 instructions per step (9 ALU, 9 FMA pipe, 2 shared) against VAR 1's 24,
-// same stack traffic.  Four steps share one asm block, whose head sets the
-// constant predicate `pt1` (true) once.  Operands as in VAR 1.
-#define NQB_STEP3_HEAD                                                                \
-    "{\n\t"                                                                           \
-    ".reg .pred pt1, pb, pd, pk, pp, pe, pq;\n\t"                                     \
-    ".reg .b32 t, bit, nc, nl, nr, na;\n\t"                                           \
-    "setp.ne.u32 pt1, %8, 0;\n\t"
-
-#define NQB_STEP3_CHILD                                                               \
-    "mul.lo.s32 t, %3, %10;\n\t"                                                      \
-    "lop3.and.b32 bit|pb, t, %3, 0, 0xC0, pt1;\n\t"                                   \
-    "mad.lo.s32 nc, bit, %8, %0;\n\t"                                                 \
-    "mad.lo.s32 nl, bit, %9, %1;\n\t"                                                 \
-    "or.b32 nr, %2, bit;\n\t"                                                         \
-    "shr.s32 nr, nr, 1;\n\t"                                                          \
-    "lop3.and.b32 na|pd, nc, nl, nr, 0x01, pb;\n\t"                                   \
-    "lop3.or.b32 %3|pk, %3, bit, 0, 0x3C, pd;\n\t"                                    \
-    "setp.eq.u32 pe, nc, 0xffffffff;\n\t"                                             \
-    "@pe add.u32 %5, %5, 1;\n\t"
-
-#define NQB_STEP3_TAIL                                                                \
-    "setp.ne.and.u32 pp, %3, 0, pd;\n\t"                                              \
-    "@pp st.shared.v4.u32 [%4], {%0, %1, %2, %3};\n\t"                                \
-    "@pp mad.lo.s32 %4, %8, %11, %4;\n\t"                                             \
-    "@pd mul.lo.s32 %0, nc, %8;\n\t"                                                  \
-    "@pd mul.lo.s32 %1, nl, %9;\n\t"                                                  \
-    "@pd mul.lo.s32 %2, nr, %8;\n\t"                                                  \
-    "@pd mul.lo.s32 %3, na, %8;\n\t"                                                  \
-    "setp.ne.and.u32 pq, %4, %7, !pk;\n\t"                                            \
-    "@pq mad.lo.s32 %4, %10, %11, %4;\n\t"                                            \
-    "@pq ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
-
-#define NQB_STEP3 NQB_STEP3_CHILD NQB_STEP3_TAIL
-#define NQB_STEP3_NODES NQB_STEP3_CHILD NQB_STEP_NODES_VAR1 NQB_STEP3_TAIL
-#define NQB_STEP3_X4 NQB_STEP3 NQB_STEP3 NQB_STEP3 NQB_STEP3
-#define NQB_STEP3_NODES_X4 NQB_STEP3_NODES NQB_STEP3_NODES NQB_STEP3_NODES NQB_STEP3_NODES
-
+// The forms: 4 and its in-place successors 6 and 7 for counts, 6 with a node counter
+// for node counts, 5 and DIH4 for the dihedral kernels.  (Steps 1 to 3, which
+// stepped every row, are gone.)
+//
 // VAR 4 ("filtered") enumerates only children that have a future.  A child C
 // of the level (placed at column `bit`) lists the columns of the next row it
 // may try (free = ~(c|l|r)); such a column b is dead when the row after it
@@ -294,12 +211,13 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
 // 12.6 % at N=21 (CPU model of the step); looking one row further would remove
 // 5 % more for another three operations, which is even.
 //
-// Lane registers: ld as in VAR 3; rd too is kept pre-shifted for the children
-// (right >> 1), so a child's right mask is (bit >> 1) + rd, which the compiler
+// Lane registers: ld holds the left mask pre-shifted for the children (left << 1),
+// so a child's left mask is one multiply-add, ld + 2*bit (bit is free, so | equals
+// +); rd too is kept pre-shifted (right >> 1), so a child's right mask is (bit >> 1) + rd, which the compiler
 // issues as one operation (shift-and-add) where `|` and the shift took two, and
 // the shift for the grandchildren rides on the descend move.  (A multiply-high
-// in its place loads the FMA pipe more than it saves, see VAR 3.)
-// Operands as in VAR 1 plus %12 = 0x3fffffff, %13 = -4, %14 = 30.
+// in its place loads the FMA pipe more than it saves: 5-7 % slower.)
+// Operands as above plus %12 = 0x3fffffff, %13 = -4, %14 = 30.
 //
 // What bounds it: integer issue (84 % of the issue slots, ALU pipe 72 %, FMA
 // 69 %, XU 55 %, shared-memory wavefronts 62 % at N=18).  Measured without and
@@ -359,7 +277,6 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
 
 #define NQB_STEP4 NQB_STEP4_CHILD NQB_STEP4_LOOK NQB_STEP4_TAIL
 #define NQB_STEP4_X4 NQB_STEP4 NQB_STEP4 NQB_STEP4 NQB_STEP4
-#define NQB_STEP4_X16 NQB_STEP4_X4 NQB_STEP4_X4 NQB_STEP4_X4 NQB_STEP4_X4
 
 // VAR 6: VAR 4 in place, the default.  VAR 4 computes a child beside its parent
 // and moves it over (four predicated moves) if it is entered.  Here the parent's
@@ -432,9 +349,9 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
 // level's is added when a task is loaded), and rows N-2 and N-1 and dead
 // children need no steps of their own.  No look-ahead: a child whose row two
 // below is full still has placements on the row between.  29 operations on 0.63
-// steps per node where VAR 3 takes 21 on one, and fewer stack accesses, which
-// bound VAR 3 (shared-memory wavefronts 65 %).  300,007 prefixes of N=17, k=6:
-// the whole call 3.39 ms with VAR 3, 3.01 with VAR 4's form, 2.78 in place.
+// steps per node where a step per placement took 21 on one, and fewer stack
+// accesses, which bound that form (shared-memory wavefronts 65 %).  300,007 prefixes
+// of N=17, k=6: the whole call 3.39 ms so, 3.01 with VAR 4's form, 2.78 in place.
 #define NQB_STEP6_NODES                                                               \
     "popc.b32 t, na;\n\t"                                                             \
     "@pb mad.lo.s32 %6, t, %8, %6;\n\t"
@@ -462,48 +379,20 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uin
 #define NQB_STEP7_X16 NQB_STEP7_X4 NQB_STEP7_X4 NQB_STEP7_X4 NQB_STEP7_X4
 #define NQB_STEP6N_X4 NQB_STEP6N NQB_STEP6N NQB_STEP6N NQB_STEP6N
 
-// Dihedral step: the VAR 1 step plus the class rules of the lane's task.
+// DIH4, the resumable dihedral kernel's step: the class rules of the lane's task,
 //   pc = popc(child cols) = 32 - N + child row
 //   pc > %12            -> the child row may not use the side columns, and
 //                          when it is row N-1 (pc == 31) only %13's columns
 //   child cols == ~0    -> one completion of weight %16 if the row N-1 queen
 //                          is at %14, else %15
-// Operands %0-%11 as in the plain step; %12 popc threshold, %13 row N-1
-// mask, %14 tie column bit, %15 weight, %16 tie weight, %17 ~side columns.
-#define NQB_STEP_HEAD_DIH                                                             \
-    "{\n\t"                                                                           \
-    ".reg .pred pb, pd, pp, pe, pq, ps, pl, px;\n\t"                                  \
-    ".reg .b32 t, bit, nc, nl, nr, na, pc, msk, w;\n\t"
-
-#define NQB_STEP_CHILD_DIH                                                            \
-    "mul.lo.s32 t, %3, %10;\n\t"                                                      \
-    "and.b32 bit, t, %3;\n\t"                                                         \
-    "setp.ne.u32 pb, bit, 0;\n\t"                                                     \
-    "mad.lo.s32 %3, bit, %10, %3;\n\t"                                                \
-    "mad.lo.s32 nc, bit, %8, %0;\n\t"                                                 \
-    "or.b32 nl, %1, bit;\n\t"                                                         \
-    "mul.lo.s32 nl, nl, %9;\n\t"                                                      \
-    "or.b32 nr, %2, bit;\n\t"                                                         \
-    "shr.s32 nr, nr, 1;\n\t"                                                          \
-    "lop3.b32 na, nc, nl, nr, 0x01;\n\t"                                              \
-    "popc.b32 pc, nc;\n\t"                                                            \
-    "setp.gt.u32 ps, pc, %12;\n\t"                                                    \
-    "setp.eq.u32 pl, pc, 31;\n\t"                                                     \
-    "selp.b32 msk, %13, %17, pl;\n\t"                                                 \
-    "@ps and.b32 na, na, msk;\n\t"                                                    \
-    "setp.eq.u32 pe, nc, 0xffffffff;\n\t"                                             \
-    "setp.eq.u32 px, bit, %14;\n\t"                                                   \
-    "selp.b32 w, %16, %15, px;\n\t"                                                   \
-    "@pe add.u32 %5, %5, w;\n\t"
-
-// The dihedral step in the filtered form (the dihedral kernels' default when
-// the count kernels run VAR 4): the left diagonal pre-shifted as in VAR 3, and
-// each child's list cut to its alive columns (those whose next row keeps a free
-// column, ignoring the class rules -- the rules only remove columns, so this
-// drops dead children only) except on row N-1, whose columns complete the
-// board.  Rows N-2 and N-1 are still stepped, because the class rules and the
-// tie weight decide what their completions count.  Operands as in the
-// dihedral step above.
+// with the left diagonal pre-shifted and each child's list cut to its alive
+// columns (those whose next row keeps a free column, ignoring the class rules --
+// the rules only remove columns, so this drops dead children only) except on row
+// N-1, whose columns complete the board.  Rows N-2 and N-1 are stepped, because the
+// class rules and the tie weight decide what their completions count, and because
+// checkpoints hold levels on those rows.
+// Operands %0-%11 as in the plain step; %12 popc threshold, %13 row N-1 mask, %14
+// tie column bit, %15 weight, %16 tie weight, %17 ~side columns.
 #define NQB_STEP_HEAD_DIH4                                                            \
     "{\n\t"                                                                           \
     ".reg .pred pb, pd, pp, pe, pq, pq0, ps, pl, px;\n\t"                              \
@@ -633,27 +522,18 @@ struct StepConsts {
     uint32_t one, two, mone, stride;  // stride: bytes between a lane's consecutive stack slots
 };
 
-// Step variant of the count kernels: 6 = filtered children in place (default; 7,
-// its form for per-owner outputs),
-// 4 = filtered children, 3 = pre-shifted left diagonal with LOP3 predicate
-// outputs, 1 = the reference's mask form with IMAD-form moves.  Kernels that
-// count DFS nodes run 6 in its node-counting form (3 and 1 themselves); the
-// dihedral kernels run variant 5 (1 with 1 and 3).
-#ifndef NQB_STEP_VAR
-#define NQB_STEP_VAR 6
-#endif
-constexpr int kStepVar = NQB_STEP_VAR;
-static_assert(kStepVar == 1 || kStepVar == 3 || kStepVar == 4 || kStepVar == 6, "step variant");
+// Step variants: of the count kernels ...
+constexpr int kStepVar = 6;
 // ... with per-owner outputs
-constexpr int kOwnerStepVar = kStepVar == 6 ? 7 : kStepVar;
-constexpr int kNodesStepVar = kStepVar == 4 ? 6 : kStepVar;
-constexpr int kDihStepVar = kStepVar >= 4 ? 5 : 1;
-// Count launches without room for the extra slots of 6 and 7, and the resumable
-// kernels, whose stated stack depth leaves none either.
-constexpr int kTightStepVar = kStepVar == 6 ? 4 : kStepVar;
-// The resumable dihedral kernel keeps the form that steps rows N-2 and N-1: its
-// checkpoints hold levels on those rows.
-constexpr int kDihResumeStepVar = kStepVar >= 4 ? 4 : 1;
+constexpr int kOwnerStepVar = 7;
+// ... that count DFS nodes
+constexpr int kNodesStepVar = 6;
+// ... of launches without room for the extra slots of 6 and 7, and of the resumable
+// kernel, whose stated stack depth leaves none either;
+constexpr int kTightStepVar = 4;
+// of the dihedral kernels, and of the resumable one (DIH4)
+constexpr int kDihStepVar = 5;
+constexpr int kDihResumeStepVar = 4;
 
 // Stack rows a step variant never pushes beyond the reference's N-1-rows: VAR 4
 // enters no level on row N-2 or N-1 and pushes what it leaves for a child, so the
@@ -666,17 +546,16 @@ constexpr int kStackRowsSpared = VAR == 4 ? 2 : VAR == 5 || VAR == 6 ? 1 : 0;
 // a level enumerates, and back (for the checkpoint file, which stores the
 // reference's form).  Going back loses left's bit 31 and right's bit 0, which
 // no later row can see (left bits only move further left, right bits further
-// right, and the level's own untried columns are stored beside them).
-template <int VAR>
-__device__ __forceinline__ uint32_t lane_ld(uint32_t left) { return VAR >= 3 ? left << 1 : left; }
-template <int VAR>
-__device__ __forceinline__ uint32_t ref_ld(uint32_t ld) { return VAR >= 3 ? ld >> 1 : ld; }
-template <int VAR>
+// right, and the level's own untried columns are stored beside them).  DIH4 keeps
+// the right mask as it is (PRE_RD false).
+__device__ __forceinline__ uint32_t lane_ld(uint32_t left) { return left << 1; }
+__device__ __forceinline__ uint32_t ref_ld(uint32_t ld) { return ld >> 1; }
+template <bool PRE_RD>
 __device__ __forceinline__ uint32_t lane_rd(uint32_t right) {
-    return VAR >= 4 ? (uint32_t)((int32_t)right >> 1) : right;
+    return PRE_RD ? (uint32_t)((int32_t)right >> 1) : right;
 }
-template <int VAR>
-__device__ __forceinline__ uint32_t ref_rd(uint32_t rd) { return VAR >= 4 ? rd << 1 : rd; }
+template <bool PRE_RD>
+__device__ __forceinline__ uint32_t ref_rd(uint32_t rd) { return PRE_RD ? rd << 1 : rd; }
 
 // The alive part of a level's untried columns (VAR 4): drops every column
 // whose child would leave the next row without a free column.  ld and rd in
@@ -691,59 +570,15 @@ __device__ __forceinline__ uint32_t alive_columns(uint32_t cols, uint32_t ld, ui
     return avail & (above | below);
 }
 
-template <bool NODES, int VAR>
-__device__ __forceinline__ void dfs_step(uint32_t &cols, uint32_t &ld, uint32_t &rd, uint32_t &avail, uint32_t &sp,
-                                         uint32_t &cnt, uint32_t &it, uint32_t bot, const StepConsts &k) {
-    static_assert(VAR == 1, "VAR 3 and 4 run in groups (dfs_steps3, dfs_steps4)");
-    if (NODES)
-        asm volatile(NQB_STEP_HEAD NQB_STEP_CHILD_VAR1 NQB_STEP_NODES_VAR1 NQB_STEP_TAIL_VAR1
-                     : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt), "+r"(it)
-                     : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride)
-                     : "memory");
-    else
-        asm volatile(NQB_STEP_HEAD NQB_STEP_CHILD_VAR1 NQB_STEP_TAIL_VAR1
-                     : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt), "+r"(it)
-                     : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride)
-                     : "memory");
-}
-
-template <int VAR>
+// One step of DIH4.
 __device__ __forceinline__ void dfs_step_dih(uint32_t &cols, uint32_t &ld, uint32_t &rd, uint32_t &avail, uint32_t &sp,
                                              uint32_t &cnt, uint32_t &it, uint32_t bot, const StepConsts &k,
                                              const DihLane &d, uint32_t noside) {
-    static_assert(VAR == 1 || VAR == 4, "dihedral step variants: 1 (reference form) and 4 (filtered)");
-    if constexpr (VAR == 4)
-        asm volatile(NQB_STEP_HEAD_DIH4 NQB_STEP_DIH4
-                     : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt), "+r"(it)
-                     : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(d.side_popc),
-                       "r"(d.last_mask), "r"(d.tie_bit), "r"(d.w), "r"(d.w_tie), "r"(noside)
-                     : "memory");
-    else
-        asm volatile(NQB_STEP_HEAD_DIH NQB_STEP_CHILD_DIH NQB_STEP_TAIL_VAR1
-                     : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt), "+r"(it)
-                     : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(d.side_popc),
-                       "r"(d.last_mask), "r"(d.tie_bit), "r"(d.w), "r"(d.w_tie), "r"(noside)
-                     : "memory");
-}
-
-// UNROLL steps of VAR 3 (UNROLL a multiple of 4), four per asm block.
-template <bool NODES, int UNROLL>
-__device__ __forceinline__ void dfs_steps3(uint32_t &cols, uint32_t &ld, uint32_t &rd, uint32_t &avail, uint32_t &sp,
-                                           uint32_t &cnt, uint32_t &it, uint32_t bot, const StepConsts &k) {
-    static_assert(UNROLL % 4 == 0, "VAR 3 unrolls in groups of 4");
-#pragma unroll
-    for (int g = 0; g < UNROLL / 4; ++g) {
-        if (NODES)
-            asm volatile(NQB_STEP3_HEAD NQB_STEP3_NODES_X4 "}\n\t"
-                         : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt), "+r"(it)
-                         : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride)
-                         : "memory");
-        else
-            asm volatile(NQB_STEP3_HEAD NQB_STEP3_X4 "}\n\t"
-                         : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt), "+r"(it)
-                         : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride)
-                         : "memory");
-    }
+    asm volatile(NQB_STEP_HEAD_DIH4 NQB_STEP_DIH4
+                 : "+r"(cols), "+r"(ld), "+r"(rd), "+r"(avail), "+r"(sp), "+r"(cnt), "+r"(it)
+                 : "r"(bot), "r"(k.one), "r"(k.two), "r"(k.mone), "r"(k.stride), "r"(d.side_popc),
+                   "r"(d.last_mask), "r"(d.tie_bit), "r"(d.w), "r"(d.w_tie), "r"(noside)
+                 : "memory");
 }
 
 // UNROLL steps of VAR 4 (no NODES form), four per asm block.  Operand %6 is
@@ -808,6 +643,23 @@ __device__ __forceinline__ void dfs_steps5(uint32_t &cols, uint32_t &ld, uint32_
                      : "memory");
 }
 
+// UNROLL steps of a kernel.
+template <int VAR, bool NODES, bool DIH, int UNROLL>
+__device__ __forceinline__ void dfs_steps(uint32_t &cols, uint32_t &ld, uint32_t &rd, uint32_t &avail, uint32_t &sp,
+                                          uint32_t &cnt, uint32_t &it, uint32_t bot, const StepConsts &k,
+                                          const DihLane &d, uint32_t noside) {
+    if constexpr (VAR == 5) {
+        dfs_steps5<UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, k, d, noside);
+    } else if constexpr (DIH) {
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) dfs_step_dih(cols, ld, rd, avail, sp, cnt, it, bot, k, d, noside);
+    } else if constexpr (VAR == 4) {
+        dfs_steps4<UNROLL>(cols, ld, rd, avail, sp, cnt, bot, k);
+    } else {
+        dfs_steps6<VAR, NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, k);
+    }
+}
+
 __device__ __forceinline__ void load_class_index(const DfsParams &p, uint32_t idx, DihLane &d) {
     const uint4 c = __ldg(p.cls_tab + idx);
     d.cls = idx;
@@ -820,14 +672,6 @@ __device__ __forceinline__ void load_class_index(const DfsParams &p, uint32_t id
 
 __device__ __forceinline__ void load_class(const DfsParams &p, long long t, DihLane &d) {
     load_class_index(p, __ldg(p.task_cls + t), d);
-}
-
-// DFS nodes (placements on rows before N-1) from a lane's counters: VAR 1 and 3
-// count every placement, of which a completion is the one on row N-1; VAR 6
-// counts the nodes themselves.
-template <int VAR>
-__device__ __forceinline__ uint32_t node_count(uint32_t it, uint32_t cnt) {
-    return VAR >= 4 ? it : it - cnt;
 }
 
 // VAR 4 and 6 keep only levels on rows 0..N-3, with their alive columns.  A level
@@ -876,7 +720,7 @@ __device__ __forceinline__ uint32_t settle_level_dih(int n, uint32_t cols, uint3
 // VAR 4 and 6: `placed` receives the columns whose placements the nodes of the task's
 // own row are (its free columns on rows before N-1).
 // SPARED: the rows by which the launch's stack may fall short of N-1-popc(cols).
-template <int VAR, bool SETTLE, int SPARED>
+template <bool PRE_RD, bool SETTLE, int SPARED>
 __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, uint32_t &cols, uint32_t &ld,
                                               uint32_t &rd, uint32_t &avail, uint32_t &placed) {
     const int n = p.task_n ? (int)p.task_n[t] : p.N;
@@ -893,10 +737,10 @@ __device__ __forceinline__ uint32_t load_task(const DfsParams &p, long long t, u
         return 0;
     }
     cols = c | ~last;
-    ld = lane_ld<VAR>(l);
-    rd = lane_rd<VAR>(r);
+    ld = lane_ld(l);
+    rd = lane_rd<PRE_RD>(r);
     avail = ~(cols | l | r);
-    if (VAR >= 4 && SETTLE) {
+    if (SETTLE) {
         placed = __popc(c) < n - 1 ? avail : 0u;
         return settle_level(n, cols, ld, rd, avail);
     }
@@ -1112,20 +956,19 @@ __device__ __forceinline__ uint32_t post_mail(const DfsParams &p, uint32_t lane,
 // instantiation so that the plain count kernel carries none of that code
 // (it measurably changed the code generated for the DFS loop).
 // DIH runs the dihedral decomposition: every task carries a class (rules and
-// weights, see DfsParams::cls_tab) and the step is dfs_step_dih.
+// weights, see DfsParams::cls_tab) and the step is VAR 5, with RESUME DIH4.
 // The count kernels are held to 32 registers (2 x 1024 threads): left to itself
 // the compiler takes 42 for one of them, and the loop's code is worse (N=19 133.6
 // -> 136.2 ms); the others spill at 32.
 template <bool PER_OWNER, bool NODES, int VAR, int UNROLL, bool RESUME = false, bool DIH = false>
 __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kernel(DfsParams p) {
-    static_assert(DIH ? VAR == 1 || VAR == 4 || VAR == 5 : VAR != 5, "dihedral step variants: 1, 4 and 5");
-    static_assert(!(NODES && (VAR == 4 || VAR == 7)), "node counts run variant 6");
-    // Lane registers of the step: the dihedral VAR 4 keeps VAR 3's form.
-    constexpr int LVAR = (DIH && VAR == 4) ? 3 : VAR;
+    static_assert(DIH ? (RESUME ? VAR == 4 : VAR == 5) : VAR == 4 || VAR == 6 || VAR == 7, "step variant");
+    static_assert(!NODES || VAR == 6, "node counts run variant 6");
+    constexpr bool kPreRd = !(DIH && VAR == 4);  // the lane form of rd, see lane_rd
     constexpr bool MAIL = !RESUME;
     // Node counts and the dihedral kernels take a stack of N-1-rows slots as
     // nq_stack_levels states it (one more than their step uses), and refuse less.
-    constexpr int kSpared = NODES || DIH ? 0 : kStackRowsSpared<LVAR>;
+    constexpr int kSpared = NODES || DIH ? 0 : kStackRowsSpared<VAR>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned long long red_cnt[32];
     __shared__ unsigned long long red_nodes[32];
@@ -1170,16 +1013,16 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
         if (PER_OWNER) {
             if (owner != kNoOwner && (avail == 0 || ((cnt | it) >> 31))) {
                 if (cnt) atomicAdd(p.out_cnt + owner, (unsigned long long)cnt);
-                if (NODES && it) atomicAdd(p.out_nodes + owner, (unsigned long long)node_count<VAR>(it, cnt));
+                if (NODES && it) atomicAdd(p.out_nodes + owner, (unsigned long long)it);
                 tot += cnt;
-                if (NODES) tot_nodes += node_count<VAR>(it, cnt);
+                if (NODES) tot_nodes += it;
                 cnt = 0;
                 it = 0;
                 if (avail == 0) owner = kNoOwner;
             }
         } else {
             tot += cnt;
-            if (NODES) tot_nodes += node_count<VAR>(it, cnt);
+            if (NODES) tot_nodes += it;
             cnt = 0;
             it = 0;
         }
@@ -1214,13 +1057,13 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                         // a level saved by an earlier, interrupted run
                         sp = bot = my_base;
                         const uint4 e = p.cont_in[q];
-                        const int need = __popc(~e.x) - 1 - kStackRowsSpared<LVAR>;
+                        const int need = __popc(~e.x) - 1 - kSpared;
                         if (need > p.levels) {
                             atomicOr(p.ctl + kCtlError, kErrDepth);
                         } else {
                             cols = e.x;
-                            ld = lane_ld<LVAR>(e.y);
-                            rd = lane_rd<LVAR>(e.z);
+                            ld = lane_ld(e.y);
+                            rd = lane_rd<kPreRd>(e.z);
                             avail = e.w;
                             // a level saved on row N-2 or N-1 (by a kernel that steps those rows)
                             if (VAR == 4 && !DIH) tot += settle_level(p.N, cols, ld, rd, avail);
@@ -1245,7 +1088,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                         if (t >= 0 && t < p.ntasks) {
                             sp = bot = my_base;
                             uint32_t placed = 0;
-                            uint32_t done = load_task<LVAR, !DIH, kSpared>(p, t, cols, ld, rd, avail, placed);
+                            uint32_t done = load_task<kPreRd, !DIH, kSpared>(p, t, cols, ld, rd, avail, placed);
                             if (DIH) {
                                 load_class(p, t, dih);
                                 done *= dih.w;
@@ -1266,7 +1109,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
                                 if (avail) owner = own;
                             }
                             tot += done;
-                            if (NODES && VAR >= 4) {
+                            if (NODES) {
                                 const uint32_t here = __popc(placed & share_mask(lg, way));
                                 if (PER_OWNER && here) atomicAdd(p.out_nodes + own, (unsigned long long)here);
                                 tot_nodes += here;
@@ -1345,40 +1188,12 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
         // ---- DFS steps
         if (check_idle) {
             for (int s = 0; s < p.inner; s += UNROLL) {
-#pragma unroll
-                for (int u = 0; u < ((VAR >= 3 && !DIH) || VAR == 5 ? 1 : UNROLL); ++u) {
-                    if constexpr (VAR == 5)
-                        dfs_steps5<UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
-                    else if constexpr (DIH)
-                        dfs_step_dih<VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
-                    else if constexpr (VAR == 6 || VAR == 7)
-                        dfs_steps6<VAR, NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
-                    else if constexpr (VAR == 4)
-                        dfs_steps4<UNROLL>(cols, ld, rd, avail, sp, cnt, bot, kc);
-                    else if constexpr (VAR == 3)
-                        dfs_steps3<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
-                    else
-                        dfs_step<NODES, VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
-                }
+                dfs_steps<VAR, NODES, DIH, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
                 if (__any_sync(kFull, avail == 0)) break;
             }
         } else {
             for (int s = 0; s < kTailTrip; s += UNROLL) {
-#pragma unroll
-                for (int u = 0; u < ((VAR >= 3 && !DIH) || VAR == 5 ? 1 : UNROLL); ++u) {
-                    if constexpr (VAR == 5)
-                        dfs_steps5<UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
-                    else if constexpr (DIH)
-                        dfs_step_dih<VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
-                    else if constexpr (VAR == 6 || VAR == 7)
-                        dfs_steps6<VAR, NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
-                    else if constexpr (VAR == 4)
-                        dfs_steps4<UNROLL>(cols, ld, rd, avail, sp, cnt, bot, kc);
-                    else if constexpr (VAR == 3)
-                        dfs_steps3<NODES, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
-                    else
-                        dfs_step<NODES, VAR>(cols, ld, rd, avail, sp, cnt, it, bot, kc);
-                }
+                dfs_steps<VAR, NODES, DIH, UNROLL>(cols, ld, rd, avail, sp, cnt, it, bot, kc, dih, p.noside);
                 const unsigned idle_now = __ballot_sync(kFull, avail == 0);
                 if (RESUME ? idle_now == kFull : (p.steal && __popc(idle_now) >= kTailIdle)) break;
             }
@@ -1397,7 +1212,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
             atomicOr(p.ctl + kCtlError, kErrContOverflow);
         } else if (mine) {
             if (avail) {
-                p.cont_out[at] = make_uint4(cols, ref_ld<LVAR>(ld), ref_rd<LVAR>(rd), avail);
+                p.cont_out[at] = make_uint4(cols, ref_ld(ld), ref_rd<kPreRd>(rd), avail);
                 if (p.cont_out_owner) p.cont_out_owner[at] = owner;
                 if (DIH) p.cont_out_cls[at] = (uint8_t)dih.cls;
                 ++at;
@@ -1405,7 +1220,7 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
             for (uint32_t a = bot; a != sp; a += stride, ++at) {
                 uint32_t x, y, z, w;
                 lds128(a, x, y, z, w);
-                p.cont_out[at] = make_uint4(x, ref_ld<LVAR>(y), ref_rd<LVAR>(z), w);
+                p.cont_out[at] = make_uint4(x, ref_ld(y), ref_rd<kPreRd>(z), w);
                 if (p.cont_out_owner) p.cont_out_owner[at] = owner;
                 if (DIH) p.cont_out_cls[at] = (uint8_t)dih.cls;
             }
@@ -1419,11 +1234,11 @@ __global__ void __launch_bounds__(1024, NODES || DIH || RESUME ? 0 : 2) dfs_kern
     if (PER_OWNER) {
         if (owner != kNoOwner) {
             if (cnt) atomicAdd(p.out_cnt + owner, (unsigned long long)cnt);
-            if (NODES && it) atomicAdd(p.out_nodes + owner, (unsigned long long)node_count<VAR>(it, cnt));
+            if (NODES && it) atomicAdd(p.out_nodes + owner, (unsigned long long)it);
         }
     }
     tot += cnt;
-    if (NODES) tot_nodes += node_count<VAR>(it, cnt);
+    if (NODES) tot_nodes += it;
 
     // ---- per-warp, per-CTA reduction
 #pragma unroll

@@ -15,29 +15,25 @@
 namespace nqb {
 
 // DFS steps per warp vote (the unroll of the kernel's inner loop), a
-// compile-time choice.  The filtered count step runs 16 between votes: fewer
-// votes and loop branches per step, for lanes that wait up to 15 steps for a
-// refill (1.1 % faster than 8 at N=21, k=6).  So does the node-count step
-// (300,007 prefixes of N=17: kernel 1.88 ms with 8, 1.79 with 16); the dihedral
-// steps keep 8.  A trip of the
+// compile-time choice.  The count steps run 16 between votes: fewer votes and loop
+// branches per step, for lanes that wait up to 15 steps for a refill (1.1 % faster
+// than 8 at N=21, k=6).  So does the node-count step (300,007 prefixes of N=17:
+// kernel 1.88 ms with 8, 1.79 with 16); the dihedral steps keep 8.  A trip of the
 // inner loop runs inner_steps rounded up to a multiple of the unroll.
-#ifndef NQB_UNROLL
-#define NQB_UNROLL 8
-#endif
 #ifndef NQB_COUNT_UNROLL
 #define NQB_COUNT_UNROLL 16
 #endif
 #ifndef NQB_NODES_UNROLL
 #define NQB_NODES_UNROLL 16
 #endif
-constexpr int kUnroll = NQB_UNROLL;
 #ifndef NQB_DIH_UNROLL
 #define NQB_DIH_UNROLL 8
 #endif
+constexpr int kCountUnroll = NQB_COUNT_UNROLL;
 constexpr int kNodesUnroll = NQB_NODES_UNROLL;
 constexpr int kDihUnroll = NQB_DIH_UNROLL;
-constexpr int kCountUnroll = kStepVar >= 4 ? NQB_COUNT_UNROLL : NQB_UNROLL;
-static_assert(kUnroll % 4 == 0 && kCountUnroll % 4 == 0, "inner_steps are rounded to multiples of 4");
+static_assert(kCountUnroll % 4 == 0 && kNodesUnroll % 4 == 0 && kDihUnroll % 4 == 0,
+              "inner_steps are rounded to multiples of 4");
 
 // DFS steps a warp runs between visits to the queue (the fold of its 32-bit
 // counters happens at the same point).
@@ -54,16 +50,17 @@ constexpr int kMaxAutoThreads = 512;
 // than the stated depth (nq_stack_levels) covers, variant 7 (per-owner outputs) on
 // two.  A launch with a stated CTA size that has no room for them runs
 // kTightStepVar, which needs none.
-inline int extra_slots(bool per_owner) { return kStepVar != 6 ? 0 : per_owner ? 2 : 1; }
+inline int extra_slots(bool per_owner) { return per_owner ? 2 : 1; }
 inline bool slots_fit(int threads, int slots, int smem_optin) {
     return (long long)(threads / 32) * slots * kSlotBytes + kDfsStaticSmem <= smem_optin;
 }
 
-// Stack slots per lane that a launch over prefixes with `placed` queens needs:
-// N-1-placed for the kernels that step every row (node counts, the dihedral
-// decomposition), two fewer for the filtered count step.  At least 1.
+// Stack slots per lane that a launch over prefixes with `placed` queens is given
+// and that nq_stack_levels states: N-1-placed for node counts and the dihedral
+// decomposition (whose steps push on one row fewer), two fewer for counts.  At
+// least 1.
 inline int stack_need(int N, int placed, bool filtered) {
-    const int need = N - 1 - placed - (filtered && kStepVar >= 4 ? kStackRowsSpared<4> : 0);
+    const int need = N - 1 - placed - (filtered ? kStackRowsSpared<4> : 0);
     return need < 1 ? 1 : need;
 }
 
