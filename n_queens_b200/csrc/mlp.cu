@@ -924,8 +924,8 @@ struct nq_mlp {
     int grad_parts_cap = 0;
     float *gsum = nullptr;  // summed gradient (nq_mlp_grad)
     // kErr* words of the forward kernels: [0] nq_mlp_predict*, [1] the scheduler.  In
-    // host memory, so that reading them costs a call neither a memset
-    // nor a copy.
+    // host memory (take_err_words), so that reading them costs a call neither a
+    // memset nor a copy.
     volatile int *err = nullptr;
     unsigned long long wait_limit = tc::kWaitLimit;
     void *loss_part = nullptr;  // floats
@@ -959,6 +959,35 @@ int grow(void *&p, size_t &cap, size_t need) {
     MLP_CUDA(cudaMalloc(&p, want));
     cap = want;
     return NQ_OK;
+}
+
+// Error words of models come from pinned pages of 64 models each, kept until exit:
+// a pinned allocation of its own took a model's creation from 1.1 to 4.2 ms.
+constexpr size_t kErrPage = 4096, kErrSlot = 64;
+std::mutex g_err_mu;
+std::vector<volatile int *> &g_err_free = *new std::vector<volatile int *>;  // outlives every model
+size_t g_err_slots = 0;
+
+cudaError_t take_err_words(volatile int *&words) {
+    std::lock_guard<std::mutex> lock(g_err_mu);
+    if (g_err_free.empty()) {
+        g_err_free.reserve(g_err_slots + kErrPage / kErrSlot);  // room for every slot, so that giving back cannot fail
+        void *page = nullptr;
+        const cudaError_t e = cudaHostAlloc(&page, kErrPage, cudaHostAllocPortable);
+        if (e != cudaSuccess) return e;
+        g_err_slots += kErrPage / kErrSlot;
+        for (size_t at = 0; at < kErrPage; at += kErrSlot) g_err_free.push_back((volatile int *)((char *)page + at));
+    }
+    words = g_err_free.back();
+    g_err_free.pop_back();
+    words[0] = words[1] = 0;
+    return cudaSuccess;
+}
+
+void give_err_words(volatile int *words) {
+    if (!words) return;
+    std::lock_guard<std::mutex> lock(g_err_mu);
+    g_err_free.push_back(words);
 }
 
 int train_blocks(nq_mlp *m) { return m->sms; }
@@ -1116,14 +1145,13 @@ int nq_mlp_create(int device, uint64_t seed, nq_mlp **out) try {
     auto room = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
     const size_t vec = room(kParams * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&m->block, 4 * vec + room(sizeof(Weights)));
-    if (e == cudaSuccess) e = cudaHostAlloc((void **)&m->err, 2 * sizeof(int), cudaHostAllocDefault);
+    if (e == cudaSuccess) e = take_err_words(m->err);
     char *at = (char *)m->block;
     for (float **v : {&m->master, &m->adam1, &m->adam2, &m->gsum}) {
         *v = (float *)at;
         at += vec;
     }
     m->w = (Weights *)at;
-    if (e == cudaSuccess) m->err[0] = m->err[1] = 0;
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(mlp_forward_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes);
     if (e == cudaSuccess)
@@ -1163,7 +1191,7 @@ int nq_mlp_destroy(nq_mlp *m) try {
     cudaFree(m->loss_part);
     cudaFree(m->data);
     cudaFree(m->sort_tmp);
-    cudaFreeHost((void *)m->err);
+    give_err_words(m->err);  // after cudaFree, which waits for the device
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
     return NQ_OK;

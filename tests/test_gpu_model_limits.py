@@ -162,3 +162,23 @@ def test_gradient_with_infinities(gpu, where, value, n):
     # FP32 sums of up to 300 terms, after layers of 96 and 128
     assert np.abs(got[finite] - want[finite]).max() <= 1e-5 * np.abs(want[finite]).max()
     assert np.isfinite(loss) == np.isfinite(want_loss)
+
+
+def test_error_words_of_many_models(gpu):
+    # more models at once than one page of error words holds; a failure shows in its own model only
+    from n_queens_b200 import learned
+    tasks = [a[:200] for a in oracle.expand(14, 5)]
+    models = [learned.CostModel(seed=k) for k in range(70)]
+    for k in (0, 63, 64, 69):
+        learned.lib.nq_mlp_set_wait_limit(models[k]._m, 0)
+    for k, m in enumerate(models):
+        if k in (0, 63, 64, 69):
+            with pytest.raises(gpu.NQError):
+                m.predict(14, *tasks)
+        else:
+            m.predict(14, *tasks)
+    for m in models:
+        m.close()
+    m = learned.CostModel(seed=0)  # takes a slot that a model before it has used
+    m.predict(14, *tasks)
+    m.close()
