@@ -20,8 +20,9 @@ Reported (one JSON line from rank 0):
              nq_count_learned; plain: nq_count): host expansion, pinned H2D
              copy of the tasks, schedule, kernel, D2H of the result; host wall
              clock per step;
-  roofline   integer-issue roofline: 22 warp-issue slots per DFS node against
-             numSMs x 4 schedulers x clock;
+  roofline   integer-issue roofline: the issue slots of the count step (30
+             operations on 0.555 steps per DFS node) against numSMs x 4
+             schedulers x clock;
   cpu_baseline  the reference's own CPU recursion (oracle/_ref, all host
              threads) on a seeded sample of the same tasks.
   dihedral   the same whole-board count through the 8-fold decomposition
@@ -51,7 +52,14 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-I_ALG = 22  # algorithmic warp-issue slots per DFS node (fixed cost model)
+# Issue slots per DFS node: the count step's operations times its steps per node (the
+# filtered step skips nodes without a future and counts rows N-2 and N-1 without
+# stepping them).  Steps from a CPU model of the step on random prefixes, k=6: 0.563
+# per node at N=18, 0.561 at N=19, 0.555 at N=21.
+STEP_OPS = 30
+STEPS_PER_NODE = 0.555
+ISSUE_PER_NODE = STEP_OPS * STEPS_PER_NODE
+REFERENCE_ISSUE_PER_NODE = 22  # the same for a step per node, as the reference's loop has
 METRIC = "DFS nodes/s (exact whole-board count, 1 B200)"
 
 # Whole-board workloads: published totals (README.md:16-25, logs/5090.log) and
@@ -506,7 +514,7 @@ def run_ours(args, world, rank, local):
         return {
             "value": world * nodes * nsteps / e_max, "unit": "nodes/s", "steps": nsteps,
             "wall_ms_per_step": 1000 * e_max / nsteps,
-            "h2d_bytes_per_step": 12 * ntasks, "d2h_bytes_per_step": 24 + 16 * grid,
+            "h2d_bytes_per_step": 12 * ntasks, "d2h_bytes_per_step": 40 + 24 * grid,
             "breakdown_ms": {key: statistics.mean(s[key] for s in stats)
                              for key in ("expand_ms", "h2d_ms", "schedule_ms", "kernel_ms", "d2h_ms", "total_ms")},
             "tail_idle_frac": statistics.mean(s["tail_idle_frac"] for s in stats),
@@ -636,14 +644,17 @@ def run_ours(args, world, rank, local):
     peak_src = "MEASURED_PEAKS.json sm_max_mhz"
     if not peak_clock:
         peak_clock, peak_src = clocks.get("sm_max_mhz") or 1965.0, "sampled clocks.max.sm"
-    achieved = (nodes * args.steps / dfs_s) * I_ALG / 32 / 1e9
+    node_rate = nodes * args.steps / dfs_s
+    achieved = node_rate * ISSUE_PER_NODE / 32 / 1e9
     peak = sms * 4 * peak_clock * 1e6 / 1e9
     roof = {
         "bound": "int-issue", "achieved": achieved, "peak": peak, "unit": "Gwarp-inst/s", "frac": achieved / peak,
         "traffic": traffic_from_profile(f"dfs_kernel_n{N}k{k}.md"),
         "kernel_ms_per_launch": 1000 * dfs_s / args.steps,
-        "note": (f"achieved = DFS nodes/s of the DFS kernel alone x {I_ALG} issue slots / 32 lanes; "
-                 f"peak = {sms} SMs x 4 schedulers x "
+        "rate_as_one_step_per_node": node_rate * REFERENCE_ISSUE_PER_NODE / 32 / 1e9 / peak,
+        "note": (f"achieved = DFS nodes/s of the DFS kernel alone x {STEPS_PER_NODE} steps per node x {STEP_OPS} "
+                 f"operations / 32 lanes; rate_as_one_step_per_node = the share of the peak that the same node rate would "
+                 f"take with {REFERENCE_ISSUE_PER_NODE} slots on every node (no bound); peak = {sms} SMs x 4 schedulers x "
                  f"{peak_clock:.0f} MHz ({peak_src}); traffic = ncu DRAM bytes per launch"),
     }
     if clocks.get("sm_mhz"):
@@ -652,7 +663,7 @@ def run_ours(args, world, rank, local):
         for arm in ("learned", "plain"):
             r22 = n22[arm]
             if "nodes_per_s_kernel" in r22:
-                r22["roofline_frac"] = r22["nodes_per_s_kernel"] * I_ALG / 32 / 1e9 / peak
+                r22["roofline_frac"] = r22["nodes_per_s_kernel"] * ISSUE_PER_NODE / 32 / 1e9 / peak
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:

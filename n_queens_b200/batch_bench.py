@@ -24,7 +24,7 @@ import numpy as np
 from . import BatchPlan, autotune_batch, count_tasks
 from .workloads import mirror_board, random_boards
 
-I_ALG = 22  # warp-issue slots per DFS node (the roofline's cost model)
+ISSUE_PER_NODE = 29 * 0.57  # the per-owner count step's operations x its steps per DFS node (CPU model, N=13..18)
 
 
 def plan_nodes(boards, split_rows: int) -> float:
@@ -109,7 +109,7 @@ def main():
         nodes = plan_nodes(boards, best["split_rows"])
         rate = nodes / (res["kernel_ms_mean"] / 1e3)
         res.update(dfs_nodes_est=nodes, nodes_per_s=rate,
-                   int_issue_frac=rate * I_ALG / 32 / (props.multi_processor_count * 4 * mhz * 1e6))
+                   int_issue_frac=rate * ISSUE_PER_NODE / 32 / (props.multi_processor_count * 4 * mhz * 1e6))
     print(json.dumps({k: v for k, v in res.items() if k != "autotune_table"}), flush=True)
     if args.json:
         with open(args.json, "w") as f:

@@ -784,13 +784,13 @@ __device__ __forceinline__ uint32_t share_mask(uint32_t lg, uint32_t way) {
 // as working from then on, so the sum reaches zero only when nothing is left;
 // the last CTA checks that (kStatMail).
 //
-// What it is worth (with the queue's shares, launch.h): 512 boards of N=12..17
-// split three rows deep 177 -> 10.2 ms (30 ms without the mailbox: single
-// subtrees of 4.5e6 nodes sat in one warp), 8 % of N=21's prefixes (2.1 tasks
-// per lane) 911 -> 838 ms.  Levels with fewer than kMailMinRows rows left cost
-// more to hand over (a ticket, a post and a poll, about 3 us, then a warp that
-// starts with a few lanes) than they hold: with 10 instead of 12 the N=18 list
-// was 6 % slower.  For the same reason launches whose deepest task has fewer
+// What it is worth beside the queue's shares (launch.h): 512 boards of N=12..17
+// split three rows deep 7.7 ms, 24 without the mailbox (single subtrees of 4.5e6
+// nodes sit in one warp); 8 % of N=21's prefixes (2.1 tasks per lane) 751 ms, 790
+// without.  Levels with fewer than kMailMinRows rows left cost more to hand over (a
+// ticket, a post and a poll, about 3 us, then a warp that starts with a few lanes)
+// than they hold: with 10 instead of 12 the batch takes 7.9 ms.  For the same
+// reason launches whose deepest task has fewer
 // than kMailRootRows rows left run without (60,001 prefixes of N=16, k=5: 0.51 ms
 // without, 0.65 with).  A list in device memory whose depth is not stated is looked
 // through first (deepest_task_kernel, 2-3 us).  With the stack depth, an empty
@@ -809,9 +809,9 @@ constexpr uint32_t kGiveMinRows = 8;   // the same for a level given to a lane o
 // Once the queue is empty a warp looks at its idle lanes after kTailTrip DFS
 // steps, or as soon as kTailIdle lanes are idle: a look (donation, mailbox) costs
 // about 290 instructions, ten steps, and with one at every newly idle lane they
-// were a quarter of all instructions of a batch.  512 boards of N=12..17
-// 9.65 ms with a look per idle lane, 8.9 at 8 lanes and 64 steps, 8.1 at 12 and
-// 96; 60,001 prefixes of N=16 538, 491, 489 us (496 at 16 lanes).  The loop of a
+// were a quarter of all instructions of a batch.  512 boards of N=12..17 9.1 ms
+// with a look per idle lane, 8.2 at 8 lanes and 64 steps, 7.7 at 12 and 96; 60,001
+// prefixes of N=16 500, 485, 484 us.  The loop of a
 // live queue keeps its plain any-vote: counting the lanes there costs 6 % (N=19).
 constexpr int kTailTrip = 96;
 constexpr int kTailIdle = 12;

@@ -101,11 +101,12 @@ constexpr int kShareInner = 256;
 // out finer, and the last ones always are.  Sixteen shares only where eight do
 // not give every lane one; half of them are empty (a level rarely has more than
 // eight alive columns), and an empty share still costs a visit to the queue.
-// Measured: 60,001 prefixes of N=16, k=5 (0.23 per lane) 0.96 ms whole, 0.59 in
-// shares; 1501 prefixes of N=13, k=4 0.19 -> 0.13 ms per call.  The line at 8, 4
-// and 2 positions per lane: 300,007 prefixes of N=17 with node counts (1.6 per
-// lane) 3.19, 3.03, 2.98 ms; 8 % of N=21's (2.1 per lane) 840, 839, 845 ms;
-// 1.1e6 of N=18 (4.8 per lane) 18.5 ms at all three.
+// Measured: 60,001 prefixes of N=16, k=5 (0.23 per lane) 1.35 ms whole, 0.48 in
+// shares; 1501 prefixes of N=13, k=4 0.131 -> 0.097 ms per call.  The line at 8, 4
+// and 2 positions per lane: a batch of 512 boards of N=12..17 7.7, 7.7, 8.0 ms;
+// 300,007 prefixes of N=17 with node counts (1.6 per lane) 1.63, 1.45, 1.39 ms of
+// kernel time; 8 % of N=21's (2.1 per lane) 750, 751, 750 ms; 1.1e6 of N=18 (4.8
+// per lane) 16.9 ms at all three.
 inline void set_shares(DfsParams &p, long long lanes) {
     const long long n = p.nqueue > 0 ? p.nqueue : p.ntasks;
     p.coarse = n;
