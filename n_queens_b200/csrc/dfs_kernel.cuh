@@ -773,8 +773,8 @@ __device__ __forceinline__ uint32_t share_mask(uint32_t lg, uint32_t way) {
 // above the kMail* value; its taker readies the slot for the next use.  A warp
 // holds one open ticket and claims one number at a time, so fewer than twice
 // the grid's warps are live at once, which is below mail_cap.  Should a slot come
-// round while its last taker still reads (a warp that stood still for a whole
-// round), its next waiter stays until that is over, so that no level is posted to
+// round while its last taker still reads (a warp that stood still while the
+// whole ring went by), its next waiter stays until that is over, so that no level is posted to
 // a ticket that was given up unseen (tests/test_mailbox_model.py).
 //
 // kCtlWork counts, as a signed number, slots posted and not yet taken minus
